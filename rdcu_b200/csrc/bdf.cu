@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "bdf.h"
+#include "prec1d.h"
 #include "spectral.h"
 
 namespace rdcu {
@@ -600,8 +601,14 @@ void make_RU(int order, double factor, double* RU) {
   } while (0)
 
 struct BDFEngine::Impl {
+  // the preconditioner: one kernel over the lines of a 1D problem, the FFT passes otherwise
   SpectralPlan prec;
-  bool have_prec = false;
+  LinePrecond prec1;
+  bool have_prec = false, line_prec = false;
+  cudaError_t precondition(const double* r_in, double* z_out, cudaStream_t st) {
+    const double* alpha_dev = &gm->alpha;
+    return line_prec ? prec1.apply(r_in, z_out, alpha_dev, st) : prec.precond(r_in, z_out, 0.0, alpha_dev, st);
+  }
   long long nN = 0;
   int blocks = 0;
   double *ytemp = nullptr, *yscale = nullptr, *f = nullptr, *d = nullptr, *dd = nullptr, *b = nullptr;
@@ -719,7 +726,10 @@ bool BDFEngine::init(FDProblem* fd, double atol, double rtol, int fixed, cudaStr
   std::vector<LinEntry> lin = linear_part(*fd);
   if (!lin.empty() && fd->n <= kMaxPrecFields) {
     std::string pm;
-    if (I.prec.init_precond(fd->n, fd->ndim, fd->Ns, fd->Ls, lin, &pm)) {
+    if (fd->ndim == 1) {
+      I.have_prec = I.line_prec = I.prec1.init(fd->n, fd->Ns[0], fd->Ls[0], lin);
+      if (I.have_prec) device_bytes += I.prec1.device_bytes;
+    } else if (I.prec.init_precond(fd->n, fd->ndim, fd->Ns, fd->Ls, lin, &pm)) {
       I.have_prec = true;
       device_bytes += I.prec.device_bytes;
     }
@@ -838,7 +848,7 @@ static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, do
     cudaError_t el = cudaSuccess;
     const double* zin = I.have_prec ? I.z : I.vj;
     k_gm_take<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, I.vj, nN);
-    if (I.have_prec) el = I.prec.precond(I.vj, I.z, 0.0, alpha_dev, st);
+    if (I.have_prec) el = I.precondition(I.vj, I.z, st);
     k_apply_A_dev<<<nb, 256, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, alpha_dev, zin, I.w, nN);
     for (int pass = 0; pass < 2; ++pass) {
       k_dots_sum<<<dim3(kRedBlocks, m + 1), kRedThreads, 0, st>>>(I.V, I.gm, -1, I.w, nN, I.part, I.arrivals,
@@ -860,7 +870,7 @@ static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, do
     k_gm_backsub<<<1, 32, 0, st>>>(I.gm);
     k_vcomb_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, nN);
     if (I.have_prec) {
-      el = I.prec.precond(I.w, I.z, 0.0, alpha_dev, st);
+      el = I.precondition(I.w, I.z, st);
       k_axpy<<<nb, 256, 0, st>>>(1.0, I.z, x, nN);
     } else {
       k_axpy<<<nb, 256, 0, st>>>(1.0, I.w, x, nN);
@@ -1002,7 +1012,7 @@ static cudaError_t build_newton_graph(BDFEngine::Impl& I, FDProblem& fd, const d
       k_gm_backsub<<<1, 32, 0, st>>>(I.gm);
       k_vcomb_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, nN);
       if (I.have_prec) {
-        RDCU_TRY(I.prec.precond(I.w, I.z, 0.0, alpha_dev, st));
+        RDCU_TRY(I.precondition(I.w, I.z, st));
         k_axpy<<<nb, 256, 0, st>>>(1.0, I.z, x, nN);
       } else {
         k_axpy<<<nb, 256, 0, st>>>(1.0, I.w, x, nN);
@@ -1014,7 +1024,7 @@ static cudaError_t build_newton_graph(BDFEngine::Impl& I, FDProblem& fd, const d
     e = capture_into(Ba, st, [&]() -> cudaError_t {
       const double* zin = I.have_prec ? I.z : I.vj;
       k_gm_take<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, I.vj, nN);
-      if (I.have_prec) RDCU_TRY(I.prec.precond(I.vj, I.z, 0.0, alpha_dev, st));
+      if (I.have_prec) RDCU_TRY(I.precondition(I.vj, I.z, st));
       k_apply_A_dev<<<nb, 256, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, alpha_dev, zin, I.w, nN);
       for (int pass = 0; pass < 2; ++pass) {
         k_dots_sum<<<dim3(kRedBlocks, m + 1), kRedThreads, 0, st>>>(I.V, I.gm, -1, I.w, nN, I.part, I.arrivals,

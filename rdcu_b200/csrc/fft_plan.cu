@@ -5,8 +5,8 @@
 
 namespace rdcu {
 
-bool make_line_plan(int L, LinePlan* p) {
-  if (L < 1 || L > kMaxLine) return false;
+bool make_line_plan(int L, LinePlan* p, int most) {
+  if (L < 1 || L > most) return false;
   p->L = L;
   p->nstages = 0;
   int rem = L;

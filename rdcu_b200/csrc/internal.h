@@ -53,7 +53,8 @@ struct LinePlan {
   FastDiv div_ns[kMaxStages];  // span Ns before stage s
 };
 
-bool make_line_plan(int L, LinePlan* p);
+// false when L has another prime factor than 2..13 or is above `most`
+bool make_line_plan(int L, LinePlan* p, int most = kMaxLine);
 // exp(-2 pi i t / L) for t < L, rounded from long double.
 void make_twiddles(int L, std::vector<double2>& tw);
 

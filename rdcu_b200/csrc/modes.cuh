@@ -1,0 +1,105 @@
+// Fourier modes of the constant-coefficient finite-difference operators (device code):
+// their symbols and the small dense solves of the BDF preconditioners.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "fft_line.cuh"
+#include "internal.h"
+
+namespace rdcu {
+
+// Symbol of the constant-coefficient FD operator of one linear entry at multi-index
+// nidx (see LinEntry): returns the complex value.
+__device__ __forceinline__ double2 lin_symbol(const LinEntry& e, const int* nidx, const LinTable& t) {
+  if (e.nax == 0) return make_double2(1.0, 0.0);
+  const int a = e.ax0;
+  const double sa = t.sinv[t.off[a] + nidx[a]];
+  if (e.nax == 1) return make_double2(0.0, sa / t.dx[a]);
+  if (e.ax0 == e.ax1) {
+    const double ca = t.cosv[t.off[a] + nidx[a]];
+    return make_double2((2.0 * ca - 2.0) / (t.dx[a] * t.dx[a]), 0.0);
+  }
+  const int b = e.ax1;
+  const double sb = t.sinv[t.off[b] + nidx[b]];
+  return make_double2(-2.0 * sa * sb / (t.dx[a] * t.dx[b]), 0.0);
+}
+
+// x = (I + alpha L(k))^-1 r at one mode, n <= NF <= kMaxPrecFields, Gaussian elimination
+// with partial pivoting; a (numerically) singular mode is passed through unchanged.
+template <int NF>
+__device__ __forceinline__ void mode_solve(const LinTable& t, const int* nidx, double2* v, int n) {
+  static_assert(NF <= kMaxPrecFields, "mode solves of at most kMaxPrecFields fields");
+  double2 A[NF][NF];
+  double2 b[NF];
+#pragma unroll
+  for (int i = 0; i < NF; ++i) {
+#pragma unroll
+    for (int j = 0; j < NF; ++j) A[i][j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+    b[i] = i < n ? v[i] : make_double2(0.0, 0.0);
+  }
+  const double alpha = t.alpha_dev ? *t.alpha_dev : t.alpha;
+  for (int q = 0; q < t.nent; ++q) {
+    const LinEntry e = t.ent[q];
+    const double2 sy = lin_symbol(e, nidx, t);
+    const double cf = alpha * e.coef;
+#pragma unroll
+    for (int i = 0; i < NF; ++i)
+#pragma unroll
+      for (int j = 0; j < NF; ++j)
+        if (i == e.row && j == e.src) {
+          A[i][j].x += cf * sy.x;
+          A[i][j].y += cf * sy.y;
+        }
+  }
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < NF; ++k) {
+    if (k >= n) break;
+    // pivot
+    int p = k;
+    double best = A[k][k].x * A[k][k].x + A[k][k].y * A[k][k].y;
+#pragma unroll
+    for (int i = k + 1; i < NF; ++i) {
+      if (i >= n) break;
+      const double m2 = A[i][k].x * A[i][k].x + A[i][k].y * A[i][k].y;
+      if (m2 > best) { best = m2; p = i; }
+    }
+    if (!(best > 1e-300)) { ok = false; break; }
+#pragma unroll
+    for (int i = 0; i < NF; ++i)
+      if (i == p && p != k) {
+#pragma unroll
+        for (int j = 0; j < NF; ++j) { const double2 tmp = A[k][j]; A[k][j] = A[i][j]; A[i][j] = tmp; }
+        const double2 tb = b[k]; b[k] = b[i]; b[i] = tb;
+      }
+    const double2 piv = A[k][k];
+    const double inv = 1.0 / (piv.x * piv.x + piv.y * piv.y);
+    const double2 ip = make_double2(piv.x * inv, -piv.y * inv);
+#pragma unroll
+    for (int i = k + 1; i < NF; ++i) {
+      if (i >= n) break;
+      const double2 f = c_mul(A[i][k], ip);
+#pragma unroll
+      for (int j = k; j < NF; ++j) A[i][j] = c_sub(A[i][j], c_mul(f, A[k][j]));
+      b[i] = c_sub(b[i], c_mul(f, b[k]));
+    }
+  }
+  if (!ok) return;
+#pragma unroll
+  for (int k = NF - 1; k >= 0; --k) {
+    if (k >= n) continue;
+    double2 acc = b[k];
+#pragma unroll
+    for (int j = k + 1; j < NF; ++j)
+      if (j < n) acc = c_sub(acc, c_mul(A[k][j], b[j]));
+    const double2 piv = A[k][k];
+    const double inv = 1.0 / (piv.x * piv.x + piv.y * piv.y);
+    b[k] = c_mul(acc, make_double2(piv.x * inv, -piv.y * inv));
+  }
+  
+#pragma unroll
+  for (int i = 0; i < NF; ++i)
+    if (i < n) v[i] = b[i];
+}
+
+}  // namespace rdcu

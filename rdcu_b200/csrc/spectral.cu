@@ -36,6 +36,7 @@
 #include <type_traits>
 
 #include "fft_line.cuh"
+#include "modes.cuh"
 #include "pencil.cuh"
 #include "spectral.h"
 
@@ -1278,95 +1279,6 @@ __global__ void k_mult1d(Mult1DArgs a) {
   a.Sc[(long long)ch * a.Mh + kx] = acc;
 }
 
-// Symbol of the constant-coefficient FD operator of one linear entry at multi-index
-// nidx (see LinEntry): returns the complex value.
-__device__ __forceinline__ double2 lin_symbol(const LinEntry& e, const int* nidx, const LinTable& t) {
-  if (e.nax == 0) return make_double2(1.0, 0.0);
-  const int a = e.ax0;
-  const double sa = t.sinv[t.off[a] + nidx[a]];
-  if (e.nax == 1) return make_double2(0.0, sa / t.dx[a]);
-  if (e.ax0 == e.ax1) {
-    const double ca = t.cosv[t.off[a] + nidx[a]];
-    return make_double2((2.0 * ca - 2.0) / (t.dx[a] * t.dx[a]), 0.0);
-  }
-  const int b = e.ax1;
-  const double sb = t.sinv[t.off[b] + nidx[b]];
-  return make_double2(-2.0 * sa * sb / (t.dx[a] * t.dx[b]), 0.0);
-}
-
-// x = (I + alpha L(k))^-1 r at one mode, n <= kMaxPrecFields, Gaussian elimination
-// with partial pivoting; a (numerically) singular mode is passed through unchanged.
-__device__ __forceinline__ void mode_solve(const LinTable& t, const int* nidx, double2* v, int n) {
-  double2 A[kMaxPrecFields][kMaxPrecFields];
-  double2 b[kMaxPrecFields];
-#pragma unroll
-  for (int i = 0; i < kMaxPrecFields; ++i) {
-#pragma unroll
-    for (int j = 0; j < kMaxPrecFields; ++j) A[i][j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-    b[i] = i < n ? v[i] : make_double2(0.0, 0.0);
-  }
-  const double alpha = t.alpha_dev ? *t.alpha_dev : t.alpha;
-  for (int q = 0; q < t.nent; ++q) {
-    const LinEntry e = t.ent[q];
-    const double2 sy = lin_symbol(e, nidx, t);
-    const double cf = alpha * e.coef;
-#pragma unroll
-    for (int i = 0; i < kMaxPrecFields; ++i)
-#pragma unroll
-      for (int j = 0; j < kMaxPrecFields; ++j)
-        if (i == e.row && j == e.src) {
-          A[i][j].x += cf * sy.x;
-          A[i][j].y += cf * sy.y;
-        }
-  }
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < kMaxPrecFields; ++k) {
-    if (k >= n) break;
-    // pivot
-    int p = k;
-    double best = A[k][k].x * A[k][k].x + A[k][k].y * A[k][k].y;
-#pragma unroll
-    for (int i = k + 1; i < kMaxPrecFields; ++i) {
-      if (i >= n) break;
-      const double m2 = A[i][k].x * A[i][k].x + A[i][k].y * A[i][k].y;
-      if (m2 > best) { best = m2; p = i; }
-    }
-    if (!(best > 1e-300)) { ok = false; break; }
-#pragma unroll
-    for (int i = 0; i < kMaxPrecFields; ++i)
-      if (i == p && p != k) {
-#pragma unroll
-        for (int j = 0; j < kMaxPrecFields; ++j) { const double2 tmp = A[k][j]; A[k][j] = A[i][j]; A[i][j] = tmp; }
-        const double2 tb = b[k]; b[k] = b[i]; b[i] = tb;
-      }
-    const double2 piv = A[k][k];
-    const double inv = 1.0 / (piv.x * piv.x + piv.y * piv.y);
-    const double2 ip = make_double2(piv.x * inv, -piv.y * inv);
-#pragma unroll
-    for (int i = k + 1; i < kMaxPrecFields; ++i) {
-      if (i >= n) break;
-      const double2 f = c_mul(A[i][k], ip);
-#pragma unroll
-      for (int j = k; j < kMaxPrecFields; ++j) A[i][j] = c_sub(A[i][j], c_mul(f, A[k][j]));
-      b[i] = c_sub(b[i], c_mul(f, b[k]));
-    }
-  }
-  if (!ok) return;
-#pragma unroll
-  for (int k = kMaxPrecFields - 1; k >= 0; --k) {
-    if (k >= n) continue;
-    double2 acc = b[k];
-#pragma unroll
-    for (int j = k + 1; j < kMaxPrecFields; ++j)
-      if (j < n) acc = c_sub(acc, c_mul(A[k][j], b[j]));
-    const double2 piv = A[k][k];
-    const double inv = 1.0 / (piv.x * piv.x + piv.y * piv.y);
-    b[k] = c_mul(acc, make_double2(piv.x * inv, -piv.y * inv));
-  }
-  for (int i = 0; i < n; ++i) v[i] = b[i];
-}
-
 struct MidSolveArgs {
   int L0, I, TW, n, ndim, Mh;
   FastDiv dTW, dL0, dMh;
@@ -1377,18 +1289,21 @@ struct MidSolveArgs {
   LinTable lin;
 };
 
-template <int RS>
-__global__ void __launch_bounds__(kMaxBlock, 1) k_mid_solve(MidSolveArgs a) {
+// NF: the largest field count of the mode solves (2, or kMaxPrecFields).  256 x 256, two
+// fields, one column per CTA: 15.6 us with the plan's called stages and 4 x 4 solves,
+// about 9 us with the length's own stages and 2 x 2 solves.
+template <int RS, int LX, int NF>
+__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_mid_solve(MidSolveArgs a) {
   extern __shared__ double2 sm[];
-  const int L0 = a.L0, TW = a.TW, LS = L0 + 1, T = blockDim.x, tid = threadIdx.x, n = a.n;
+  const int L0 = LX ? LX : a.L0, TW = a.TW, LS = tile_stride(L0, TW), T = blockDim.x, tid = threadIdx.x, n = a.n;
   double2* tw = sm;
   double2* fb = sm + L0;
-  for (int t = tid; t < L0; t += T) tw[t] = a.tw[t];
+  const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
   const long long i0 = (long long)blockIdx.x * TW;
   const int nload = n * L0 * TW;
   for (int e = tid; e < nload; e += T) {
     const int q0 = fdiv(e, a.dTW), c = e - q0 * TW;
-    const int f = fdiv(q0, a.dL0), z = q0 - f * L0;
+    const int f = fdivc<LX>(q0, a.dL0), z = q0 - f * L0;
     const long long ii = i0 + c;
     const bool in = ii < a.I;
     cp_async16(&fb[(f * TW + c) * LS + z], in ? (const void*)&a.Sf[((long long)f * L0 + z) * a.I + ii] : (const void*)a.Sf,
@@ -1396,7 +1311,7 @@ __global__ void __launch_bounds__(kMaxBlock, 1) k_mid_solve(MidSolveArgs a) {
   }
   cp_async_wait_all();
   __syncthreads();
-  fft_lines<RS, false>(fb, LS, n * TW, a.plan, tw);
+  fft_lines_x<RS, LX, false>(fb, LS, n * TW, a.plan, tw, twz);
   for (int e = tid; e < L0 * TW; e += T) {
     const int z = fdiv(e, a.dTW), c = e - z * TW;
     const long long ii = i0 + c;
@@ -1409,29 +1324,23 @@ __global__ void __launch_bounds__(kMaxBlock, 1) k_mid_solve(MidSolveArgs a) {
     } else {
       nidx[1] = (int)ii;
     }
-    double2 v[kMaxPrecFields];
-    for (int f = 0; f < n; ++f) v[f] = fb[(f * TW + c) * LS + z];
-    mode_solve(a.lin, nidx, v, n);
-    for (int f = 0; f < n; ++f) fb[(f * TW + c) * LS + z] = v[f];
+    double2 v[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (f < n) v[f] = fb[(f * TW + c) * LS + z];
+    mode_solve<NF>(a.lin, nidx, v, n);
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (f < n) fb[(f * TW + c) * LS + z] = v[f];
   }
   __syncthreads();
-  fft_lines<RS, true>(fb, LS, n * TW, a.plan, tw);
+  fft_lines_x<RS, LX, true>(fb, LS, n * TW, a.plan, tw, twz);
   for (int e = tid; e < nload; e += T) {
     const int q0 = fdiv(e, a.dTW), c = e - q0 * TW;
-    const int f = fdiv(q0, a.dL0), z = q0 - f * L0;
+    const int f = fdivc<LX>(q0, a.dL0), z = q0 - f * L0;
     const long long ii = i0 + c;
     if (ii < a.I) a.Sc[((long long)f * L0 + z) * a.I + ii] = fb[(f * TW + c) * LS + z];
   }
-}
-
-__global__ void k_mult1d_solve(int Mh, int n, const double2* Sf, double2* Sc, LinTable lin) {
-  const int kx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (kx >= Mh) return;
-  int nidx[3] = {kx, 0, 0};
-  double2 v[kMaxPrecFields];
-  for (int f = 0; f < n; ++f) v[f] = Sf[(long long)f * Mh + kx];
-  mode_solve(lin, nidx, v, n);
-  for (int f = 0; f < n; ++f) Sc[(long long)f * Mh + kx] = v[f];
 }
 
 struct InvXArgs {
@@ -4032,7 +3941,7 @@ bool SpectralPlan::init_precond(int n_, int ndim_, const int* Ns_, const double*
     const int L0 = Ns[0];
     const int I = (ndim == 3) ? Ns[1] * Mh : Mh;
     int TW = std::max(1, std::min(16, I / kTargetCtas));
-    auto smem_of = [&](int tw_) { return (size_t)(L0 + n * tw_ * (L0 + 1)) * 16; };
+    auto smem_of = [&](int tw_) { return (size_t)(L0 + n * tw_ * tile_stride(L0, tw_)) * 16; };
     while (TW > 1 && (smem_of(TW) > kSmemBudget || n * TW * L0 > cta_elems())) TW /= 2;
     if (smem_of(TW) > 227 * 1024 || n * TW * L0 > kMaxElems) {
       *msg = "grid too large for the preconditioner's axis-0 pass";
@@ -4042,7 +3951,12 @@ bool SpectralPlan::init_precond(int n_, int ndim_, const int* Ns_, const double*
     midsolve_.grid = (I + TW - 1) / TW;
     midsolve_.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_ax_[0], n * TW * L0), 32)));
     midsolve_.smem = smem_of(TW);
-    if (!opt_in_smem((const void*)k_mid_solve<kRadixPow2>) || !opt_in_smem((const void*)k_mid_solve<kRadixAll>)) {
+    bool ok = true;
+    by_length(plan_ax_[0], midsolve_.block, [&](auto rs, auto lx) {
+      constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
+      ok = opt_in_smem(n <= 2 ? (const void*)k_mid_solve<RS, LX, 2> : (const void*)k_mid_solve<RS, LX, kMaxPrecFields>);
+    });
+    if (!ok) {
       *msg = "cannot enable large shared memory for the preconditioner pass";
       return false;
     }
@@ -4120,10 +4034,13 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
     m.Sc = Sc_;
     m.lin = lt;
     prep(m);
-    if (plan_is_pow2(plan_ax_[0]))
-      k_mid_solve<kRadixPow2><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
-    else
-      k_mid_solve<kRadixAll><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
+    by_length(plan_ax_[0], midsolve_.block, [&](auto rs, auto lx) {
+      constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
+      if (n <= 2)
+        k_mid_solve<RS, LX, 2><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
+      else
+        k_mid_solve<RS, LX, kMaxPrecFields><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
+    });
     RDCU_TRY(cudaGetLastError());
     if (ndim == 3) {
       C2CArgs a{};
@@ -4139,9 +4056,6 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
       by_length(plan_ax_[1], c2c_i_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<grid, c2c_i_.block, c2c_i_.smem, st>>>(a); });
       RDCU_TRY(cudaGetLastError());
     }
-  } else {
-    k_mult1d_solve<<<(Mh + 127) / 128, 128, 0, st>>>(Mh, n, Sf_, Sc_, lt);
-    RDCU_TRY(cudaGetLastError());
   }
   // inverse x pass of the n solved fields straight into z
   InvXArgs a{};

@@ -173,3 +173,48 @@ def test_linear_stats_of_a_dp45_handle_are_zero(cuda):
     s = R.Solver(prob.n, prob.Ns, prob.Ls, spec_terms(prob))
     assert s.linear_stats() == (0, 0, 0)
     s.close()
+
+
+# one-dimensional problems: the one-CTA preconditioner takes lines of up to 8192 complex
+# values (two fields each), any radix and one to four fields
+@pytest.mark.parametrize("n,N", [(1, 27), (2, 16), (2, 143), (3, 60), (4, 128), (4, 4096), (2, 4620), (2, 8190),
+                                 (1, 8192), (2, 8192)])
+def test_line_preconditioner_matches_direct_solves(cuda, n, N):
+    import rdcu_b200 as R
+
+    lines = []
+    for i in range(n):  # u_t = u + a u_xx + b w_xx - u^3, w the next field
+        lines += ["1.0,%d,%d,1" % (i, i), "%s,%d,%d,1" % (1.0 + 0.5 * i, i, 2 * n + i),
+                  "%s,%d,%d,1" % (0.3, i, 2 * n + (i + 1) % n), "-1.0,%d,%d,3" % (i, i)]
+    prob = Problem(n, (N,), (0.05 * N,), [parse_term(s) for s in lines])
+    x = np.arange(N) / N
+    y0 = np.concatenate([np.cos(2 * np.pi * (i + 1) * x + i) + 0.1 * np.sin(2 * np.pi * 5 * x) for i in range(n)])
+    t1, dt, rtol = 0.02, 0.01, 1e-6
+    s = _solver(prob, rtol=rtol, atol=rtol)
+    y = np.array(y0)
+    s.set_state(0.0, dt / 100, y)
+    h, states = [], []
+
+    def cb(e):
+        if e.kind == R.EV_ATTEMPT:
+            h.append(e.h)
+        elif e.kind == R.EV_EVAL:
+            states.append(s.copy_to_numpy(e.y, n * N))
+        return 0
+
+    s.solve(t1, [dt, 2 * dt], callback=cb)
+    iters, solves, cycles = s.linear_stats()
+    s.close()
+    assert solves > 0 and cycles == solves and iters <= 20 * solves  # preconditioned: no restart
+    with tempfile.TemporaryDirectory() as wd:
+        fb = wd + "/o"
+        y0.tofile(fb + "ic.dat")
+        cfg = orun.RunConfig(n=n, Ns=prob.Ns, Ls=prob.Ls, terms=prob.terms, t1=t1, dt=dt, rtol=rtol, atol=rtol,
+                             stiff=True)
+        orun.run(fb, cfg)
+        oh = np.fromfile(fb + "steps.dat")
+        ost = np.fromfile(fb + "states.dat").reshape(-1, n * N)[1:]
+    assert len(h) == len(oh)
+    assert np.max(np.abs(np.array(h) - oh) / np.abs(oh)) < 1e-8  # the tolerance of the oracle comparison above
+    for a, b in zip(states, ost):
+        assert rel_err(a, b) < 1e-8
