@@ -124,6 +124,12 @@ __global__ void k_scale(const double* x, double s, double* y, long long nN) {
   if (i < nN) y[i] = s * x[i];
 }
 
+// V_0 = out = s x
+__global__ void k_first_vector(const double* x, double s, double* V, double* out, long long nN) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nN) V[i] = out[i] = s * x[i];
+}
+
 __global__ void k_axpy(double a, const double* x, double* y, long long nN) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nN) y[i] += a * x[i];
@@ -145,23 +151,30 @@ __global__ void k_residual(const int* rows, const int* cols, const double* vals,
 // device: the column j, alpha, the Givens factors, g and the Hessenberg matrix.  The
 // scalar update uses round-to-nearest intrinsics without contraction, so every value
 // is the one the same recurrence gives on the host.
+//
+// An iteration is the preconditioner and four kernels.  The vectors (1 MB each at 256^2,
+// two fields) stay in L2, so an iteration is bound by the latency of its launches and
+// reductions, not by bandwidth: each kernel does all that one grid-wide reduction allows
+// (A z with the first Gram-Schmidt products; subtraction with the second products;
+// subtraction with the norm; Givens update with the next basis vector), and a reduction's
+// partial sums (one per block) are added up by every block of the next kernel, in the same
+// order, instead of by a last block behind a fence.  Brusselator 256^2, per iteration
+// without the preconditioner: 36 us in eight launches before, 20 us in four.
 constexpr int kGmresM = 40;  // restart length m
 
 struct GmresState {
   double alpha;   // A = I + alpha J
   double tol;     // absolute residual target
-  double inv_hn;  // 1 / ||w|| of the last column: scale of the next basis vector
-  int j;          // column being built
+  int jn;         // column of the next iteration (written by its last kernel)
+  int j;          // column being built (jn, copied by its first kernel)
   int jdone;      // columns done
   int total;      // iterations over all cycles of this solve
   int max_total;
   int cont;       // the loop goes on (the next basis vector was formed)
   int conv;
   int guard;      // iterations of this cycle: bounds the loop whatever j does
-  int pad;
   double cs[kGmresM], sn[kGmresM], g[kGmresM + 1];
   double H[kGmresM * kGmresM];  // H[k * m + j], k <= j
-  double y[kGmresM];            // least-squares solution (back-substitution)
 };
 
 __global__ void k_gm_init(GmresState* s, double alpha, double tol, double beta, int total, int max_total) {
@@ -169,8 +182,7 @@ __global__ void k_gm_init(GmresState* s, double alpha, double tol, double beta, 
   if (threadIdx.x == 0) {
     s->alpha = alpha;
     s->tol = tol;
-    s->inv_hn = 0.0;
-    s->j = 0;
+    s->j = s->jn = 0;
     s->jdone = 0;
     s->total = total;
     s->max_total = max_total;
@@ -180,136 +192,241 @@ __global__ void k_gm_init(GmresState* s, double alpha, double tol, double beta, 
   }
 }
 
-// Start of iteration j: for j > 0, V_j = w / ||w|| from the previous iteration (the
-// scaling k_scale did); out = V_j, the preconditioner's input.
-__global__ void k_gm_take(double* V, const GmresState* s, const double* w, double* out, long long nN) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
-  const int j = s->j;
-  double v;
-  if (j > 0) {
-    v = s->inv_hn * w[i];
-    V[(long long)j * nN + i] = v;
-  } else {
-    v = V[i];
-  }
-  out[i] = v;
+constexpr int kArnThreads = 512;
+constexpr int kArnWarps = kArnThreads / 32;
+constexpr int kArnBlocks = 148;  // one per SM: also the number of partials every block adds up
+constexpr int kArnElems = 4;     // elements a thread holds at a time
+
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-// y = x + alpha * (J x), alpha read on the device: the action of A = I + alpha J
-// (csrgeam2 of bdf.cu:153)
-__global__ void k_apply_A_dev(const int* rows, const int* cols, const double* vals, const double* alpha,
-                              const double* x, double* y, long long nN) {
-  const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nN) return;
-  const double al = *alpha;
-  double acc = 0.0;
-  for (int p = rows[r]; p < rows[r + 1]; ++p) acc += vals[p] * x[cols[p]];
-  y[r] = x[r] + al * acc;
-}
-
-// k_dots then k_sum_rows over the j + 1 basis vectors (nvec < 0: j + 1 read on the
-// device; rows past it return) in one launch: the last block of each row to finish
-// sums that row's partials with the threads and order of k_sum_rows (bitwise the
-// same), then clears the row's arrival count.
-__global__ void k_dots_sum(const double* V, const GmresState* s, int nvec, const double* w, long long nN,
-                           double* part, unsigned int* count, double* out) {
-  if (nvec < 0) nvec = s->j + 1;
-  const int row = blockIdx.y;
-  if (row > nvec) return;
-  const double* a = row < nvec ? V + (long long)row * nN : w;
-  double sum = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x)
-    sum += a[i] * w[i];
-  sum = block_reduce(sum);
-  __shared__ int last;
-  if (threadIdx.x == 0) {
-    part[(long long)row * gridDim.x + blockIdx.x] = sum;
-    __threadfence();
-    last = atomicAdd(&count[row], 1u) == gridDim.x - 1;
+// h[0..nrow) = the sums of the rows of part[row][gridDim.x], one warp per row, in the same
+// order in every block; ends with a barrier
+__device__ __forceinline__ void sum_partials(const double* part, int nrow, double* h) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = gridDim.x;
+  for (int k = warp; k < nrow; k += kArnWarps) {
+    double t = 0.0;
+    for (int c = lane; c < nb; c += 32) t += part[(long long)k * nb + c];
+    t = warp_sum(t);
+    if (lane == 0) h[k] = t;
   }
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double t = 0.0;
-  for (int c = threadIdx.x; c < (int)gridDim.x; c += blockDim.x) t += __ldcg(&part[(long long)row * gridDim.x + c]);
-  t = block_reduce(t);
-  if (threadIdx.x == 0) {
-    out[row] = t;
-    count[row] = 0u;
+}
+
+// Adds this chunk's products V_k . w (k < nvec) of the thread's elements to the warp's
+// sums red[warp][k] (first: sets them).  Four basis vectors at a time keep as many loads
+// in flight.
+__device__ __forceinline__ void add_dots(const double* V, long long nN, int nvec, const long long (&i)[kArnElems],
+                                         const double (&w)[kArnElems], double (*red)[kGmresM + 1], bool first) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k0 = 0; k0 < nvec; k0 += 4) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k0 + q < nvec) {
+#pragma unroll
+        for (int e = 0; e < kArnElems; ++e)
+          if (i[e] < nN) acc[q] += V[(long long)(k0 + q) * nN + i[e]] * w[e];
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (k0 + q < nvec) red[warp][k0 + q] = first ? acc[q] : red[warp][k0 + q] + acc[q];
   }
 }
 
-__global__ void k_vsub_j(const double* V, const GmresState* s, const double* h, double* w, long long nN) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
+// the block's sums over its warps, one partial per row
+__device__ __forceinline__ void put_partials(double (*red)[kGmresM + 1], int nvec, double* part) {
+  __syncthreads();
+  for (int k = threadIdx.x; k < nvec; k += kArnThreads) {
+    double t = 0.0;
+    for (int w = 0; w < kArnWarps; ++w) t += red[w][k];
+    part[(long long)k * gridDim.x + blockIdx.x] = t;
+  }
+}
+
+// The elements of a thread: chunk c, element e.
+#define RDCU_ARN_CHUNKS(c, i, nN)                                                        \
+  const long long arn_span = (long long)gridDim.x * kArnThreads;                         \
+  const long long arn_i0 = (long long)blockIdx.x * kArnThreads + threadIdx.x;            \
+  long long i[kArnElems];                                                                \
+  for (long long c = 0; c * kArnElems * arn_span < (nN); ++c)
+
+// w = A z = z + alpha (J z) (csrgeam2 of bdf.cu:153) and the products V_k . w, k <= j
+__global__ void __launch_bounds__(kArnThreads, 1) k_arn_apply(const int* rows, const int* cols, const double* vals,
+                                                              GmresState* s, const double* z, double* w,
+                                                              const double* V, long long nN, double* part) {
+  __shared__ double red[kArnWarps][kGmresM + 1];
+  const int j = s->jn;
+  if (blockIdx.x == 0 && threadIdx.x == 0) s->j = j;
+  const double al = s->alpha;
+  RDCU_ARN_CHUNKS(c, i, nN) {
+    double wv[kArnElems];
+#pragma unroll
+    for (int e = 0; e < kArnElems; ++e) {
+      i[e] = arn_i0 + (c * kArnElems + e) * arn_span;
+      wv[e] = 0.0;
+      if (i[e] < nN) {
+        double acc = 0.0;
+        const int p1 = rows[i[e] + 1];
+        for (int p = rows[i[e]]; p < p1; p += 4) {  // four gathers in flight, summed in order
+          double t[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) t[q] = p + q < p1 ? vals[p + q] * z[cols[p + q]] : 0.0;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc += t[q];
+        }
+        wv[e] = z[i[e]] + al * acc;
+        w[i[e]] = wv[e];
+      }
+    }
+    add_dots(V, nN, j + 1, i, wv, red, c == 0);
+  }
+  put_partials(red, j + 1, part);
+}
+
+// First Gram-Schmidt subtraction, w -= sum_k h_k V_k with h the sums of part_in (kept in
+// dots), and the products V_k . w of what is left; NORM: the second subtraction, and w . w
+template <bool NORM>
+__global__ void __launch_bounds__(kArnThreads, 1) k_arn_sub(const double* V, const GmresState* s, const double* part_in,
+                                                            double* dots, double* w, long long nN, double* part) {
+  __shared__ double red[kArnWarps][kGmresM + 1];
+  __shared__ double h[kGmresM + 1];
   const int nvec = s->j + 1;
-  double acc = w[i];
-  for (int k = 0; k < nvec; ++k) acc -= h[k] * V[(long long)k * nN + i];
-  w[i] = acc;
+  sum_partials(part_in, nvec, h);
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < nvec; k += kArnThreads) dots[k] = h[k];
+  double ss = 0.0;
+  RDCU_ARN_CHUNKS(c, i, nN) {
+    double wv[kArnElems];
+#pragma unroll
+    for (int e = 0; e < kArnElems; ++e) {
+      i[e] = arn_i0 + (c * kArnElems + e) * arn_span;
+      wv[e] = i[e] < nN ? w[i[e]] : 0.0;
+    }
+#pragma unroll 4
+    for (int k = 0; k < nvec; ++k) {
+      const double hk = h[k];
+#pragma unroll
+      for (int e = 0; e < kArnElems; ++e)
+        if (i[e] < nN) wv[e] -= hk * V[(long long)k * nN + i[e]];
+    }
+#pragma unroll
+    for (int e = 0; e < kArnElems; ++e)
+      if (i[e] < nN) {
+        w[i[e]] = wv[e];
+        if (NORM) ss += wv[e] * wv[e];
+      }
+    if (!NORM) add_dots(V, nN, nvec, i, wv, red, c == 0);
+  }
+  if (NORM) {
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = ss;
+    put_partials(red, 1, part);
+  } else {
+    put_partials(red, nvec, part);
+  }
 }
 
 // Column j of the Hessenberg matrix from the two Gram-Schmidt passes (dots rows 0 and
-// 1, stride `row`) and the norm of w (row 2); Givens rotations; stop test; the loop
-// condition.  One thread.
-__global__ void k_gm_update(GmresState* s, const double* dots, int row, cudaGraphConditionalHandle cond) {
-  if (threadIdx.x != 0) return;
+// 1, stride `row`) and the norm of w; Givens rotations; stop test; the loop condition (block
+// 0).  Every block: the next basis vector w / ||w|| into V_(j+1) and out, the next
+// iteration's preconditioner input.
+__global__ void __launch_bounds__(kArnThreads, 1) k_arn_next(GmresState* s, const double* dots, int row,
+                                                             const double* part, const double* w, double* V,
+                                                             double* out, long long nN,
+                                                             cudaGraphConditionalHandle cond) {
+  __shared__ double h[1];
+  __shared__ double hcol[kGmresM + 1], cs[kGmresM], sn[kGmresM];
   const int j = s->j;
-  double hcol[kGmresM + 1];
-  for (int k = 0; k <= j; ++k) hcol[k] = __dadd_rn(__dadd_rn(0.0, dots[k]), dots[row + k]);
-  const double hn = sqrt(dots[2 * row]);
-  const int total = s->total + 1;
-  s->total = total;
-  for (int k = 0; k < j; ++k) {
-    const double a = __dadd_rn(__dmul_rn(s->cs[k], hcol[k]), __dmul_rn(s->sn[k], hcol[k + 1]));
-    hcol[k + 1] = __dadd_rn(__dmul_rn(-s->sn[k], hcol[k]), __dmul_rn(s->cs[k], hcol[k + 1]));
-    hcol[k] = a;
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k <= j; k += kArnThreads) {
+      hcol[k] = __dadd_rn(__dadd_rn(0.0, dots[k]), dots[row + k]);
+      if (k < j) {
+        cs[k] = s->cs[k];
+        sn[k] = s->sn[k];
+      }
+    }
+  sum_partials(part, 1, h);  // (its barrier also orders the loads above)
+  const double hn = sqrt(h[0]);
+  if (hn > 0) {
+    const double inv = 1.0 / hn;
+    double* Vn = V + (long long)(j + 1) * nN;
+    for (long long i = (long long)blockIdx.x * kArnThreads + threadIdx.x; i < nN; i += (long long)gridDim.x * kArnThreads) {
+      const double v = inv * w[i];
+      Vn[i] = v;
+      out[i] = v;
+    }
   }
-  const double den = sqrt(__dadd_rn(__dmul_rn(hcol[j], hcol[j]), __dmul_rn(hn, hn)));
-  const double c = den > 0 ? hcol[j] / den : 1.0;
-  const double sj = den > 0 ? hn / den : 0.0;
-  s->cs[j] = c;
-  s->sn[j] = sj;
-  hcol[j] = den;
-  const double gj = s->g[j];
-  s->g[j + 1] = __dmul_rn(-sj, gj);
-  s->g[j] = __dmul_rn(c, gj);
-  for (int k = 0; k <= j; ++k) s->H[k * kGmresM + j] = hcol[k];
-  s->jdone = j + 1;
-  const bool met = fabs(s->g[j + 1]) <= s->tol || !(hn > 0);
-  const bool stop = met || total >= s->max_total;
-  s->conv = met ? 1 : 0;
-  const int guard = s->guard + 1;
-  s->guard = guard;
-  const int cont = (!stop && j + 1 < kGmresM && guard < kGmresM) ? 1 : 0;
-  s->cont = cont;
-  if (cont) {
-    s->inv_hn = 1.0 / hn;
-    s->j = j + 1;
+  if (blockIdx.x != 0) return;
+  if (threadIdx.x == 0) {
+    const int total = s->total + 1;
+    s->total = total;
+    for (int k = 0; k < j; ++k) {
+      const double a = __dadd_rn(__dmul_rn(cs[k], hcol[k]), __dmul_rn(sn[k], hcol[k + 1]));
+      hcol[k + 1] = __dadd_rn(__dmul_rn(-sn[k], hcol[k]), __dmul_rn(cs[k], hcol[k + 1]));
+      hcol[k] = a;
+    }
+    const double den = sqrt(__dadd_rn(__dmul_rn(hcol[j], hcol[j]), __dmul_rn(hn, hn)));
+    const double c = den > 0 ? hcol[j] / den : 1.0;
+    const double sj = den > 0 ? hn / den : 0.0;
+    s->cs[j] = c;
+    s->sn[j] = sj;
+    hcol[j] = den;
+    const double gj = s->g[j];
+    const double gn = __dmul_rn(-sj, gj);
+    s->g[j + 1] = gn;
+    s->g[j] = __dmul_rn(c, gj);
+    s->jdone = j + 1;
+    const bool met = fabs(gn) <= s->tol || !(hn > 0);
+    const bool stop = met || total >= s->max_total;
+    s->conv = met ? 1 : 0;
+    const int guard = s->guard + 1;
+    s->guard = guard;
+    const int cont = (!stop && j + 1 < kGmresM && guard < kGmresM) ? 1 : 0;
+    s->cont = cont;
+    if (cont) s->jn = j + 1;
+    cudaGraphSetConditional(cond, (unsigned int)cont);
   }
-  cudaGraphSetConditional(cond, (unsigned int)cont);
+  __syncthreads();
+  for (int k = threadIdx.x; k <= j; k += kArnThreads) s->H[k * kGmresM + j] = hcol[k];
 }
 
-// back-substitution H y = g over the columns done (one thread)
-__global__ void k_gm_backsub(GmresState* s) {
-  if (threadIdx.x != 0) return;
+// u = sum_{k < jdone} y_k V_k, y from the back-substitution H y = g over the columns done
+// (by every block: one warp, a row per lane, a column at a time)
+__global__ void __launch_bounds__(kArnThreads, 1) k_gm_solution(const double* V, const GmresState* s, double* u,
+                                                                long long nN) {
+  __shared__ double H[kGmresM * kGmresM];
+  __shared__ double y[kGmresM];
   const int jd = s->jdone;
-  for (int k = jd - 1; k >= 0; --k) {
-    double acc = s->g[k];
-    for (int q = k + 1; q < jd; ++q) acc = __dsub_rn(acc, __dmul_rn(s->H[k * kGmresM + q], s->y[q]));
-    const double d = s->H[k * kGmresM + k];
-    s->y[k] = d != 0 ? acc / d : 0.0;
+  for (int t = threadIdx.x; t < jd * jd; t += kArnThreads) {
+    const int k = t / jd, q = t - k * jd;
+    H[k * kGmresM + q] = q >= k ? s->H[k * kGmresM + q] : 0.0;
   }
-}
-
-// u = sum_{k < jdone} y_k V_k
-__global__ void k_vcomb_j(const double* V, const GmresState* s, double* u, long long nN) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
-  const int nvec = s->jdone;
-  double acc = 0.0;
-  for (int k = 0; k < nvec; ++k) acc += s->y[k] * V[(long long)k * nN + i];
-  u[i] = acc;
+  for (int k = threadIdx.x; k < jd; k += kArnThreads) y[k] = s->g[k];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    for (int k = jd - 1; k >= 0; --k) {
+      const double d = H[k * kGmresM + k];
+      const double yk = d != 0 ? y[k] / d : 0.0;
+      __syncwarp();
+      for (int q = threadIdx.x; q <= k; q += 32) y[q] = q == k ? yk : y[q] - H[q * kGmresM + k] * yk;
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (long long i = (long long)blockIdx.x * kArnThreads + threadIdx.x; i < nN; i += (long long)gridDim.x * kArnThreads) {
+    double acc = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < jd; ++k) acc += y[k] * V[(long long)k * nN + i];
+    u[i] = acc;
+  }
 }
 
 // ytemp += dd; d += dd (the two Daxpy of bdf.cu:187-188)
@@ -370,14 +487,15 @@ struct NewtonCtl {
   double hh;         // step size
   double coef;       // (1 - kappa_k) gamma_k of the order
   double alpha_new;  // -hh / coef: alpha after a refactorisation
-  double gam[6];     // gamma_j
+  double hc;         // hh / coef
+  double gc[6];      // gamma_j / coef
   int order;
   int refactor;      // a refactorisation is due (cleared when done)
   // persistent
   double alpha;      // alpha of the current "factorisation"
   // loop state
   double dnorm, dnormold, rate, beta, tol;
-  int it, converged, update, restart, proceed, total;
+  int it, converged, update, newton_cont, restart, proceed, total;
   // results
   double errsq;  // sum of (d / yscale)^2 after the loop
   long long lin_iters, lin_cycles, lin_solves;
@@ -388,7 +506,8 @@ __global__ void k_newton_arm(NewtonCtl* c, double hh, double coef, double alpha_
   c->hh = hh;
   c->coef = coef;
   c->alpha_new = alpha_new;
-  for (int j = 0; j < 6; ++j) c->gam[j] = gam.v[j];
+  c->hc = hh / coef;
+  for (int j = 0; j < 6; ++j) c->gc[j] = gam.v[j] / coef;
   c->order = order;
   if (refactor) c->refactor = 1;
   c->lin_iters = 0;
@@ -407,36 +526,10 @@ __global__ void k_newton_start(NewtonCtl* c, cudaGraphConditionalHandle cond) {
   cudaGraphSetConditional(cond, 1u);
 }
 
-// start of an iteration: the refactorisation's alpha (bdf.cu:152-156)
-__global__ void k_newton_begin(NewtonCtl* c) {
-  if (c->refactor) {
-    c->alpha = c->alpha_new;
-    c->refactor = 0;
-  }
-}
-
-// k_newton_rhs with the order, h and coefficients of the record
-__global__ void k_newton_rhs_dev(double* b, const double* f, const double* d, const double* D, long long nN,
-                                 const NewtonCtl* c) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
-  const int order = c->order;
-  const double h = c->hh, alpha = c->coef;
-  double v = h / alpha * f[i];
-  for (int j = 1; j <= order; ++j) v -= D[nN * j + i] * c->gam[j] / alpha;
-  v -= d[i];
-  b[i] = v;
-}
-
-// k_wsq then k_sum_rows in one launch (k_dots_sum's last-block pattern, bitwise the
-// same sums): out[0] = sum of (x / yscale)^2
-__global__ void k_wsq_sum(const double* x, const double* yscale, long long nN, double* part, unsigned int* count,
-                          double* out) {
-  double sum = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x) {
-    const double v = x[i] / yscale[i];
-    sum += v * v;
-  }
+// The block's sum joins the others (block_reduce's value in thread 0); true in the block
+// that arrives last, whose thread 0 then has the total (every partial in k_sum_rows' order).
+// The count is left at zero.
+__device__ __forceinline__ bool last_block_sum(double sum, double* part, unsigned int* count, double* total) {
   sum = block_reduce(sum);
   __shared__ int last;
   if (threadIdx.x == 0) {
@@ -445,91 +538,32 @@ __global__ void k_wsq_sum(const double* x, const double* yscale, long long nN, d
     last = atomicAdd(count, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
   double t = 0.0;
   for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) t += __ldcg(&part[q]);
   t = block_reduce(t);
-  if (threadIdx.x == 0) {
-    out[0] = t;
-    *count = 0u;
+  if (threadIdx.x == 0) *count = 0u;
+  *total = t;
+  return true;
+}
+
+// out[0] = sum of (x / yscale)^2
+__global__ void k_wsq_sum(const double* x, const double* yscale, long long nN, double* part, unsigned int* count,
+                          double* out) {
+  double sum = 0.0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x) {
+    const double v = x[i] / yscale[i];
+    sum += v * v;
   }
+  double t;
+  if (last_block_sum(sum, part, count, &t) && threadIdx.x == 0) out[0] = t;
 }
 
-// start of a linear solve (gmres): beta0 = ||b||, the tolerance, the restart loop's
-// condition (no restart when b = 0: x stays 0)
-__global__ void k_solve_begin(NewtonCtl* c, const double* bb, double lin_tol, cudaGraphConditionalHandle cond) {
-  const double beta0 = sqrt(bb[0]);
-  c->beta = beta0;
-  c->tol = lin_tol * beta0;
-  c->total = 0;
-  c->restart = 0;
-  c->proceed = 0;
-  c->lin_solves += 1;
-  cudaGraphSetConditional(cond, beta0 > 0 ? 1u : 0u);
-}
-
-// r = b - A x from the second restart on
-__global__ void k_residual_dev(const int* rows, const int* cols, const double* vals, const NewtonCtl* c,
-                               const double* x, const double* b, double* r, long long nN) {
-  if (c->restart == 0) return;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
-  const double alpha = c->alpha;
-  double acc = 0.0;
-  for (int p = rows[i]; p < rows[i + 1]; ++p) acc += vals[p] * x[cols[p]];
-  r[i] = b[i] - (x[i] + alpha * acc);
-}
-
-// restart test (beta = ||r|| > tol from the second restart on), V_0 = r / beta and the
-// cycle's GMRES state (k_gm_init); the Arnoldi loop runs only when the cycle goes on
-__global__ void k_restart_begin(NewtonCtl* c, GmresState* s, const double* rr, int max_total,
-                                cudaGraphConditionalHandle cond) {
-  if (c->restart > 0) c->beta = sqrt(rr[0]);
-  const int proceed = (c->restart == 0 || c->beta > c->tol) ? 1 : 0;
-  c->proceed = proceed;
-  for (int k = 0; k <= kGmresM; ++k) s->g[k] = k == 0 ? c->beta : 0.0;
-  s->alpha = c->alpha;
-  s->tol = c->tol;
-  s->inv_hn = 0.0;
-  s->j = 0;
-  s->jdone = 0;
-  s->total = c->total;
-  s->max_total = max_total;
-  s->cont = 0;
-  s->conv = 0;
-  s->guard = 0;
-  if (proceed) c->lin_cycles += 1;
-  cudaGraphSetConditional(cond, (unsigned)proceed);
-}
-
-// V_0 = (1 / beta) * (b on the first restart, else r)
-__global__ void k_scale_dev(const NewtonCtl* c, const double* b, const double* r, double* V, long long nN) {
-  if (!c->proceed) return;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
-  const double s = 1.0 / c->beta;
-  V[i] = s * (c->restart == 0 ? b[i] : r[i]);
-}
-
-// end of a restart: iterations so far, convergence, the restart loop's condition
-__global__ void k_restart_end(NewtonCtl* c, const GmresState* s, int max_total, cudaGraphConditionalHandle cond) {
-  int cont = 0;
-  if (c->proceed) {
-    c->total = s->total;
-    c->restart += 1;
-    cont = (!s->conv && c->restart < 50 && c->total < max_total) ? 1 : 0;
-  }
-  cudaGraphSetConditional(cond, (unsigned)cont);
-}
-
-__global__ void k_solve_end(NewtonCtl* c) { c->lin_iters += c->total; }
-
-// Newton convergence tests (bdf.cu:168-183) on ||dd|| (weighted RMS): stop, converge,
+// Newton convergence tests (bdf.cu:168-183) on the sum of (dd / yscale)^2: stop, converge,
 // or apply the correction and go on
-__global__ void k_newton_ctl(NewtonCtl* c, const double* ss, double sqN, double ntol, int nwit,
-                             cudaGraphConditionalHandle cond) {
-  const double dnorm = sqrt(ss[0]) / sqN;
+__device__ __forceinline__ void newton_test(NewtonCtl* c, double ss, double sqN, double ntol, int nwit) {
+  const double dnorm = sqrt(ss) / sqN;
   c->dnorm = dnorm;
   const double dnormold = c->dnormold;
   double rate = c->rate;
@@ -552,21 +586,145 @@ __global__ void k_newton_ctl(NewtonCtl* c, const double* ss, double sqN, double 
     c->it = it + 1;
     cont = it + 1 < nwit ? 1 : 0;
   }
+  c->newton_cont = cont;
+}
+
+// Start of a linear solve: b (the rhs kernel of bdf.cu:104-113, with the order, h and
+// coefficients of the record), x = 0 and, in the last block, the refactorisation's alpha
+// (bdf.cu:152-156), beta0 = ||b||, the tolerance and the restart loop's condition.  b = 0: no
+// restart, x stays 0 and the Newton test runs here.
+__global__ void __launch_bounds__(kRedThreads) k_solve_begin(double* b, double* x, const double* f, const double* d,
+                                                             const double* D, long long nN, NewtonCtl* c,
+                                                             double* part, unsigned int* count, double lin_tol,
+                                                             double sqN, double ntol, int nwit,
+                                                             cudaGraphConditionalHandle cond) {
+  const int order = c->order;
+  const double hc = c->hc;
+  double gc[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) gc[j] = c->gc[j];
+  double sum = 0.0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x) {
+    double v = hc * f[i];
+#pragma unroll
+    for (int j = 1; j < 6; ++j)
+      if (j <= order) v -= D[nN * j + i] * gc[j];
+    v -= d[i];
+    b[i] = v;
+    x[i] = 0.0;
+    sum += v * v;
+  }
+  double bb;
+  if (!last_block_sum(sum, part, count, &bb) || threadIdx.x != 0) return;
+  if (c->refactor) {
+    c->alpha = c->alpha_new;
+    c->refactor = 0;
+  }
+  const double beta0 = sqrt(bb);
+  c->beta = beta0;
+  c->tol = lin_tol * beta0;
+  c->total = 0;
+  c->restart = 0;
+  c->proceed = 0;
+  c->lin_solves += 1;
+  if (!(beta0 > 0)) newton_test(c, 0.0, sqN, ntol, nwit);
+  cudaGraphSetConditional(cond, beta0 > 0 ? 1u : 0u);
+}
+
+// Start of a restart: from the second on r = b - A x and beta = ||r||; in the last block
+// the test (beta > tol), the cycle's GMRES state (k_gm_init) and the Arnoldi loop's
+// condition: it runs only when the cycle goes on
+__global__ void __launch_bounds__(kRedThreads) k_restart_begin(const int* rows, const int* cols, const double* vals,
+                                                               NewtonCtl* c, const double* x, const double* b,
+                                                               double* r, long long nN, double* part,
+                                                               unsigned int* count, GmresState* s, int max_total,
+                                                               cudaGraphConditionalHandle cond) {
+  const int restart = c->restart;
+  double rr = 0.0;
+  if (restart > 0) {
+    const double alpha = c->alpha;
+    double sum = 0.0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x) {
+      double acc = 0.0;
+      for (int p = rows[i]; p < rows[i + 1]; ++p) acc += vals[p] * x[cols[p]];
+      const double v = b[i] - (x[i] + alpha * acc);
+      r[i] = v;
+      sum += v * v;
+    }
+    if (!last_block_sum(sum, part, count, &rr)) return;
+  } else if (blockIdx.x != 0) {
+    return;
+  }
+  if (threadIdx.x != 0) return;
+  if (restart > 0) c->beta = sqrt(rr);
+  const int proceed = (restart == 0 || c->beta > c->tol) ? 1 : 0;
+  c->proceed = proceed;
+  s->g[0] = c->beta;
+  s->alpha = c->alpha;
+  s->tol = c->tol;
+  s->j = s->jn = 0;
+  s->jdone = 0;
+  s->total = c->total;
+  s->max_total = max_total;
+  s->cont = 0;
+  s->conv = 0;
+  s->guard = 0;
+  if (proceed) c->lin_cycles += 1;
+  cudaGraphSetConditional(cond, (unsigned)proceed);
+}
+
+// V_0 = out = (1 / beta) * (b on the first restart, else r)
+__global__ void k_first_vector_dev(const NewtonCtl* c, const double* b, const double* r, double* V, double* out,
+                                   long long nN) {
+  if (!c->proceed) return;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nN) return;
+  const double s = 1.0 / c->beta;
+  V[i] = out[i] = s * (c->restart == 0 ? b[i] : r[i]);
+}
+
+// End of a restart: x += z and the sum of (x / yscale)^2; in the last block the iterations
+// so far, convergence and the restart loop's condition, and at the end of the solve the
+// Newton tests
+__global__ void __launch_bounds__(kRedThreads) k_restart_end(const double* z, double* x, const double* yscale,
+                                                             long long nN, double* part, unsigned int* count,
+                                                             NewtonCtl* c, const GmresState* s, int max_total,
+                                                             double sqN, double ntol, int nwit,
+                                                             cudaGraphConditionalHandle cond) {
+  double sum = 0.0;
+  const bool add = s->jdone > 0;  // (no column was built: x is what it was)
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nN; i += (long long)gridDim.x * blockDim.x) {
+    double xv = x[i];
+    if (add) {
+      xv += z[i];
+      x[i] = xv;
+    }
+    const double v = xv / yscale[i];
+    sum += v * v;
+  }
+  double ss;
+  if (!last_block_sum(sum, part, count, &ss) || threadIdx.x != 0) return;
+  int cont = 0;
+  if (c->proceed) {
+    c->total = s->total;
+    c->restart += 1;
+    cont = (!s->conv && c->restart < 50 && c->total < max_total) ? 1 : 0;
+  }
+  if (!cont) {
+    c->lin_iters += c->total;
+    newton_test(c, ss, sqN, ntol, nwit);
+  }
   cudaGraphSetConditional(cond, (unsigned)cont);
 }
 
-// ytemp += dd; d += dd when the iteration goes on
-__global__ void k_newton_update_dev(const NewtonCtl* c, const double* dd, double* ytemp, double* d, long long nN) {
-  if (!c->update) return;
+// End of a Newton iteration: ytemp += dd; d += dd when it goes on; the Newton loop's condition
+__global__ void k_newton_update_dev(const NewtonCtl* c, const double* dd, double* ytemp, double* d, long long nN,
+                                    cudaGraphConditionalHandle cond) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nN) return;
+  if (i == 0) cudaGraphSetConditional(cond, (unsigned)c->newton_cont);
+  if (!c->update || i >= nN) return;
   ytemp[i] += dd[i];
   d[i] += dd[i];
-}
-
-__global__ void k_zero(double* x, long long nN) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nN) x[i] = 0.0;
 }
 
 // makeRU (bdf.cu:35-69)
@@ -615,14 +773,16 @@ struct BDFEngine::Impl {
   double *y_eval = nullptr, *w = nullptr, *z = nullptr, *vj = nullptr, *r = nullptr;
   double* V = nullptr;
   int m = kGmresM;
-  double* part = nullptr;   // [(m+2)][kRedBlocks]
+  int arn_blocks = 1, red_blocks = 1;  // grids of the Arnoldi kernels and of the solve's reductions
+  double* part = nullptr;   // two blocks of [(m+2)][kRedBlocks]
+  double* part2 = nullptr;  // the second of them
   double* dots = nullptr;   // 3 rows of [m+2] (device)
   double* hdots = nullptr;  // pinned
   // the restart cycle as a graph (build_cycle_graph), its device state and a pinned
   // copy of the state's header
   GmresState* gm = nullptr;
   GmresState* gm_host = nullptr;
-  unsigned int* arrivals = nullptr;  // per-row block counts of k_dots_sum (zero between launches)
+  unsigned int* arrivals = nullptr;  // block count of last_block_sum (zero between launches)
   cudaGraph_t cycle_graph = nullptr;
   cudaGraphExec_t cycle_exec = nullptr;
   double* cycle_x = nullptr;  // the solution vector the graph updates
@@ -630,7 +790,6 @@ struct BDFEngine::Impl {
   // pinned copy; newton_failed: the graph could not be built (host loop instead)
   NewtonCtl* nctl = nullptr;
   NewtonCtl* nctl_host = nullptr;
-  double* ndots = nullptr;  // ||b||^2, ||r||^2, ||dd||^2 (weighted) of the graph
   cudaGraph_t newton_graph = nullptr;
   cudaGraphExec_t newton_exec = nullptr;
   bool newton_failed = false;
@@ -708,18 +867,20 @@ bool BDFEngine::init(FDProblem* fd, double atol, double rtol, int fixed, cudaStr
   for (double** p : vecs)
     if (cudaMalloc((void**)p, sb) != cudaSuccess) return fail("BDF vectors");
   if (cudaMalloc((void**)&I.V, sb * (I.m + 1)) != cudaSuccess) return fail("GMRES basis");
-  if (cudaMalloc((void**)&I.part, sizeof(double) * (I.m + 2) * kRedBlocks) != cudaSuccess) return fail("reductions");
+  if (cudaMalloc((void**)&I.part, sizeof(double) * 2 * (I.m + 2) * kRedBlocks) != cudaSuccess) return fail("reductions");
+  I.part2 = I.part + (I.m + 2) * kRedBlocks;
+  I.arn_blocks = (int)std::max<long long>(1, std::min<long long>(kArnBlocks, (I.nN + kArnThreads - 1) / kArnThreads));
+  I.red_blocks = (int)std::max<long long>(1, std::min<long long>(kArnBlocks, (I.nN + kRedThreads - 1) / kRedThreads));
   // three rows of m+2: the two Gram-Schmidt passes and the new vector's norm
   if (cudaMalloc((void**)&I.dots, sizeof(double) * 3 * (I.m + 2)) != cudaSuccess) return fail("reductions");
   if (cudaMalloc((void**)&I.gm, sizeof(GmresState)) != cudaSuccess) return fail("GMRES state");
-  if (cudaMalloc((void**)&I.arrivals, sizeof(unsigned int) * (I.m + 2)) != cudaSuccess ||
-      cudaMemset(I.arrivals, 0, sizeof(unsigned int) * (I.m + 2)) != cudaSuccess)
+  if (cudaMalloc((void**)&I.arrivals, sizeof(unsigned int)) != cudaSuccess ||
+      cudaMemset(I.arrivals, 0, sizeof(unsigned int)) != cudaSuccess)
     return fail("GMRES state");
   if (cudaMallocHost((void**)&I.hdots, sizeof(double) * 3 * (I.m + 2)) != cudaSuccess) return fail("pinned");
   if (cudaMallocHost((void**)&I.gm_host, sizeof(GmresState)) != cudaSuccess) return fail("pinned");
   if (cudaMalloc((void**)&I.nctl, sizeof(NewtonCtl)) != cudaSuccess ||
-      cudaMemset(I.nctl, 0, sizeof(NewtonCtl)) != cudaSuccess ||
-      cudaMalloc((void**)&I.ndots, sizeof(double) * 4) != cudaSuccess)
+      cudaMemset(I.nctl, 0, sizeof(NewtonCtl)) != cudaSuccess)
     return fail("Newton state");
   if (cudaMallocHost((void**)&I.nctl_host, sizeof(NewtonCtl)) != cudaSuccess) return fail("pinned");
   device_bytes = sb * (8 + 11 + I.m + 1) + fd->device_bytes;
@@ -745,7 +906,6 @@ void BDFEngine::release() {
     if (I.newton_exec) cudaGraphExecDestroy(I.newton_exec);
     if (I.newton_graph) cudaGraphDestroy(I.newton_graph);
     if (I.nctl) cudaFree(I.nctl);
-    if (I.ndots) cudaFree(I.ndots);
     if (I.nctl_host) cudaFreeHost(I.nctl_host);
     double* vecs[] = {I.ytemp, I.yscale, I.f, I.d, I.dd, I.b, I.y_eval, I.w, I.z, I.vj, I.r, I.V, I.part, I.dots};
     for (double* p : vecs)
@@ -811,11 +971,30 @@ cudaError_t vdots(BDFEngine::Impl& I, int nvec, const double* w, cudaStream_t st
 
 }  // namespace
 
+// One Arnoldi iteration on st: z = P^-1 V_j (V_j in vj), w = A z, two classical Gram-Schmidt
+// passes, ||w||, the Givens update (which clears the loop condition `cond` on convergence,
+// after m columns or on the iteration limit) and V_(j+1).
+static cudaError_t arnoldi_iteration(BDFEngine::Impl& I, const FDProblem& fd, cudaGraphConditionalHandle cond,
+                                     cudaStream_t st) {
+  const long long nN = I.nN;
+  const int row = I.m + 2, g = I.arn_blocks;
+  if (I.have_prec) RDCU_TRY(I.precondition(I.vj, I.z, st));
+  k_arn_apply<<<g, kArnThreads, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, I.gm, I.have_prec ? I.z : I.vj, I.w, I.V, nN,
+                                         I.part);
+  k_arn_sub<false><<<g, kArnThreads, 0, st>>>(I.V, I.gm, I.part, I.dots, I.w, nN, I.part2);
+  k_arn_sub<true><<<g, kArnThreads, 0, st>>>(I.V, I.gm, I.part2, I.dots + row, I.w, nN, I.part);
+  k_arn_next<<<g, kArnThreads, 0, st>>>(I.gm, I.dots, row, I.part, I.w, I.V, I.vj, nN, cond);
+  return cudaGetLastError();
+}
+
+// z = P^-1 (V y): the correction of a restart cycle
+static cudaError_t cycle_solution(BDFEngine::Impl& I, double* z, cudaStream_t st) {
+  k_gm_solution<<<I.arn_blocks, kArnThreads, 0, st>>>(I.V, I.gm, I.have_prec ? I.w : z, I.nN);
+  return I.have_prec ? I.precondition(I.w, z, st) : cudaGetLastError();
+}
+
 // The GMRES(m) restart cycle as one CUDA graph: a WHILE node whose body is one Arnoldi
-// iteration -- V_j = w/||w|| of the previous iteration, z = P^-1 V_j, w = A z, two
-// classical Gram-Schmidt passes, ||w||, the Givens update (which clears the loop
-// condition on convergence, after m columns or on the iteration limit) -- then the
-// back-substitution and x += P^-1 (V y).  No host round trip per iteration: the host
+// iteration, then the back-substitution and x += P^-1 (V y).  No host round trip per iteration: the host
 // launches the graph once per cycle and reads back the state's header.
 static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, double* x, cudaStream_t st) {
   if (I.cycle_exec) cudaGraphExecDestroy(I.cycle_exec);
@@ -824,9 +1003,6 @@ static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, do
   I.cycle_graph = nullptr;
   const long long nN = I.nN;
   const int nb = I.blocks;
-  const int m = I.m;
-  const int row = m + 2;
-  const double* alpha_dev = &I.gm->alpha;
   cudaGraph_t graph = nullptr;
   RDCU_TRY(cudaGraphCreate(&graph, 0));
   cudaGraphConditionalHandle cond;
@@ -845,20 +1021,7 @@ static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, do
   // one Arnoldi iteration
   if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    cudaError_t el = cudaSuccess;
-    const double* zin = I.have_prec ? I.z : I.vj;
-    k_gm_take<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, I.vj, nN);
-    if (I.have_prec) el = I.precondition(I.vj, I.z, st);
-    k_apply_A_dev<<<nb, 256, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, alpha_dev, zin, I.w, nN);
-    for (int pass = 0; pass < 2; ++pass) {
-      k_dots_sum<<<dim3(kRedBlocks, m + 1), kRedThreads, 0, st>>>(I.V, I.gm, -1, I.w, nN, I.part, I.arrivals,
-                                                                  I.dots + pass * row);
-      k_vsub_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.dots + pass * row, I.w, nN);
-    }
-    k_dots_sum<<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(I.V, I.gm, 0, I.w, nN, I.part, I.arrivals,
-                                                            I.dots + 2 * row);
-    k_gm_update<<<1, 32, 0, st>>>(I.gm, I.dots, row, cond);
-    if (el == cudaSuccess) el = cudaGetLastError();
+    const cudaError_t el = arnoldi_iteration(I, fd, cond, st);
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(st, &captured);
     if (e == cudaSuccess) e = el;
@@ -866,15 +1029,8 @@ static cudaError_t build_cycle_graph(BDFEngine::Impl& I, const FDProblem& fd, do
   // after the loop: x += P^-1 (V y)
   if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(st, graph, &loop, nullptr, 1, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    cudaError_t el = cudaSuccess;
-    k_gm_backsub<<<1, 32, 0, st>>>(I.gm);
-    k_vcomb_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, nN);
-    if (I.have_prec) {
-      el = I.precondition(I.w, I.z, st);
-      k_axpy<<<nb, 256, 0, st>>>(1.0, I.z, x, nN);
-    } else {
-      k_axpy<<<nb, 256, 0, st>>>(1.0, I.w, x, nN);
-    }
+    cudaError_t el = cycle_solution(I, I.z, st);
+    k_axpy<<<nb, 256, 0, st>>>(1.0, I.z, x, nN);
     if (el == cudaSuccess) el = cudaGetLastError();
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(st, &captured);
@@ -917,7 +1073,7 @@ static cudaError_t gmres(BDFEngine::Impl& I, const FDProblem& fd, double alpha, 
       if (!(beta > tol)) break;
       r = I.r;
     }
-    k_scale<<<nb, 256, 0, st>>>(r, 1.0 / beta, I.V, nN);
+    k_first_vector<<<nb, 256, 0, st>>>(r, 1.0 / beta, I.V, I.vj, nN);
     k_gm_init<<<1, 64, 0, st>>>(I.gm, alpha, tol, beta, total, I.lin_max_iters);
     RDCU_TRY(cudaGetLastError());
     RDCU_TRY(cudaGraphLaunch(I.cycle_exec, st));
@@ -967,8 +1123,7 @@ static cudaError_t capture_into(cudaGraph_t g, cudaStream_t st, F&& fill) {
 // update }, then yscale at ytemp and ||d||^2 for the error test (bdf.cu:231-239).
 static cudaError_t build_newton_graph(BDFEngine::Impl& I, FDProblem& fd, const double* D, cudaStream_t st) {
   const long long nN = I.nN;
-  const int nb = I.blocks, m = I.m, row = m + 2;
-  const double* alpha_dev = &I.gm->alpha;
+  const int nb = I.blocks, rb = I.red_blocks;
   const double sqN = std::pow((double)nN, 0.5);
   double* x = I.dd;
   cudaGraph_t G = nullptr;
@@ -981,61 +1136,33 @@ static cudaError_t build_newton_graph(BDFEngine::Impl& I, FDProblem& fd, const d
       k_newton_start<<<1, 1, 0, st>>>(I.nctl, hn);
       RDCU_TRY(add_while_node(G, st, hn, &Bn));
       k_errscale<<<nb, 256, 0, st>>>(I.ytemp, nN, I.atl, I.rtl, I.yscale);
-      k_wsq_sum<<<kRedBlocks, kRedThreads, 0, st>>>(I.d, I.yscale, nN, I.part, I.arrivals, &I.nctl->errsq);
+      k_wsq_sum<<<rb, kRedThreads, 0, st>>>(I.d, I.yscale, nN, I.part, I.arrivals, &I.nctl->errsq);
       return cudaSuccess;
     });
   if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hr, Bn, 0, cudaGraphCondAssignDefault);
   if (e == cudaSuccess)
     e = capture_into(Bn, st, [&]() -> cudaError_t {
       RDCU_TRY(fd.rhs(I.ytemp, I.f, nullptr));
-      k_newton_begin<<<1, 1, 0, st>>>(I.nctl);
-      k_newton_rhs_dev<<<nb, 256, 0, st>>>(I.b, I.f, I.d, D, nN, I.nctl);
-      k_dots_sum<<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(I.V, I.gm, 0, I.b, nN, I.part, I.arrivals, I.ndots);
-      k_solve_begin<<<1, 1, 0, st>>>(I.nctl, I.ndots, I.lin_tol, hr);
-      k_zero<<<nb, 256, 0, st>>>(x, nN);
+      k_solve_begin<<<rb, kRedThreads, 0, st>>>(I.b, x, I.f, I.d, D, nN, I.nctl, I.part, I.arrivals, I.lin_tol, sqN,
+                                                I.ntol, kNwit, hr);
       RDCU_TRY(add_while_node(Bn, st, hr, &Br));
-      k_solve_end<<<1, 1, 0, st>>>(I.nctl);
-      k_wsq_sum<<<kRedBlocks, kRedThreads, 0, st>>>(x, I.yscale, nN, I.part, I.arrivals, I.ndots + 2);
-      k_newton_ctl<<<1, 1, 0, st>>>(I.nctl, I.ndots + 2, sqN, I.ntol, kNwit, hn);
-      k_newton_update_dev<<<nb, 256, 0, st>>>(I.nctl, x, I.ytemp, I.d, nN);
+      k_newton_update_dev<<<nb, 256, 0, st>>>(I.nctl, x, I.ytemp, I.d, nN, hn);
       return cudaSuccess;
     });
   if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&ha, Br, 0, cudaGraphCondAssignDefault);
   if (e == cudaSuccess)
     e = capture_into(Br, st, [&]() -> cudaError_t {
-      k_residual_dev<<<nb, 256, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, I.nctl, x, I.b, I.r, nN);
-      k_dots_sum<<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(I.V, I.gm, 0, I.r, nN, I.part, I.arrivals,
-                                                              I.ndots + 1);
-      k_restart_begin<<<1, 1, 0, st>>>(I.nctl, I.gm, I.ndots + 1, I.lin_max_iters, ha);
-      k_scale_dev<<<nb, 256, 0, st>>>(I.nctl, I.b, I.r, I.V, nN);
+      k_restart_begin<<<rb, kRedThreads, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, I.nctl, x, I.b, I.r, nN, I.part,
+                                                  I.arrivals, I.gm, I.lin_max_iters, ha);
+      k_first_vector_dev<<<nb, 256, 0, st>>>(I.nctl, I.b, I.r, I.V, I.vj, nN);
       RDCU_TRY(add_while_node(Br, st, ha, &Ba));
-      k_gm_backsub<<<1, 32, 0, st>>>(I.gm);
-      k_vcomb_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, nN);
-      if (I.have_prec) {
-        RDCU_TRY(I.precondition(I.w, I.z, st));
-        k_axpy<<<nb, 256, 0, st>>>(1.0, I.z, x, nN);
-      } else {
-        k_axpy<<<nb, 256, 0, st>>>(1.0, I.w, x, nN);
-      }
-      k_restart_end<<<1, 1, 0, st>>>(I.nctl, I.gm, I.lin_max_iters, hr);
+      RDCU_TRY(cycle_solution(I, I.z, st));
+      k_restart_end<<<rb, kRedThreads, 0, st>>>(I.z, x, I.yscale, nN, I.part, I.arrivals, I.nctl, I.gm, I.lin_max_iters,
+                                                sqN, I.ntol, kNwit, hr);
       return cudaSuccess;
     });
   if (e == cudaSuccess)
-    e = capture_into(Ba, st, [&]() -> cudaError_t {
-      const double* zin = I.have_prec ? I.z : I.vj;
-      k_gm_take<<<nb, 256, 0, st>>>(I.V, I.gm, I.w, I.vj, nN);
-      if (I.have_prec) RDCU_TRY(I.precondition(I.vj, I.z, st));
-      k_apply_A_dev<<<nb, 256, 0, st>>>(fd.rows_, fd.cols_, fd.vals_, alpha_dev, zin, I.w, nN);
-      for (int pass = 0; pass < 2; ++pass) {
-        k_dots_sum<<<dim3(kRedBlocks, m + 1), kRedThreads, 0, st>>>(I.V, I.gm, -1, I.w, nN, I.part, I.arrivals,
-                                                                    I.dots + pass * row);
-        k_vsub_j<<<nb, 256, 0, st>>>(I.V, I.gm, I.dots + pass * row, I.w, nN);
-      }
-      k_dots_sum<<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(I.V, I.gm, 0, I.w, nN, I.part, I.arrivals,
-                                                              I.dots + 2 * row);
-      k_gm_update<<<1, 32, 0, st>>>(I.gm, I.dots, row, ha);
-      return cudaSuccess;
-    });
+    e = capture_into(Ba, st, [&]() -> cudaError_t { return arnoldi_iteration(I, fd, ha, st); });
   if (e == cudaSuccess) e = cudaGraphInstantiate(&I.newton_exec, G, 0);
   if (e != cudaSuccess) {
     cudaGraphDestroy(G);

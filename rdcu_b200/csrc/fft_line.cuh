@@ -132,11 +132,10 @@ __device__ __forceinline__ int swz8(int i) { return i ^ ((i >> 3) & 7); }
 // inputs from swz8 positions (the stage after it).  twz: the twiddle table is stored at
 // swz8 positions (the span-8 stage reads twiddles r*kk*L/64 for kk = 0..7, which
 // otherwise share a bank group).  Values are unchanged.
-// ELEMS: values a thread stages (kStageElems; the one-CTA line kernels hold more).
-template <int R, bool INV, bool POW2, int SWZ = 0, int ELEMS = kStageElems>
+template <int R, bool INV, bool POW2, int SWZ = 0>
 __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines, int L, int Ns, FastDiv dm,
                                                FastDiv dns, const double2* tw, bool twz = false) {
-  constexpr int QMAX = (R >= ELEMS) ? 1 : (ELEMS / R);
+  constexpr int QMAX = (R >= kStageElems) ? 1 : (kStageElems / R);
   const int m = L / R;
   const int nb = nlines * m;
   const int T = blockDim.x;
@@ -182,10 +181,10 @@ __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines,
 // A stage of the runtime-planned transform as a called function: the plan's stage loop
 // then holds one stage's registers at a time (inlined, the union of every radix's
 // registers exceeds the budget and spills).
-template <int R, bool INV, bool POW2, int ELEMS = kStageElems>
+template <int R, bool INV, bool POW2>
 __device__ __noinline__ void stockham_stage_call(double2* buf, int LS, int nlines, int L, int Ns, FastDiv dm,
                                                  FastDiv dns, const double2* tw) {
-  stockham_stage<R, INV, POW2, 0, ELEMS>(buf, LS, nlines, L, Ns, dm, dns, tw);
+  stockham_stage<R, INV, POW2>(buf, LS, nlines, L, Ns, dm, dns, tw);
 }
 
 // Radix sets a kernel is compiled for: power-of-two lengths use radices 8, 4, 2 only
@@ -201,7 +200,7 @@ inline bool plan_is_pow2(const LinePlan& p) {
 
 // Full transform of nlines lines.  All threads of the block must call it; the data
 // must be visible (a barrier before the call).  Returns after a barrier.
-template <int RS, bool INV, int ELEMS = kStageElems>
+template <int RS, bool INV>
 __device__ void fft_lines(double2* buf, int LS, int nlines, const LinePlan& p, const double2* tw) {
   int Ns = 1;
   for (int s = 0; s < p.nstages; ++s) {
@@ -209,21 +208,21 @@ __device__ void fft_lines(double2* buf, int LS, int nlines, const LinePlan& p, c
     const FastDiv dm = p.div_m[s], dns = p.div_ns[s];
     if (RS == kRadixPow2) {
       if (R == 8)
-        stockham_stage_call<8, INV, true, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
+        stockham_stage_call<8, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
       else if (R == 4)
-        stockham_stage_call<4, INV, true, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
+        stockham_stage_call<4, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
       else
-        stockham_stage_call<2, INV, true, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
+        stockham_stage_call<2, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
     } else {
       switch (R) {
-        case 2: stockham_stage_call<2, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 3: stockham_stage_call<3, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 4: stockham_stage_call<4, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 5: stockham_stage_call<5, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 7: stockham_stage_call<7, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 8: stockham_stage_call<8, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 11: stockham_stage_call<11, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 13: stockham_stage_call<13, INV, false, ELEMS>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 2: stockham_stage_call<2, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 3: stockham_stage_call<3, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 4: stockham_stage_call<4, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 5: stockham_stage_call<5, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 7: stockham_stage_call<7, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 8: stockham_stage_call<8, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 11: stockham_stage_call<11, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        case 13: stockham_stage_call<13, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
         default: break;  // plans only contain the radices above
       }
     }

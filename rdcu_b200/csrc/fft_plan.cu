@@ -5,8 +5,8 @@
 
 namespace rdcu {
 
-bool make_line_plan(int L, LinePlan* p, int most) {
-  if (L < 1 || L > most) return false;
+bool make_line_plan(int L, LinePlan* p) {
+  if (L < 1 || L > kMaxLine) return false;
   p->L = L;
   p->nstages = 0;
   int rem = L;
@@ -50,6 +50,25 @@ void make_twiddles(int L, std::vector<double2>& tw) {
     }
     if (num == 0) { c = 1.0L; s = 0.0L; }
     tw[t] = make_double2((double)c, (double)(-s));
+  }
+}
+
+void set_lin_ops(const std::vector<LinEntry>& lin, LinTable* t) {
+  t->nops = 0;
+  for (const LinEntry& e : lin) {
+    int g = 0;
+    while (g < t->nops && !(t->op[g].nax == e.nax && (e.nax < 1 || t->op[g].ax0 == e.ax0) &&
+                            (e.nax < 2 || t->op[g].ax1 == e.ax1)))
+      ++g;
+    if (g == t->nops) {  // at most 1 + 3 + 9 operators exist
+      t->op[g].nax = e.nax;
+      t->op[g].ax0 = e.nax >= 1 ? e.ax0 : 0;
+      t->op[g].ax1 = e.nax >= 2 ? e.ax1 : 0;
+      for (auto& row : t->coef[g])
+        for (double& c : row) c = 0.0;
+      ++t->nops;
+    }
+    t->coef[g][e.row][e.src] += e.coef;
   }
 }
 

@@ -53,8 +53,7 @@ struct LinePlan {
   FastDiv div_ns[kMaxStages];  // span Ns before stage s
 };
 
-// false when L has another prime factor than 2..13 or is above `most`
-bool make_line_plan(int L, LinePlan* p, int most = kMaxLine);
+bool make_line_plan(int L, LinePlan* p);
 // exp(-2 pi i t / L) for t < L, rounded from long double.
 void make_twiddles(int L, std::vector<double2>& tw);
 
@@ -151,9 +150,14 @@ struct LinEntry {
 };
 constexpr int kMaxPrecFields = 4;  // per-mode dense solve size of the preconditioner
 
+// The linear entries by operator (identity, d_a, d_a d_b): J_lin = sum_g symbol_g C_g.
+constexpr int kMaxLinOps = 13;
 struct LinTable {
-  int n, nent, ndim;
-  const LinEntry* ent;
+  int n, nops, ndim;
+  struct {
+    int nax, ax0, ax1;
+  } op[kMaxLinOps];
+  double coef[kMaxLinOps][kMaxPrecFields][kMaxPrecFields];
   const double* sinv;  // sin(2 pi m / N_a) at sinv + off[a]
   const double* cosv;
   int off[3];
@@ -162,6 +166,8 @@ struct LinTable {
   double alpha;        // preconditioner of I + alpha * J_lin
   const double* alpha_dev;  // when set, alpha is read from here (device-resident solves)
 };
+// Fills the operators and coefficients of t from the entries.
+void set_lin_ops(const std::vector<LinEntry>& lin, LinTable* t);
 
 // ----------------------------------------------------------------------------- DP45
 enum StopReason { kStopNone = 0, kStopDone = 1, kStopOutput = 2, kStopLog = 3, kStopChunk = 4 };

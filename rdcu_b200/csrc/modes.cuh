@@ -8,22 +8,22 @@
 
 namespace rdcu {
 
-// Symbol of the constant-coefficient FD operator of one linear entry at multi-index
-// nidx (see LinEntry): returns the complex value.
-__device__ __forceinline__ double2 lin_symbol(const LinEntry& e, const int* nidx, const LinTable& t) {
-  if (e.nax == 0) return make_double2(1.0, 0.0);
-  const int a = e.ax0;
+// Symbol of operator g of the table at multi-index nidx.
+__device__ __forceinline__ double2 lin_symbol(const LinTable& t, int g, const int* nidx) {
+  const int nax = t.op[g].nax, a = t.op[g].ax0, b = t.op[g].ax1;
+  if (nax == 0) return make_double2(1.0, 0.0);
   const double sa = t.sinv[t.off[a] + nidx[a]];
-  if (e.nax == 1) return make_double2(0.0, sa / t.dx[a]);
-  if (e.ax0 == e.ax1) {
+  if (nax == 1) return make_double2(0.0, sa / t.dx[a]);
+  if (a == b) {
     const double ca = t.cosv[t.off[a] + nidx[a]];
     return make_double2((2.0 * ca - 2.0) / (t.dx[a] * t.dx[a]), 0.0);
   }
-  const int b = e.ax1;
   const double sb = t.sinv[t.off[b] + nidx[b]];
   return make_double2(-2.0 * sa * sb / (t.dx[a] * t.dx[b]), 0.0);
 }
 
+// The operators and their coefficients are kernel parameters (constant memory): reading
+// the entry list from global memory, entry by entry, was a third of k_mid_solve's time.
 // x = (I + alpha L(k))^-1 r at one mode, n <= NF <= kMaxPrecFields, Gaussian elimination
 // with partial pivoting; a (numerically) singular mode is passed through unchanged.
 template <int NF>
@@ -38,18 +38,17 @@ __device__ __forceinline__ void mode_solve(const LinTable& t, const int* nidx, d
     b[i] = i < n ? v[i] : make_double2(0.0, 0.0);
   }
   const double alpha = t.alpha_dev ? *t.alpha_dev : t.alpha;
-  for (int q = 0; q < t.nent; ++q) {
-    const LinEntry e = t.ent[q];
-    const double2 sy = lin_symbol(e, nidx, t);
-    const double cf = alpha * e.coef;
+#pragma unroll 2
+  for (int g = 0; g < t.nops; ++g) {
+    const double2 sy = lin_symbol(t, g, nidx);
 #pragma unroll
     for (int i = 0; i < NF; ++i)
 #pragma unroll
-      for (int j = 0; j < NF; ++j)
-        if (i == e.row && j == e.src) {
-          A[i][j].x += cf * sy.x;
-          A[i][j].y += cf * sy.y;
-        }
+      for (int j = 0; j < NF; ++j) {
+        const double cf = alpha * t.coef[g][i][j];
+        A[i][j].x += cf * sy.x;
+        A[i][j].y += cf * sy.y;
+      }
   }
   bool ok = true;
 #pragma unroll

@@ -8,13 +8,11 @@
 
 namespace rdcu {
 
-// Complex values of all lines that one CTA transforms (128 KB of shared memory).
-constexpr int kLinePrecElems = 8192;
-
 class LinePrecond {
  public:
   // The lines of n fields of N points (two fields per complex line): false when they do
-  // not fit one CTA, N has a prime factor above 13, or memory runs out.
+  // not fit a cluster of up to eight CTAs (N / C complex values each, at most 4096 over
+  // all lines), N has a prime factor above 13, or memory runs out.
   bool init(int n, int N, double L, const std::vector<LinEntry>& lin);
   void release();
   ~LinePrecond() { release(); }
@@ -24,12 +22,11 @@ class LinePrecond {
   size_t device_bytes = 0;
 
  private:
-  int n_ = 0, N_ = 0, block_ = 0;
+  int n_ = 0, N_ = 0, C_ = 1, block_ = 0;
   double dx_ = 1.0;
   LinePlan plan_{};
   double2* tw_ = nullptr;
-  LinEntry* lin_ = nullptr;
-  int nlin_ = 0;
+  LinTable lin_{};
   double* sinv_ = nullptr;
   double* cosv_ = nullptr;
 };

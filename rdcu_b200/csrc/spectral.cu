@@ -1293,7 +1293,7 @@ struct MidSolveArgs {
 // fields, one column per CTA: 15.6 us with the plan's called stages and 4 x 4 solves,
 // about 9 us with the length's own stages and 2 x 2 solves.
 template <int RS, int LX, int NF>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_mid_solve(MidSolveArgs a) {
+__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_mid_solve(const __grid_constant__ MidSolveArgs a) {
   extern __shared__ double2 sm[];
   const int L0 = LX ? LX : a.L0, TW = a.TW, LS = tile_stride(L0, TW), T = blockDim.x, tid = threadIdx.x, n = a.n;
   double2* tw = sm;
@@ -3658,7 +3658,7 @@ void SpectralPlan::release() {
   if (ch_sorted_ && !arena_) cudaFree(ch_sorted_);
   ch_sorted_ = nullptr;
   void* ptrs[] = {tw_x_, tw_ax_[0], tw_ax_[1], tw_ax_[2], kv_, ch_off_, ch_ent_, d_terms_, d_fac_, d_poly_,
-                  d_field_begin_, d_fold_, ych_off_, ych_ent_, ych_dst_, Sf_, Sc_, lin_ent_, sinv_, cosv_,
+                  d_field_begin_, d_fold_, ych_off_, ych_ent_, ych_dst_, Sf_, Sc_, sinv_, cosv_,
                   mid_grp_, mid_A_, pipe_err_, mid_mz_, mid_mc_, mid_bz_, mid_rz_};
   if (!arena_)  // arena memory belongs to the caller
     for (void* p : ptrs)
@@ -3678,7 +3678,6 @@ void SpectralPlan::release() {
   ych_dst_ = nullptr;
   Sf_ = nullptr;
   Sc_ = nullptr;
-  lin_ent_ = nullptr;
   sinv_ = nullptr;
   cosv_ = nullptr;
   mid_grp_ = nullptr;
@@ -3690,7 +3689,6 @@ void SpectralPlan::release() {
   mid2_ = false;
   pipe_err_ = nullptr;
   pipe_mid_ = pipe_c2c_ = inv_row_ = false;
-  nlin_ = 0;
   built_ = false;
 }
 
@@ -3927,9 +3925,8 @@ bool SpectralPlan::init_precond(int n_, int ndim_, const int* Ns_, const double*
     }
   }
   (void)PI;
-  nlin_ = (int)lin.size();
-  cudaError_t e = upload(&lin_ent_, lin, &device_bytes);
-  if (e == cudaSuccess) e = upload(&sinv_, sv, &device_bytes);
+  set_lin_ops(lin, &lin_);
+  cudaError_t e = upload(&sinv_, sv, &device_bytes);
   if (e == cudaSuccess) e = upload(&cosv_, cv, &device_bytes);
   if (e == cudaSuccess) e = ensure_channel_capacity(n);
   if (e == cudaSuccess && !ych_dst_) e = cudaErrorInvalidValue;
@@ -4006,11 +4003,9 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cuda
 cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, const double* alpha_dev,
                                   cudaStream_t st) {
   RDCU_TRY(launch_forward(r, st));
-  LinTable lt{};
+  LinTable lt = lin_;
   lt.n = n;
-  lt.nent = nlin_;
   lt.ndim = ndim;
-  lt.ent = lin_ent_;
   lt.sinv = sinv_;
   lt.cosv = cosv_;
   lt.alpha = alpha;

@@ -143,8 +143,7 @@ class SpectralPlan {
   ChanEntry* ych_ent_ = nullptr;
   int* ych_dst_ = nullptr;
   // preconditioner tables
-  LinEntry* lin_ent_ = nullptr;
-  int nlin_ = 0;
+  LinTable lin_{};  // operators of the preconditioner (tables filled per call)
   double* sinv_ = nullptr;
   double* cosv_ = nullptr;
   int sc_off_[3] = {0, 0, 0};
