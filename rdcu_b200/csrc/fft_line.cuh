@@ -1,8 +1,7 @@
 // Shared-memory FP64 Stockham FFT over a batch of complex lines (device code).
 //
 // Method: the Stockham autosort formulation (Van Loan, "Computational Frameworks for
-// the Fast Fourier Transform", SIAM 1992, ch. 1.7) with mixed radices 2, 3, 4, 5, 7, 8,
-// 11, 13.  Stage s with radix R and span Ns (product of earlier radices) maps butterfly
+// the Fast Fourier Transform", SIAM 1992, ch. 1.7) with mixed radices 2..16.  Stage s with radix R and span Ns (product of earlier radices) maps butterfly
 // j of a line of length L (m = L/R butterflies) as
 //     in:  x[j + r*m] * w^(r * (j mod Ns) * L/(Ns*R)),   r < R
 //     out: y[(j/Ns)*Ns*R + (j mod Ns) + r*Ns]  = R-point DFT of the inputs,
@@ -46,22 +45,80 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
-// In-register R-point DFT of v (forward: exp(-2 pi i rk/R); inverse: conjugate).
+// cos and sin of 2 pi k / R, k = 1..(R-1)/2, for the odd radices, and of 2 pi k / 9 and
+// 2 pi k / 16: correctly rounded from the definition.  In constant memory, where the FP64
+// instructions read them as operands: as literals the compiler moves those of every radix
+// out of the stage loop and spills them.
+static __constant__ double c_root3[2] = {-0.5, 0.86602540378443864676};
+static __constant__ double c_root5[4] = {0.30901699437494742410, -0.80901699437494742410, 0.95105651629515357212,
+                                         0.58778525229247312917};
+static __constant__ double c_root7[6] = {0.62348980185873353053, -0.22252093395631440429, -0.90096886790241912624,
+                                         0.78183148246802980871, 0.97492791218182360702,  0.43388373911755812048};
+static __constant__ double c_root11[10] = {0.84125353283118116886,  0.41541501300188642553,  -0.14231483827328514044,
+                                           -0.65486073394528506406, -0.95949297361449738989, 0.54064081745559758211,
+                                           0.90963199535451837141,  0.98982144188093273238,  0.75574957435425828377,
+                                           0.28173255684142969771};
+static __constant__ double c_root13[12] = {
+    0.88545602565320989590,  0.56806474673115580251,  0.12053668025532305335, -0.35460488704253562597,
+    -0.74851074817110109863, -0.97094181742605202716, 0.46472317204376854566, 0.82298386589365639458,
+    0.99270887409805399280,  0.93501624268541482344,  0.66312265824079520238, 0.23931566428755776715};
+// W_9^e = (c_w9[2 e], -c_w9[2 e + 1]), e <= 4, and W_16^e likewise, e <= 9
+static __constant__ double c_w9[10] = {1.0, 0.0, 0.76604444311897803520, 0.64278760968653932632,
+                                       0.17364817766693034885, 0.98480775301220805937, -0.5, 0.86602540378443864676,
+                                       -0.93969262078590838405, 0.34202014332566873304};
+static __constant__ double c_w16[20] = {
+    1.0, 0.0, 0.92387953251128675613, 0.38268343236508977173, 0.70710678118654752440, 0.70710678118654752440,
+    0.38268343236508977173, 0.92387953251128675613, 0.0, 1.0, -0.38268343236508977173, 0.92387953251128675613,
+    -0.70710678118654752440, 0.70710678118654752440, -0.92387953251128675613, 0.38268343236508977173, -1.0, 0.0,
+    -0.92387953251128675613, -0.38268343236508977173};
+template <int R>
+__device__ __forceinline__ double root_cos(int k) {
+  return R == 3 ? c_root3[k - 1] : R == 5 ? c_root5[k - 1] : R == 7 ? c_root7[k - 1] : R == 11 ? c_root11[k - 1] : c_root13[k - 1];
+}
+template <int R>
+__device__ __forceinline__ double root_sin(int k) {
+  return R == 3 ? c_root3[k] : R == 5 ? c_root5[k + 1] : R == 7 ? c_root7[k + 2] : R == 11 ? c_root11[k + 4] : c_root13[k + 5];
+}
+
+// In-register R-point DFT of v (forward: exp(-2 pi i rk/R); inverse: conjugate).  Odd
+// primes: the sums and differences of the inputs r and R - r take the cosines and sines
+// of the definition, (R-1)^2 real-by-complex products and no table reads (a 5-point DFT
+// by complex products with table entries took 20 products and 20 shared-memory reads).
 template <int R, bool INV>
 struct Dft {
-  __device__ __forceinline__ static void run(double2 (&v)[R], const double2* tw, int L) {
-    // generic small prime: O(R^2) with the line's twiddle table (R divides L)
-    double2 out[R];
-    const int step = L / R;
+  static_assert(R == 3 || R == 5 || R == 7 || R == 11 || R == 13, "odd primes");
+  __device__ __forceinline__ static void run(double2 (&v)[R], const double2*, int) {
+    constexpr int H = (R - 1) / 2;
+    double2 a[H], b[H];  // per output pair (k, R - k): cosine and sine sums
+    const double2 v0 = v[0];
+    double2 sum = v0;
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      double2 acc = v[0];
-#pragma unroll
-      for (int r = 1; r < R; ++r) acc = c_add(acc, c_mul(v[r], tw_get<INV>(tw, ((r * k) % R) * step)));
-      out[k] = acc;
+    for (int k = 0; k < H; ++k) {
+      a[k] = v0;
+      b[k] = make_double2(0.0, 0.0);
     }
 #pragma unroll
-    for (int k = 0; k < R; ++k) v[k] = out[k];
+    for (int r = 1; r <= H; ++r) {
+      const double2 p = c_add(v[r], v[R - r]), m = c_sub(v[r], v[R - r]);
+      sum = c_add(sum, p);
+#pragma unroll
+      for (int k = 1; k <= H; ++k) {
+        const int t = (r * k) % R;
+        const double c = root_cos<R>(t <= H ? t : R - t);
+        const double s = t <= H ? root_sin<R>(t) : -root_sin<R>(R - t);
+        a[k - 1].x += c * p.x;
+        a[k - 1].y += c * p.y;
+        b[k - 1].x += s * m.x;
+        b[k - 1].y += s * m.y;
+      }
+    }
+    v[0] = sum;
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+      const double2 ib = c_rot<INV>(b[k - 1]);  // -i b forward, +i b inverse
+      v[k] = c_add(a[k - 1], ib);
+      v[R - k] = c_sub(a[k - 1], ib);
+    }
   }
 };
 
@@ -113,6 +170,94 @@ struct Dft<8, INV> {
   }
 };
 
+// N1 N2-point DFT of coprime factors without twiddles (I. J. Good, "The interaction
+// algorithm and practical Fourier analysis", J. R. Stat. Soc. B 20, 1958): with inputs
+// n = (N2 n1 + N1 n2) mod N, output k is output (k mod N1, k mod N2) of the 2D DFT.
+template <int N1, int N2, bool INV>
+struct DftCoprime {
+  __device__ __forceinline__ static void run(double2 (&v)[N1 * N2]) {
+    constexpr int N = N1 * N2;
+    double2 t[N2][N1];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1) t[n2][n1] = v[(N2 * n1 + N1 * n2) % N];
+      Dft<N1, INV>::run(t[n2], nullptr, 0);
+    }
+    double2 u[N1][N2];
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+#pragma unroll
+      for (int n2 = 0; n2 < N2; ++n2) u[k1][n2] = t[n2][k1];
+      Dft<N2, INV>::run(u[k1], nullptr, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = u[k % N1][k % N2];
+  }
+};
+#define RDCU_DFT_COPRIME(R, N1, N2)                                                        \
+  template <bool INV>                                                                      \
+  struct Dft<R, INV> {                                                                     \
+    __device__ __forceinline__ static void run(double2 (&v)[R], const double2*, int) {     \
+      DftCoprime<N1, N2, INV>::run(v);                                                     \
+    }                                                                                      \
+  }
+RDCU_DFT_COPRIME(6, 2, 3);
+RDCU_DFT_COPRIME(10, 2, 5);
+RDCU_DFT_COPRIME(12, 4, 3);
+RDCU_DFT_COPRIME(14, 2, 7);
+RDCU_DFT_COPRIME(15, 3, 5);
+#undef RDCU_DFT_COPRIME
+
+// R x R points in two steps: X[k1 + R k2] = sum_n2 W^(n2 k1) W_R^(n2 k2) sum_n1 x[R n1 + n2] W_R^(n1 k1)
+template <bool INV>
+struct Dft<9, INV> {
+  __device__ __forceinline__ static void run(double2 (&v)[9], const double2*, int) {
+    double2 t[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 3; ++n1) t[n2][n1] = v[3 * n1 + n2];
+      Dft<3, INV>::run(t[n2], nullptr, 0);
+#pragma unroll
+      for (int k1 = 1; k1 < 3; ++k1)
+        if (n2 > 0) t[n2][k1] = c_mul(t[n2][k1], make_double2(c_w9[2 * n2 * k1], INV ? c_w9[2 * n2 * k1 + 1] : -c_w9[2 * n2 * k1 + 1]));
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      double2 u[3] = {t[0][k1], t[1][k1], t[2][k1]};
+      Dft<3, INV>::run(u, nullptr, 0);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = u[k2];
+    }
+  }
+};
+template <bool INV>
+struct Dft<16, INV> {
+  __device__ __forceinline__ static void run(double2 (&v)[16], const double2*, int) {
+    double2 t[4][4];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 4; ++n1) t[n2][n1] = v[4 * n1 + n2];
+      Dft<4, INV>::run(t[n2], nullptr, 0);
+#pragma unroll
+      for (int k1 = 1; k1 < 4; ++k1) {
+        if (n2 == 0) continue;
+        const int e = n2 * k1;
+        t[n2][k1] = e == 4 ? c_rot<INV>(t[n2][k1]) : c_mul(t[n2][k1], make_double2(c_w16[2 * e], INV ? c_w16[2 * e + 1] : -c_w16[2 * e + 1]));
+      }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+      double2 u[4] = {t[0][k1], t[1][k1], t[2][k1], t[3][k1]};
+      Dft<4, INV>::run(u, nullptr, 0);
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = u[k2];
+    }
+  }
+};
+
 // Complex values a thread holds per stage (register budget of the staging), and the
 // largest block of an FFT pass (kMaxBlock x 128 registers fills the register file).
 constexpr int kStageElems = 8;
@@ -132,9 +277,12 @@ __device__ __forceinline__ int swz8(int i) { return i ^ ((i >> 3) & 7); }
 // inputs from swz8 positions (the stage after it).  twz: the twiddle table is stored at
 // swz8 positions (the span-8 stage reads twiddles r*kk*L/64 for kk = 0..7, which
 // otherwise share a bank group).  Values are unchanged.
+// SWZ < 0: the flags swz instead (lines of a multiple of 8 points only).
 template <int R, bool INV, bool POW2, int SWZ = 0>
 __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines, int L, int Ns, FastDiv dm,
-                                               FastDiv dns, const double2* tw, bool twz = false) {
+                                               FastDiv dns, const double2* tw, bool twz = false, int swz = 0) {
+  const bool swz_in = SWZ < 0 ? (swz & 2) != 0 : (SWZ & 2) != 0;
+  const bool swz_out = SWZ < 0 ? (swz & 1) != 0 : (SWZ & 1) != 0;
   constexpr int QMAX = (R >= kStageElems) ? 1 : (kStageElems / R);
   const int m = L / R;
   const int nb = nlines * m;
@@ -158,13 +306,18 @@ __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines,
       const int tstep = kk * tstride;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        double2 x = src[(SWZ & 2) ? swz8(j + r * m) : j + r * m];
+        double2 x = src[swz_in ? swz8(j + r * m) : j + r * m];
         if (r > 0 && tstep != 0) x = c_mul(x, tw_get<INV>(tw, twz ? swz8(r * tstep) : r * tstep));
         v[q][r] = x;
       }
       Dft<R, INV>::run(v[q], tw, L);
       dbase[q] = line * LS;
       dst[q] = jd * Ns * R + kk;
+    } else {
+      // defined on every path: a value that looks live around the stage loop keeps its
+      // registers in every other radix's stage too
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[q][r] = make_double2(0.0, 0.0);
     }
   }
   __syncthreads();
@@ -172,19 +325,10 @@ __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines,
   for (int q = 0; q < QMAX; ++q) {
     if (dst[q] >= 0) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) buf[dbase[q] + ((SWZ & 1) ? swz8(dst[q] + r * Ns) : dst[q] + r * Ns)] = v[q][r];
+      for (int r = 0; r < R; ++r) buf[dbase[q] + (swz_out ? swz8(dst[q] + r * Ns) : dst[q] + r * Ns)] = v[q][r];
     }
   }
   __syncthreads();
-}
-
-// A stage of the runtime-planned transform as a called function: the plan's stage loop
-// then holds one stage's registers at a time (inlined, the union of every radix's
-// registers exceeds the budget and spills).
-template <int R, bool INV, bool POW2>
-__device__ __noinline__ void stockham_stage_call(double2* buf, int LS, int nlines, int L, int Ns, FastDiv dm,
-                                                 FastDiv dns, const double2* tw) {
-  stockham_stage<R, INV, POW2>(buf, LS, nlines, L, Ns, dm, dns, tw);
 }
 
 // Radix sets a kernel is compiled for: power-of-two lengths use radices 8, 4, 2 only
@@ -199,33 +343,54 @@ inline bool plan_is_pow2(const LinePlan& p) {
 }
 
 // Full transform of nlines lines.  All threads of the block must call it; the data
-// must be visible (a barrier before the call).  Returns after a barrier.
+// must be visible (a barrier before the call).  Returns after a barrier.  The stages are
+// inlined: calls cost the saved registers of every thread and stage (the first stage's
+// outputs are swizzled for the second where its radix is even, see radix_seq).
 template <int RS, bool INV>
-__device__ void fft_lines(double2* buf, int LS, int nlines, const LinePlan& p, const double2* tw) {
+__device__ __forceinline__ void fft_lines(double2* buf, int LS, int nlines, const LinePlan& p, const double2* tw) {
   int Ns = 1;
+  const bool sw = p.nstages > 1 && (p.L & 7) == 0 && (p.radix[0] & 1) == 0;
+#pragma unroll 1
   for (int s = 0; s < p.nstages; ++s) {
+    // (opaque to the compiler, which otherwise hoists every radix's L / R multiples out of
+    // the loop and spills them)
+    int L = p.L;
+    asm volatile("" : "+r"(L));
     const int R = p.radix[s];
     const FastDiv dm = p.div_m[s], dns = p.div_ns[s];
+    const int swz = sw ? (s == 0 ? 1 : s == 1 ? 2 : 0) : 0;
+#define RDCU_STAGE(K, P2)                                                                          \
+  case K:                                                                                         \
+    stockham_stage<K, INV, P2, -1>(buf, LS, nlines, L, Ns, dm, dns, tw, false, swz);               \
+    break;
     if (RS == kRadixPow2) {
-      if (R == 8)
-        stockham_stage_call<8, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
-      else if (R == 4)
-        stockham_stage_call<4, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
-      else
-        stockham_stage_call<2, INV, true>(buf, LS, nlines, p.L, Ns, dm, dns, tw);
+      switch (R) {
+        RDCU_STAGE(8, true)
+        RDCU_STAGE(4, true)
+        RDCU_STAGE(2, true)
+        default: break;
+      }
     } else {
       switch (R) {
-        case 2: stockham_stage_call<2, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 3: stockham_stage_call<3, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 4: stockham_stage_call<4, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 5: stockham_stage_call<5, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 7: stockham_stage_call<7, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 8: stockham_stage_call<8, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 11: stockham_stage_call<11, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
-        case 13: stockham_stage_call<13, INV, false>(buf, LS, nlines, p.L, Ns, dm, dns, tw); break;
+        RDCU_STAGE(2, false)
+        RDCU_STAGE(3, false)
+        RDCU_STAGE(4, false)
+        RDCU_STAGE(5, false)
+        RDCU_STAGE(6, false)
+        RDCU_STAGE(7, false)
+        RDCU_STAGE(8, false)
+        RDCU_STAGE(9, false)
+        RDCU_STAGE(10, false)
+        RDCU_STAGE(11, false)
+        RDCU_STAGE(12, false)
+        RDCU_STAGE(13, false)
+        RDCU_STAGE(14, false)
+        RDCU_STAGE(15, false)
+        RDCU_STAGE(16, false)
         default: break;  // plans only contain the radices above
       }
     }
+#undef RDCU_STAGE
     Ns *= R;
   }
 }
@@ -246,24 +411,18 @@ __device__ __forceinline__ void fft_pow2_t(double2* buf, int LS, int nlines, con
   }
 }
 
-// Radix of the next stage when `rem` points of the line remain to be factored, in
-// make_line_plan's order (all 8s, then 4s, 2s, 3s, 5s, 7s, 11s, 13s).
-__host__ __device__ constexpr int plan_radix(int rem) {
-  return rem % 8 == 0 ? 8 : rem % 4 == 0 ? 4 : rem % 2 == 0 ? 2 : rem % 3 == 0 ? 3 : rem % 5 == 0 ? 5
-         : rem % 7 == 0 ? 7 : rem % 11 == 0 ? 11 : 13;
-}
-
 // The transform for any supported length L known at compile time (the plan's stage
-// sequence, constant spans and divisors; bitwise equal to fft_lines on that plan).  A
-// radix-8 first stage writes swizzled for the stage after it; twiddles are read plainly.
-template <int L, bool INV, int NS = 1>
+// sequence, constant spans and divisors; bitwise equal to fft_lines on that plan).
+// Twiddles are read plainly.
+template <int L, bool INV, int S = 0, int NS = 1>
 __device__ __forceinline__ void fft_fixed_t(double2* buf, int LS, int nlines, const double2* tw) {
-  if constexpr (NS < L) {
-    constexpr int R = plan_radix(L / NS);
-    constexpr int R0 = plan_radix(L);
-    constexpr int SWZ = (NS == 1 && R == 8 && L > 8) ? 1 : (NS == 8 && R0 == 8 ? 2 : 0);
+  constexpr RadixSeq seq = radix_seq(L);
+  if constexpr (S < seq.n) {
+    constexpr int R = seq.r[S];
+    constexpr bool SW = seq.n > 1 && L % 8 == 0 && seq.r[0] % 2 == 0;
+    constexpr int SWZ = SW ? (S == 0 ? 1 : S == 1 ? 2 : 0) : 0;
     stockham_stage<R, INV, false, SWZ>(buf, LS, nlines, L, NS, make_fastdiv_c(L / R), make_fastdiv_c(NS), tw);
-    fft_fixed_t<L, INV, NS * R>(buf, LS, nlines, tw);
+    fft_fixed_t<L, INV, S + 1, NS * R>(buf, LS, nlines, tw);
   }
 }
 

@@ -8,18 +8,10 @@ namespace rdcu {
 bool make_line_plan(int L, LinePlan* p) {
   if (L < 1 || L > kMaxLine) return false;
   p->L = L;
-  p->nstages = 0;
-  int rem = L;
-  // larger radices first; the Stockham stage handles any order
-  const int radices[] = {8, 4, 2, 3, 5, 7, 11, 13};
-  for (int r : radices) {
-    while (rem % r == 0) {
-      if (p->nstages >= kMaxStages) return false;
-      p->radix[p->nstages++] = r;
-      rem /= r;
-    }
-  }
-  if (rem != 1) return false;
+  const RadixSeq q = radix_seq(L);
+  if (q.n == 0 && L > 1) return false;
+  p->nstages = q.n;
+  for (int st = 0; st < q.n; ++st) p->radix[st] = q.r[st];
   int Ns = 1;
   for (int st = 0; st < p->nstages; ++st) {
     p->div_m[st] = make_fastdiv((unsigned)(L / p->radix[st]));

@@ -53,6 +53,45 @@ struct LinePlan {
   FastDiv div_ns[kMaxStages];  // span Ns before stage s
 };
 
+// Stage radices of a line of L points; n = 0 when L has a prime factor above 13 (n = 0 also
+// for L = 1, which needs no stage).  Powers of two: 8s, then 4 or 2 (the register kernels' sequence).
+// Other lengths: the largest divisor up to 16 at a time, since every stage is a trip
+// through shared memory and two barriers, in the order of gcd(R, 8): the first stage's
+// stores go R elements apart, which is free of bank conflicts for odd R.
+struct RadixSeq {
+  int n;
+  int r[kMaxStages];
+};
+__host__ __device__ constexpr RadixSeq radix_seq(int L) {
+  RadixSeq q{};
+  int rem = L;
+  if ((L & (L - 1)) == 0) {
+    while (rem > 1) {
+      const int R = rem % 8 == 0 ? 8 : rem;
+      q.r[q.n++] = R;
+      rem /= R;
+    }
+    return q;
+  }
+  while (rem > 1) {
+    int R = 16;
+    while (R > 1 && rem % R != 0) --R;
+    if (R == 1) return RadixSeq{};
+    q.r[q.n++] = R;
+    rem /= R;
+  }
+  for (int i = 1; i < q.n; ++i)  // stable insertion sort
+    for (int k = i; k > 0; --k) {
+      const int a = q.r[k - 1] % 8 == 0 ? 8 : q.r[k - 1] % 4 == 0 ? 4 : q.r[k - 1] % 2 == 0 ? 2 : 1;
+      const int b = q.r[k] % 8 == 0 ? 8 : q.r[k] % 4 == 0 ? 4 : q.r[k] % 2 == 0 ? 2 : 1;
+      if (a <= b) break;
+      const int t = q.r[k];
+      q.r[k] = q.r[k - 1];
+      q.r[k - 1] = t;
+    }
+  return q;
+}
+
 bool make_line_plan(int L, LinePlan* p);
 // exp(-2 pi i t / L) for t < L, rounded from long double.
 void make_twiddles(int L, std::vector<double2>& tw);

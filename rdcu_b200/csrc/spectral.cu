@@ -245,13 +245,21 @@ __device__ __forceinline__ void fft_lines_x(double2* buf, int LS, int nlines, co
     fft_lines<RS, INV>(buf, LS, nlines, p, tw);
 }
 
-// Copies the L-point twiddle table into shared memory; kernels specialised to a
-// power-of-two length store it swizzled (see fft_pow2_t).  Returns whether it did.
+// Starts the copy of the L-point twiddle table into shared memory (cp.async, so that its
+// latency overlaps the other tables' and the data's: the caller waits once for all);
+// kernels specialised to a power-of-two length store it swizzled (see fft_pow2_t).
+// Returns whether it did.
 template <int LX>
 __device__ __forceinline__ bool stage_twiddles(double2* dst, const double2* src, int L) {
   constexpr bool swz = LX > 0 && (LX & (LX - 1)) == 0;
-  for (int t = threadIdx.x; t < L; t += blockDim.x) dst[swz ? swz8(t) : t] = src[t];
+  for (int t = threadIdx.x; t < L; t += blockDim.x) cp_async16(&dst[swz ? swz8(t) : t], &src[t], true);
   return swz;
+}
+
+// Starts the copy of `bytes` (a multiple of 16, both addresses 16-byte aligned).
+__device__ __forceinline__ void stage_table(void* dst, const void* src, int bytes) {
+  for (int t = threadIdx.x * 16; t < bytes; t += blockDim.x * 16)
+    cp_async16(static_cast<char*>(dst) + t, static_cast<const char*>(src) + t, true);
 }
 
 // Stage state with the stage number known at compile time (slopes in registers).
@@ -463,6 +471,7 @@ __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
     }
   }
   if (!a.do_fft) return;
+  cp_async_wait_all();
   __syncthreads();
   fft_lines_x<RS, LX, false>(buf, M, a.P, a.plan, tw, twz);
   const int Mh = LX ? LX / 2 + 1 : a.Mh;
@@ -535,6 +544,9 @@ struct MidArgs {
   int sorted;      // entries sorted by operator, .pad = local channel (all G <= 4 channels at once)
   FastDiv dTW, dL0, dMh;
   int ent0, nent;  // entries [ent0, ent0+nent) of the launched channels, staged in smem
+  int ngrp;              // sorted: operator groups,
+  const ChanEntry* grp;  // one entry each,
+  const double* grpA;    // and their coefficients A[g][channel * 4 + source]
   int ndim, D1, Mh;
   LinePlan plan;
   const double2* tw;
@@ -555,14 +567,13 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
   // belongs to one thread), so its channel lines reuse the source lines
   const bool inplace = a.sorted && a.G <= a.nsrc;
   double2* cb = inplace ? fb : fb + a.nsrc * TW * LS;
-  // channel entries, offsets (relative to ent0) and wavenumbers staged in shared memory
+  // The tables in shared memory: the operator groups and their coefficient matrices, or
+  // the channel entries and offsets (relative to ent0); and the wavenumbers.
   ChanEntry* se = reinterpret_cast<ChanEntry*>(inplace ? fb + a.nsrc * TW * LS : cb + a.GB * TW * LS);
-  double* skv = reinterpret_cast<double*>(se + a.nent);
-  int* soff = reinterpret_cast<int*>(skv + a.chan.kv_total);
-  const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
-  for (int t = tid; t < a.nent; t += T) se[t] = a.chan.ent[a.ent0 + t];
-  for (int t = tid; t < a.chan.kv_total; t += T) skv[t] = a.chan.kv[t];
-  for (int t = tid; t <= a.G; t += T) soff[t] = a.chan.off[a.ch0 + t] - a.ent0;
+  const int nse = a.sorted ? a.ngrp : a.nent;
+  double* sA = reinterpret_cast<double*>(se + nse);
+  double* skv = sA + (a.sorted ? a.ngrp * 16 : 0);
+  int* soff = reinterpret_cast<int*>(skv + ((a.chan.kv_total + 1) & ~1));
   const long long i0 = (long long)bx * TW;
   const int nload = a.nsrc * L0 * TW;
   for (int e = tid; e < nload; e += T) {
@@ -573,36 +584,20 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
     cp_async16(&fb[(f * TW + c) * LS + z], in ? (const void*)&a.Sf[((long long)f * L0 + z) * a.I + ii] : (const void*)a.Sf,
                in);
   }
+  const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
+  stage_table(se, a.sorted ? a.grp : a.chan.ent + a.ent0, nse * (int)sizeof(ChanEntry));
+  if (a.sorted) stage_table(sA, a.grpA, a.ngrp * 16 * (int)sizeof(double));
+  stage_table(skv, a.chan.kv, (a.chan.kv_total + 1) / 2 * 16);
+  if (!a.sorted)
+    for (int t = tid; t <= a.G; t += T) soff[t] = a.chan.off[a.ch0 + t] - a.ent0;
   cp_async_wait_all();
   __syncthreads();
   fft_lines_x<RS, LX, false>(fb, LS, a.nsrc * TW, a.plan, tw, twz);
   if (a.sorted) {
-    // Every channel at once in dense form.  The operator-sorted entries become groups of
-    // one operator each with a coefficient matrix A[g][channel][source] (built once per
-    // CTA); per point, each group's multiplier beta_g is formed once and
-    //   channel c += i^q_g beta_g sum_s A[g][c][s] u_s.
-    int* sng = soff + a.G + 1;
-    ChanEntry* sgrp = reinterpret_cast<ChanEntry*>(reinterpret_cast<char*>(sm) +
-                                                   ((reinterpret_cast<char*>(sng + 1) - reinterpret_cast<char*>(sm) + 15) / 16 * 16));
-    double* sA = reinterpret_cast<double*>(sgrp + a.nent);
-    __syncthreads();  // staged entries visible
-    if (tid == 0) {
-      int g = -1, last = -1;
-      for (int qi = 0; qi < a.nent; ++qi) {
-        const ChanEntry en = se[qi];
-        const int key = en.nax | (en.ax0 << 2) | (en.ax1 << 4) | (en.part << 6);
-        if (key != last) {
-          last = key;
-          ++g;
-          sgrp[g] = en;
-          for (int k = 0; k < 16; ++k) sA[g * 16 + k] = 0.0;
-        }
-        sA[g * 16 + en.pad * 4 + en.src] += en.coef;
-      }
-      *sng = g + 1;
-    }
-    __syncthreads();
-    const int ngrp = *sng;
+    // Every channel at once in dense form: per point, each operator group's multiplier
+    // beta_g is formed once and channel c += i^q_g beta_g sum_s A[g][c][s] u_s.  (The groups
+    // are formed at plan time: one thread forming them here took over 1 us of every launch.)
+    const int ngrp = a.ngrp;
     const int npts = L0 * TW;
     for (int e = tid; e < npts; e += T) {
       const int z = fdiv(e, a.dTW), c = e - z * TW;
@@ -630,7 +625,7 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
 #pragma unroll
         for (int s4 = 0; s4 < 4; ++s4) u[s4] = s4 < a.nsrc ? fb[(s4 * TW + c) * LS + z] : make_double2(0.0, 0.0);
         for (int g = 0; g < ngrp; ++g) {
-          const ChanEntry en = sgrp[g];
+          const ChanEntry en = se[g];
           double ap = 1.0, am = 1.0;
           if (en.nax >= 1) {
             ap *= sel3(kp[0], kp[1], kp[2], en.ax0);
@@ -1291,7 +1286,7 @@ struct MidSolveArgs {
 
 // NF: the largest field count of the mode solves (2, or kMaxPrecFields).  256 x 256, two
 // fields, one column per CTA: 15.6 us with the plan's called stages and 4 x 4 solves,
-// about 9 us with the length's own stages and 2 x 2 solves.
+// 9.6 us with the length's own stages and 2 x 2 solves.
 template <int RS, int LX, int NF>
 __global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_mid_solve(const __grid_constant__ MidSolveArgs a) {
   extern __shared__ double2 sm[];
@@ -1376,19 +1371,12 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   double* phys = reinterpret_cast<double*>(lines + (a.do_fft ? P * np * M : 0));
   const long long r0 = (long long)bx * P;
   // dictionary tables staged in shared memory (read by every point)
-  double* spoly = phys + (long long)P * n * M;
+  double* spoly = phys + (((long long)P * n * M + 1) & ~1LL);  // 16-byte aligned
   const int npoly = a.dict.poly_nf ? n * a.dict.poly_count : 0;
   DictTerm* sterm = reinterpret_cast<DictTerm*>(spoly + npoly);
   DictFactor* sfac = reinterpret_cast<DictFactor*>(sterm + a.dict.nterms);
   int* sfb = reinterpret_cast<int*>(sfac + a.dict.nfac);
   int* sfold = sfb + n + 1;
-  if (!a.Yout) {
-    for (int t = tid; t < npoly; t += T) spoly[t] = a.dict.poly[t];
-    for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
-    for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
-    for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
-    for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
-  }
   if (!a.Yout) {
     // physical fields of the P rows: asynchronous 16-byte copies where rows and the
     // array's alignment allow (a caller's y may be only 8-byte aligned)
@@ -1459,6 +1447,15 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
         lines[(pr * np + cp) * M + kx] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
       }
     }
+  }
+  if (!a.Yout) {
+    stage_table(spoly, a.dict.poly, npoly * (int)sizeof(double));  // (npoly is even)
+    if (!a.dict.poly_nf) {
+      for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
+      for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
+      for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
+    }
+    for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
   }
   cp_async_wait_all();
   __syncthreads();
@@ -2510,7 +2507,7 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
   auto block_of = [&](int p) { return std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan, p * npm * M), 32))); };
   auto bytes = [&](int p, bool tws) {
     return (size_t)((spectral && tws ? M : 0) + (spectral ? p * np * M : 0)) * 16 +
-           (yout ? 0 : (size_t)p * n * M * 8 + extra);
+           (yout ? 0 : ((size_t)p * n * M + 1) / 2 * 16 + extra);
   };
   while (P > 1 && bytes(P, true) > kSmemBudget) P /= 2;
   const bool tws = bytes(P, true) <= kSmemBudget;
@@ -2656,8 +2653,7 @@ static std::vector<ChanEntry> sorted_entries(const std::vector<ChanEntry>& ent, 
   return srt;
 }
 
-// Operator groups of the operator-sorted hot entries, as k_mid forms them in each CTA:
-// one group per distinct operator (its first entry), and A[g][channel * 4 + source] the
+// Operator groups of the operator-sorted hot entries: one group per distinct operator (its first entry), and A[g][channel * 4 + source] the
 // sum of the group's coefficients in entry order.
 static void operator_groups(const std::vector<ChanEntry>& srt, std::vector<ChanEntry>* grp, std::vector<double>* A) {
   grp->clear();
@@ -2957,6 +2953,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   }
   kv_total_ = (int)kv.size();
   h_kv_ = kv;
+  if (kv.size() & 1) kv.push_back(0.0);  // k_mid copies it 16 bytes at a time
 
   // ---- device tables
   device_bytes = 0;
@@ -2977,8 +2974,15 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   chk(upload_vec(&kv_, kv));
   chk(upload_vec(&ch_off_, ch_off));
   chk(upload_vec(&ch_ent_, ch_ent));
-  // operator-sorted copy of the hot entries with the local channel in .pad
-  if (nch >= 1 && nch <= 4 && n <= 4) chk(upload_vec(&ch_sorted_, sorted_entries(ch_ent, ch_off, nch)));
+  // operator groups of the hot entries
+  if (nch >= 1 && nch <= 4 && n <= 4) {
+    std::vector<ChanEntry> grp;
+    std::vector<double> A;
+    operator_groups(sorted_entries(ch_ent, ch_off, nch), &grp, &A);
+    mid_ngrp_ = (int)grp.size();
+    chk(upload_vec(&mid_grp_, grp));
+    chk(upload_vec(&mid_A_, A));
+  }
   chk(upload_vec(&d_terms_, dterms));
   chk(upload_vec(&d_fac_, dfac));
   if (poly_nf_) chk(upload_vec(&d_poly_, poly_table()));
@@ -3043,7 +3047,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
       c.grid = (I + TW - 1) / TW;
       c.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_ax_[0], std::max(n, GB) * TW * L0), 32)));
       c.smem = smem_of(TW, GB);
-      if (which == 0 && ch_sorted_ && nch <= GB && nch <= n)  // in-place channel lines (k_mid)
+      if (which == 0 && mid_grp_ && nch <= GB && nch <= n)  // in-place channel lines (k_mid)
         c.smem = (size_t)(L0 + n * TW * tile_stride(L0, TW)) * 16 + extra;
       c.per_cta = TW | (GB << 16);  // columns per CTA | channel lines held at once
     }
@@ -3183,7 +3187,7 @@ void SpectralPlan::setup_pipes() {
       cudaGetLastError();
     }
   }
-  if (!(Ns[0] == 128 || Ns[0] == 256) || !ch_sorted_ || nch < 1 || nch > n || n > 2) return;
+  if (!(Ns[0] == 128 || Ns[0] == 256) || !mid_grp_ || nch < 1 || nch > n || n > 2) return;
   const long long I = (long long)Ns[1] * Mh;
   if (2 * I > 0x7fffffffLL) return;
   std::vector<ChanEntry> grp;
@@ -3223,10 +3227,6 @@ void SpectralPlan::setup_pipes() {
     cudaGetLastError();
     return;
   }
-  if (upload_vec(&mid_grp_, grp) != cudaSuccess || upload_vec(&mid_A_, A) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
   if (!pipe_err_ && (dev_alloc(&pipe_err_, sizeof(int)) != cudaSuccess ||
                      cudaMemsetAsync(pipe_err_, 0, sizeof(int), arena_ ? arena_->stream : 0) != cudaSuccess)) {
     cudaGetLastError();
@@ -3236,7 +3236,6 @@ void SpectralPlan::setup_pipes() {
   const int cols = 8 * (256 / Ns[0]);  // columns per tile
   const int ntiles = (int)((I + cols - 1) / cols);
   pipe_grid_ = std::max(1, std::min(ntiles, sms_));
-  mid_ngrp_ = (int)grp.size();
   pipe_mid_ = true;
   if (Ns[1] == 128 || Ns[1] == 256) {
     const void* ff = Ns[1] == 128 ? (const void*)k_c2c_pipe<128, false> : (const void*)k_c2c_pipe<256, false>;
@@ -3655,8 +3654,6 @@ cudaError_t SpectralPlan::ensure_channel_capacity(int rows) {
 }
 
 void SpectralPlan::release() {
-  if (ch_sorted_ && !arena_) cudaFree(ch_sorted_);
-  ch_sorted_ = nullptr;
   void* ptrs[] = {tw_x_, tw_ax_[0], tw_ax_[1], tw_ax_[2], kv_, ch_off_, ch_ent_, d_terms_, d_fac_, d_poly_,
                   d_field_begin_, d_fold_, ych_off_, ych_ent_, ych_dst_, Sf_, Sc_, sinv_, cosv_,
                   mid_grp_, mid_A_, pipe_err_, mid_mz_, mid_mc_, mid_bz_, mid_rz_};
@@ -3722,9 +3719,11 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
     m.io = io;
     m.ent0 = hoff[g_first];
     m.nent = hoff[g_first + nch_run] - m.ent0;
-    if (ct.ent == ch_ent_ && ch_sorted_ && nch_run <= m.GB && g_first == 0) {
+    if (ct.ent == ch_ent_ && mid_grp_ && nch_run <= m.GB && g_first == 0) {
       m.sorted = 1;
-      m.chan.ent = ch_sorted_;  // staged into shared memory in operator order
+      m.ngrp = mid_ngrp_;
+      m.grp = mid_grp_;
+      m.grpA = mid_A_;
     }
     const size_t smem = c.smem;  // includes the staged tables
     if (which == 0 && pipe_mid_ && g_first == 0 && nch_run == nch) {
@@ -4150,9 +4149,11 @@ cudaError_t SpectralPlan::profile(const RhsIO& io, int reps, cudaStream_t st, st
   m.io = io;
   m.ent0 = 0;
   m.nent = h_ch_off_[nch];
-  if (ch_sorted_ && nch <= m.GB) {
+  if (mid_grp_ && nch <= m.GB) {
     m.sorted = 1;
-    m.chan.ent = ch_sorted_;
+    m.ngrp = mid_ngrp_;
+    m.grp = mid_grp_;
+    m.grpA = mid_A_;
   }
   prep(m);
   InvXArgs a{};
@@ -4292,18 +4293,14 @@ cudaError_t SpectralPlan::set_coefficients(const std::vector<double>& C) {
   std::vector<DictTerm> dt = h_dterms_;
   for (size_t q = 0; q < dt.size(); ++q) dt[q].C = C[h_dict_term_[q]];
   if (!ent.empty()) RDCU_TRY(cudaMemcpy(ch_ent_, ent.data(), ent.size() * sizeof(ChanEntry), cudaMemcpyHostToDevice));
-  if (ch_sorted_ && nch >= 1 && nch <= 4) {
-    const std::vector<ChanEntry> srt = sorted_entries(ent, h_ch_off_, nch);
-    RDCU_TRY(cudaMemcpy(ch_sorted_, srt.data(), srt.size() * sizeof(ChanEntry), cudaMemcpyHostToDevice));
-    if (pipe_mid_) {
-      std::vector<ChanEntry> grp;
-      std::vector<double> A;
-      operator_groups(srt, &grp, &A);
-      if ((int)grp.size() != mid_ngrp_) return cudaErrorInvalidValue;
-      RDCU_TRY(cudaMemcpy(mid_grp_, grp.data(), grp.size() * sizeof(ChanEntry), cudaMemcpyHostToDevice));
-      RDCU_TRY(cudaMemcpy(mid_A_, A.data(), A.size() * sizeof(double), cudaMemcpyHostToDevice));
-      if (mid_tab_) RDCU_TRY(build_mid_tables(grp, A));
-    }
+  if (mid_grp_) {
+    std::vector<ChanEntry> grp;
+    std::vector<double> A;
+    operator_groups(sorted_entries(ent, h_ch_off_, nch), &grp, &A);
+    if ((int)grp.size() != mid_ngrp_) return cudaErrorInvalidValue;
+    RDCU_TRY(cudaMemcpy(mid_grp_, grp.data(), grp.size() * sizeof(ChanEntry), cudaMemcpyHostToDevice));
+    RDCU_TRY(cudaMemcpy(mid_A_, A.data(), A.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (pipe_mid_ && mid_tab_) RDCU_TRY(build_mid_tables(grp, A));
   }
   if (!dt.empty()) RDCU_TRY(cudaMemcpy(d_terms_, dt.data(), dt.size() * sizeof(DictTerm), cudaMemcpyHostToDevice));
   h_ch_ent_ = ent;
@@ -4408,7 +4405,7 @@ bool SpectralBatch::init(const std::vector<BatchMember>& members, int elems_, st
     // mid tiles: TW columns per item, every channel at once when the plan does so
     const int L0 = p.Ns[0], I = Mh;
     const int GBp = p.mid_[0].per_cta >> 16;
-    const bool sorted = p.ch_sorted_ && nch <= GBp;
+    const bool sorted = p.mid_grp_ && nch <= GBp;
     int GB = sorted ? nch : std::min(std::max(nch, 1), 4);
     int TW = std::max(1, std::min(elems_for(L0) / (std::max(n, GB) * L0), I));
     const size_t extra = (size_t)p.h_ch_off_[nch] * sizeof(ChanEntry) + (size_t)p.kv_total_ * 8 + (size_t)(nch + 2) * 4 +
@@ -4471,7 +4468,9 @@ bool SpectralBatch::init(const std::vector<BatchMember>& members, int elems_, st
       md.nent = p.h_ch_off_[nch];
       if (sorted) {
         md.sorted = 1;
-        md.chan.ent = p.ch_sorted_;
+        md.ngrp = p.mid_ngrp_;
+        md.grp = p.mid_grp_;
+        md.grpA = p.mid_A_;
       }
       prep(md);
       hmid[st].push_back(md);

@@ -125,7 +125,6 @@ class SpectralPlan {
   // hot-path channels and dictionary
   int* ch_off_ = nullptr;
   ChanEntry* ch_ent_ = nullptr;
-  ChanEntry* ch_sorted_ = nullptr;  // hot entries in operator order (mid pass fast path)
   DictTerm* d_terms_ = nullptr;
   DictFactor* d_fac_ = nullptr;
   int* d_field_begin_ = nullptr;
@@ -171,7 +170,7 @@ class SpectralPlan {
   bool pipe_mid_ = false, pipe_c2c_ = false, inv_row_ = false;
   int pipe_grid_ = 0, mid_ngrp_ = 0, sms_ = 1;
   CUtensorMap tm_sf_{}, tm_sc_{}, tm_sf_c2c_{}, tm_sc_c2c_{};
-  ChanEntry* mid_grp_ = nullptr;
+  ChanEntry* mid_grp_ = nullptr;  // operator groups of the hot entries (at most four channels and fields)
   double* mid_A_ = nullptr;
   bool mid_tab_ = false;           // multiplier tables (no group mixes axis 0 with another axis)
   double2* mid_mz_ = nullptr;      // [L0][nch][n]
