@@ -335,10 +335,19 @@ __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines,
 // (no register spills); any other supported length uses the general set.
 constexpr int kRadixPow2 = 0;
 constexpr int kRadixAll = 1;
+// radices up to 10 only: kernels of this set fit 80 registers where the full set takes 128
+// (and spills), which is half as many warps again for passes bound by latency
+constexpr int kRadixMid = 2;
 
 inline bool plan_is_pow2(const LinePlan& p) {
   for (int s = 0; s < p.nstages; ++s)
     if (p.radix[s] != 2 && p.radix[s] != 4 && p.radix[s] != 8) return false;
+  return true;
+}
+
+inline bool plan_is_mid(const LinePlan& p) {
+  for (int s = 0; s < p.nstages; ++s)
+    if (p.radix[s] > 10) return false;
   return true;
 }
 
@@ -368,6 +377,19 @@ __device__ __forceinline__ void fft_lines(double2* buf, int LS, int nlines, cons
         RDCU_STAGE(8, true)
         RDCU_STAGE(4, true)
         RDCU_STAGE(2, true)
+        default: break;
+      }
+    } else if (RS == kRadixMid) {
+      switch (R) {
+        RDCU_STAGE(2, false)
+        RDCU_STAGE(3, false)
+        RDCU_STAGE(4, false)
+        RDCU_STAGE(5, false)
+        RDCU_STAGE(6, false)
+        RDCU_STAGE(7, false)
+        RDCU_STAGE(8, false)
+        RDCU_STAGE(9, false)
+        RDCU_STAGE(10, false)
         default: break;
       }
     } else {

@@ -55,9 +55,11 @@ struct LinePlan {
 
 // Stage radices of a line of L points; n = 0 when L has a prime factor above 13 (n = 0 also
 // for L = 1, which needs no stage).  Powers of two: 8s, then 4 or 2 (the register kernels' sequence).
-// Other lengths: the largest divisor up to 16 at a time, since every stage is a trip
-// through shared memory and two barriers, in the order of gcd(R, 8): the first stage's
-// stores go R elements apart, which is free of bank conflicts for odd R.
+// Other lengths: as few radices up to 16 as possible, since every stage is a trip through
+// shared memory and two barriers, and as even as possible, since the smallest one sets the
+// number of threads (100 = 10 x 10, 80 = 8 x 10 rather than 5 x 16); in the order of
+// gcd(R, 8): the first stage's stores go R elements apart, which is free of bank
+// conflicts for odd R.
 struct RadixSeq {
   int n;
   int r[kMaxStages];
@@ -73,12 +75,47 @@ __host__ __device__ constexpr RadixSeq radix_seq(int L) {
     }
     return q;
   }
-  while (rem > 1) {
+  // all but the last three factors: the largest divisors; then the most even split into
+  // as few factors as possible
+  while (rem > 16 * 16 * 16) {
     int R = 16;
     while (R > 1 && rem % R != 0) --R;
     if (R == 1) return RadixSeq{};
     q.r[q.n++] = R;
     rem /= R;
+  }
+  int best[3] = {0, 0, 0};
+  if (rem <= 16) {
+    best[0] = rem;
+  } else {
+    for (int a = 16; a >= 2 && !best[0]; --a)  // two factors a >= b, the smallest a
+      if (rem % a == 0 && rem / a <= a)
+        for (int c = a; c >= 2; --c)
+          if (rem % c == 0 && rem / c <= c) {
+            best[0] = c;
+            best[1] = rem / c;
+          }
+    if (!best[0])
+      for (int a = 16; a >= 2; --a)  // three factors a >= b >= c, the largest c
+        if (rem % a == 0)
+          for (int b = a; b >= 2; --b)
+            if (rem / a % b == 0 && rem / a / b <= b && rem / a / b > best[2]) {
+              best[0] = a;
+              best[1] = b;
+              best[2] = rem / a / b;
+            }
+  }
+  if (!best[0]) {  // no three factors up to 16: the largest divisors one by one
+    while (rem > 1) {
+      int R = 16;
+      while (R > 1 && rem % R != 0) --R;
+      if (R == 1) return RadixSeq{};
+      q.r[q.n++] = R;
+      rem /= R;
+    }
+  } else {
+    for (int i = 0; i < 3; ++i)
+      if (best[i] > 1) q.r[q.n++] = best[i];
   }
   for (int i = 1; i < q.n; ++i)  // stable insertion sort
     for (int k = i; k > 0; --k) {

@@ -205,7 +205,7 @@ __device__ __forceinline__ double2 apply_entry_k(const ChanEntry& e, const doubl
 // ------------------------------------------------------------------------- kernels
 struct FwdXArgs {
   int M, Mh, nrows, P, do_fft, tw_smem;
-  FastDiv d2M, dM, d2Mh, dMh;  // invariant divisors (prep)
+  FastDiv dM, dH, dMh;  // invariant divisors (prep)
   LinePlan plan;
   const double2* tw;
   double2* S;
@@ -216,6 +216,10 @@ struct FwdXArgs {
 // resident 256-thread CTAs per SM, at most 85 registers per thread, to hide shared-memory
 // and FP64 latency); a launch that needs more threads takes the general kernels.
 constexpr int kSpecBlock = 256;
+// Launch bounds of a kernel for line length LX and radix set RS: threads, and CTAs per SM
+// (`spec` for a length of its own).
+constexpr int lb_threads(int RS, int LX) { return LX > 0 || RS == kRadixMid ? kSpecBlock : kMaxBlock; }
+constexpr int lb_ctas(int RS, int LX, int spec, int mid = 3) { return LX > 0 ? spec : RS == kRadixMid ? mid : 1; }
 
 // Line stride (in double2) of the column tiles of the strided-axis passes: TW columns of
 // one row are consecutive threads, so line c starts at c * LS; LS = L + 8/TW (at least
@@ -262,59 +266,52 @@ __device__ __forceinline__ void stage_table(void* dst, const void* src, int byte
     cp_async16(static_cast<char*>(dst) + t, static_cast<const char*>(src) + t, true);
 }
 
+// acc + c k rounded once: the stage sums are formed by several kernels, which must agree
+// (a sum of two products leaves the compiler the choice of which one to fuse)
+__device__ __forceinline__ double mac(double c, double k, double acc) { return __fma_rn(c, k, acc); }
+
 // Stage state with the stage number known at compile time (slopes in registers).
 template <int S>
 __device__ __forceinline__ double stage_value_t(long long i, const Resolved& r) {
   const double yi = r.y[i];
   if (S <= 1) return yi;
   if (S == 2) return yi + r.h * c_a[2][0] * r.k[0][i];
-  double acc = c_a[S][0] * r.k[0][i];
-  if (S != 7) acc += c_a[S][1] * r.k[1][i];
+  double acc = __dmul_rn(c_a[S][0], r.k[0][i]);
+  if (S != 7) acc = mac(c_a[S][1], r.k[1][i], acc);
 #pragma unroll
-  for (int j = 2; j < S - 1; ++j) acc += c_a[S][j] * r.k[j][i];
-  return yi + r.h * acc;
+  for (int j = 2; j < S - 1; ++j) acc = mac(c_a[S][j], r.k[j][i], acc);
+  return mac(r.h, acc, yi);
 }
 
 // Loads (with the stage combination) the rows of P line pairs into the complex lines
-// of buf, real row in .x, partner row in .y; writes the stage state when asked.  Each
-// thread issues the loads of kUnroll elements before storing any of them.
+// of buf, real row in .x, partner row in .y; writes the stage state when asked.  The rows
+// of a CTA are consecutive in memory, so an element's address needs no division and its
+// place in buf one.  Each thread issues the loads of kUnroll elements before storing any
+// of them.
 template <int S, int LX>
 __device__ __forceinline__ void fwd_load(const FwdXArgs& a, const Resolved& r, double2* buf, long long row0) {
   constexpr int kUnroll = 4;
   const int M = LX ? LX : a.M, T = blockDim.x, tid = threadIdx.x;
   const int nel = a.P * 2 * M;
+  const int live = (int)min((long long)nel, (a.nrows - row0) * M);
+  const long long g0 = row0 * M;
   for (int e0 = tid; e0 < nel; e0 += T * kUnroll) {
     double v[kUnroll];
-    long long gi[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const int e = e0 + u * T;
-      gi[u] = -1;
-      v[u] = 0.0;
-      if (e < nel) {
-        const int pl = fdivc<2 * LX>(e, a.d2M);
-        const int w = e - pl * 2 * M;
-        const int half = fdivc<LX>(w, a.dM);
-        const int x = w - half * M;
-        const long long g = row0 + 2 * pl + half;
-        if (g < a.nrows) {
-          gi[u] = g * M + x;
-          v[u] = stage_value_t<S>(gi[u], r);
-        }
-      }
+      v[u] = e < live ? stage_value_t<S>(g0 + e, r) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const int e = e0 + u * T;
       if (e >= nel) break;
-      if (r.ytemp && gi[u] >= 0) r.ytemp[gi[u]] = v[u];
-      if (S == 7 && r.aux && gi[u] >= 0) r.aux[gi[u]] = stage7_slope_sum(gi[u], r);
+      if (r.ytemp && e < live) r.ytemp[g0 + e] = v[u];
+      if (S == 7 && r.aux && e < live) r.aux[g0 + e] = stage7_slope_sum(g0 + e, r);
       if (a.do_fft) {
-        const int pl = fdivc<2 * LX>(e, a.d2M);
-        const int w = e - pl * 2 * M;
-        const int half = fdivc<LX>(w, a.dM);
-        const int x = w - half * M;
-        reinterpret_cast<double*>(buf)[2 * (pl * M + x) + half] = v[u];
+        const int row = fdivc<LX>(e, a.dM);
+        const int x = e - row * M;
+        reinterpret_cast<double*>(buf)[2 * ((row >> 1) * M + x) + (row & 1)] = v[u];
       }
     }
   }
@@ -331,19 +328,19 @@ __device__ __forceinline__ double2 stage_value_t2(long long i, const Resolved& r
     return make_double2(yi.x + r.h * c_a[2][0] * k0.x, yi.y + r.h * c_a[2][0] * k0.y);
   }
   const double2 k0 = *reinterpret_cast<const double2*>(r.k[0] + i);
-  double ax = c_a[S][0] * k0.x, ay = c_a[S][0] * k0.y;
+  double ax = __dmul_rn(c_a[S][0], k0.x), ay = __dmul_rn(c_a[S][0], k0.y);
   if (S != 7) {
     const double2 k1 = *reinterpret_cast<const double2*>(r.k[1] + i);
-    ax += c_a[S][1] * k1.x;
-    ay += c_a[S][1] * k1.y;
+    ax = mac(c_a[S][1], k1.x, ax);
+    ay = mac(c_a[S][1], k1.y, ay);
   }
 #pragma unroll
   for (int j = 2; j < S - 1; ++j) {
     const double2 kj = *reinterpret_cast<const double2*>(r.k[j] + i);
-    ax += c_a[S][j] * kj.x;
-    ay += c_a[S][j] * kj.y;
+    ax = mac(c_a[S][j], kj.x, ax);
+    ay = mac(c_a[S][j], kj.y, ay);
   }
-  return make_double2(yi.x + r.h * ax, yi.y + r.h * ay);
+  return make_double2(mac(r.h, ax, yi.x), mac(r.h, ay, yi.y));
 }
 
 // Stage 7 at the two points i, i+1 with the error term from the same loads: the new
@@ -370,40 +367,31 @@ __device__ __forceinline__ double2 stage7_value_terms2(long long i, const Resolv
   return v;
 }
 
-// fwd_load for a compile-time power-of-two row length: each thread moves pairs of
-// consecutive points (16-byte loads and stores of the state arrays).
+// fwd_load for even row lengths: each thread moves pairs of consecutive points (16-byte
+// loads and stores of the state arrays).
 template <int S, int LX>
 __device__ __forceinline__ void fwd_load2(const FwdXArgs& a, const Resolved& r, double2* buf, long long row0) {
-  static_assert(LX % 2 == 0, "even compile-time row length");
-  if constexpr (LX > 0) {
-  constexpr int kUnroll = 4, H = LX / 2;
-  const int T = blockDim.x, tid = threadIdx.x;
-  const int npair = a.P * LX;  // P line pairs of two rows, LX/2 point pairs per row
+  static_assert(LX % 2 == 0, "even row length");
+  constexpr int kUnroll = 4;
+  const int M = LX ? LX : a.M, H = M / 2, T = blockDim.x, tid = threadIdx.x;
+  const int npair = a.P * M;  // P line pairs of two rows, M/2 point pairs per row
+  const int live = (int)min((long long)npair, (a.nrows - row0) * H);
+  const long long g0 = row0 * M;
   const bool terms = S == 7 && r.aux != nullptr;
   for (int e0 = tid; e0 < npair; e0 += T * kUnroll) {
     double2 v[kUnroll];
-    long long gi[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const int e = e0 + u * T;
-      gi[u] = -1;
       v[u] = make_double2(0.0, 0.0);
-      if (e < npair) {
-        const int pl = (unsigned)e / LX;
-        const int w = e - pl * LX;
-        const int half = (unsigned)w / H;
-        const int x = (w - half * H) * 2;
-        const long long g = row0 + 2 * pl + half;
-        if (g < a.nrows) {
-          gi[u] = g * LX + x;
-          if (terms) {
-            // the error term leaves at once (no registers held across the unrolled loads)
-            double2 es_p;
-            v[u] = stage7_value_terms2(gi[u], r, &es_p);
-            *reinterpret_cast<double2*>(r.aux + gi[u]) = es_p;
-          } else {
-            v[u] = stage_value_t2<S>(gi[u], r);
-          }
+      if (e < live) {
+        if (terms) {
+          // the error term leaves at once (no registers held across the unrolled loads)
+          double2 es_p;
+          v[u] = stage7_value_terms2(g0 + 2 * e, r, &es_p);
+          *reinterpret_cast<double2*>(r.aux + g0 + 2 * e) = es_p;
+        } else {
+          v[u] = stage_value_t2<S>(g0 + 2 * e, r);
         }
       }
     }
@@ -411,19 +399,32 @@ __device__ __forceinline__ void fwd_load2(const FwdXArgs& a, const Resolved& r, 
     for (int u = 0; u < kUnroll; ++u) {
       const int e = e0 + u * T;
       if (e >= npair) break;
-      if (r.ytemp && gi[u] >= 0) *reinterpret_cast<double2*>(r.ytemp + gi[u]) = v[u];
-
+      if (r.ytemp && e < live) *reinterpret_cast<double2*>(r.ytemp + g0 + 2 * e) = v[u];
       if (a.do_fft) {
-        const int pl = (unsigned)e / LX;
-        const int w = e - pl * LX;
-        const int half = (unsigned)w / H;
-        const int x = (w - half * H) * 2;
-        double* b = reinterpret_cast<double*>(buf) + 2 * (pl * LX + x) + half;
+        const int row = fdivc<LX / 2>(e, a.dH);
+        const int x = (e - row * H) * 2;
+        double* b = reinterpret_cast<double*>(buf) + 2 * ((row >> 1) * M + x) + (row & 1);
         b[0] = v[u].x;
         b[2] = v[u].y;
       }
     }
   }
+}
+
+// The half spectra of the row pairs transformed in buf (line stride LS), row0 the first
+// row: the rows are consecutive in S.
+template <int LX>
+__device__ __forceinline__ void fwd_split(const double2* buf, int LS, int M, int Mh, FastDiv dMh, int rows,
+                                          long long row0, double2* S) {
+  const int nout = rows * Mh;
+  for (int e = threadIdx.x; e < nout; e += blockDim.x) {
+    const int row = fdivc<LX ? LX / 2 + 1 : 0>(e, dMh);
+    const int kx = e - row * Mh;
+    const double2* line = buf + (row >> 1) * LS;
+    const double2 z = line[kx];
+    const double2 zm = line[kx == 0 ? 0 : M - kx];
+    S[row0 * Mh + e] = (row & 1) == 0 ? make_double2(0.5 * (z.x + zm.x), 0.5 * (z.y - zm.y))
+                                      : make_double2(0.5 * (z.y + zm.y), -0.5 * (z.x - zm.x));
   }
 }
 
@@ -436,7 +437,7 @@ __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
   if (a.io.mode == 1 && !a.io.ctl->running) return;
   Resolved r = resolve(a.io);
   r.nN = (long long)a.nrows * (LX ? LX : a.M);
-  const int M = LX ? LX : a.M, T = blockDim.x, tid = threadIdx.x;
+  const int M = LX ? LX : a.M;
   const double2* tw = a.tw;
   double2* buf = sm;
   bool twz = false;
@@ -449,7 +450,7 @@ __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
   // 16-byte state loads need 16-byte aligned arrays (a caller's y may be offset)
   unsigned long long align = reinterpret_cast<unsigned long long>(r.y) | reinterpret_cast<unsigned long long>(r.ytemp);
   for (int j = 0; j < 7; ++j) align |= reinterpret_cast<unsigned long long>(r.k[j]);
-  if (LX > 0 && (align & 15) == 0) {
+  if ((M & 1) == 0 && (align & 15) == 0) {
     switch (SF > 0 ? SF : r.stage) {
       case 2: fwd_load2<2, LX>(a, r, buf, row0); break;
       case 3: fwd_load2<3, LX>(a, r, buf, row0); break;
@@ -474,31 +475,14 @@ __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
   cp_async_wait_all();
   __syncthreads();
   fft_lines_x<RS, LX, false>(buf, M, a.P, a.plan, tw, twz);
-  const int Mh = LX ? LX / 2 + 1 : a.Mh;
-  const int nout = a.P * 2 * Mh;
-  for (int e = tid; e < nout; e += T) {
-    const int pl = fdivc<LX ? 2 * (LX / 2 + 1) : 0>(e, a.d2Mh);
-    const int w = e - pl * 2 * Mh;
-    const int half = fdivc<LX ? LX / 2 + 1 : 0>(w, a.dMh);
-    const int kx = w - half * Mh;
-    const long long g = row0 + 2 * pl + half;
-    if (g >= a.nrows) continue;
-    const double2 z = buf[pl * M + kx];
-    const double2 zm = buf[pl * M + (kx == 0 ? 0 : M - kx)];
-    double2 o;
-    if (half == 0)
-      o = make_double2(0.5 * (z.x + zm.x), 0.5 * (z.y - zm.y));
-    else
-      o = make_double2(0.5 * (z.y + zm.y), -0.5 * (z.x - zm.x));
-    a.S[g * Mh + kx] = o;
-  }
+  fwd_split<LX>(buf, M, M, LX ? LX / 2 + 1 : a.Mh, a.dMh, (int)min(2LL * a.P, a.nrows - row0), row0, a.S);
 }
 
 // The CTAs take the rows from the last to the first: the previous stage's row kernel
 // ended on the last rows of the slope this stage reads (still in L2), and the axis-1
 // pass after it starts on the first planes, written last here.
 template <int RS, int LX, int SF = 0>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? (SF > 0 ? 4 : 2) : 1) k_fwd_x(FwdXArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, (SF > 0 ? 4 : 2))) k_fwd_x(FwdXArgs a) {
   fwd_x_body<RS, LX, SF>(a, gridDim.x - 1 - blockIdx.x);
 }
 
@@ -512,7 +496,7 @@ struct C2CArgs {
 };
 
 template <int RS, bool INV, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_c2c(C2CArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2)) k_c2c(C2CArgs a) {
   extern __shared__ double2 sm[];
   if (a.io.mode == 1 && !a.io.ctl->running) return;
   const int La = LX ? LX : a.La, TW = a.TW, LS = tile_stride(La, TW), T = blockDim.x, tid = threadIdx.x;
@@ -733,7 +717,7 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
 }
 
 template <int RS, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 3 : 1) k_mid(MidArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3)) k_mid(MidArgs a) {
   mid_body<RS, LX>(a, blockIdx.x);
 }
 
@@ -1288,7 +1272,7 @@ struct MidSolveArgs {
 // fields, one column per CTA: 15.6 us with the plan's called stages and 4 x 4 solves,
 // 9.6 us with the length's own stages and 2 x 2 solves.
 template <int RS, int LX, int NF>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1) k_mid_solve(const __grid_constant__ MidSolveArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2, 2)) k_mid_solve(const __grid_constant__ MidSolveArgs a) {
   extern __shared__ double2 sm[];
   const int L0 = LX ? LX : a.L0, TW = a.TW, LS = tile_stride(L0, TW), T = blockDim.x, tid = threadIdx.x, n = a.n;
   double2* tw = sm;
@@ -1340,7 +1324,7 @@ __global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 
 
 struct InvXArgs {
   int M, Mh, R, P, n, nch_run, npairs, do_fft, tw_smem;
-  FastDiv dM, dnpM, dnhalf, dhalf, dnM, dncM;
+  FastDiv dM, dMh, dnp, dnhalf, dhalf, dnM, dncM;
   long long N;
   LinePlan plan;
   const double2* tw;
@@ -1351,9 +1335,78 @@ struct InvXArgs {
   const int* ydst;
   int yplain;         // 1: channel c -> real array Yout[c*N + point]
   int ch_base;        // first channel row of Sc this launch reads
+  int fuse_off;       // fused pass: offset of its staging in shared memory, in doubles
+  // the fused pass (inv_x_body with FUSE): stage s + 1's state and half spectra out
+  RhsIO io2;
+  double2* Sf;
 };
 
-template <int RS, int LX>
+// y and stage S's sum over the slopes before the newest one (stage_value_t's terms in its
+// order) at the P rows of every field into shared memory; the rows of a field are
+// consecutive in memory.  Issued before the transform, which covers the loads' latency;
+// V points at a time (16-byte loads), kUnroll of them in flight.
+template <int S, int V>
+__device__ __forceinline__ void stage_older_slopes(const Resolved& r, int n, int PM, int live, long long g0,
+                                                   long long RM, double* sy, double* ss) {
+  using T = typename std::conditional<V == 2, double2, double>::type;
+  constexpr int kUnroll = 2;
+  const int cnt = live / V;
+  for (int i = 0; i < n; ++i) {
+    const long long gf = i * RM + g0;
+    for (int e0 = threadIdx.x; e0 < cnt; e0 += blockDim.x * kUnroll) {
+      T yv[kUnroll];
+      double acc[kUnroll][V];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int e = e0 + u * blockDim.x;
+        if (e >= cnt) break;
+        yv[u] = *reinterpret_cast<const T*>(r.y + gf + (long long)e * V);
+        T k[6];
+#pragma unroll
+        for (int j = 0; j < S - 2; ++j)
+          if (j != 1 || (S != 7 && S >= 4)) k[j] = *reinterpret_cast<const T*>(r.k[j] + gf + (long long)e * V);
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+          auto part = [c](const T& t) { return reinterpret_cast<const double*>(&t)[c]; };
+          double a = __dmul_rn(c_a[S][0], part(k[0]));
+#pragma unroll
+          for (int j = 1; j < S - 2; ++j)
+            if (j != 1 || (S != 7 && S >= 4)) a = mac(c_a[S][j], part(k[j]), a);
+          acc[u][c] = a;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int e = e0 + u * blockDim.x;
+        if (e >= cnt) break;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+          sy[i * PM + e * V + c] = reinterpret_cast<const double*>(&yv[u])[c];
+          ss[i * PM + e * V + c] = acc[u][c];
+        }
+      }
+    }
+  }
+}
+template <int V>
+__device__ __forceinline__ void stage_older_slopes(const Resolved& r, int n, int PM, int live, long long g0,
+                                                   long long RM, double* sy, double* ss) {
+  switch (r.stage) {
+    case 3: stage_older_slopes<3, V>(r, n, PM, live, g0, RM, sy, ss); break;
+    case 4: stage_older_slopes<4, V>(r, n, PM, live, g0, RM, sy, ss); break;
+    case 5: stage_older_slopes<5, V>(r, n, PM, live, g0, RM, sy, ss); break;
+    case 6: stage_older_slopes<6, V>(r, n, PM, live, g0, RM, sy, ss); break;
+    default: stage_older_slopes<7, V>(r, n, PM, live, g0, RM, sy, ss); break;
+  }
+}
+
+// FUSE: the inverse x pass of DP45 stage s (2..6, no error epilogue, a dense-polynomial
+// dictionary) and the forward x pass of stage s + 1 in one kernel, P even and R even, so
+// that the forward pass's row pairs lie in the CTA.  After the dictionary the new slope
+// completes stage s + 1's state (stage_value_t's terms in its order), which is written,
+// transformed and split into half spectra: the separate passes' arithmetic, bit for bit,
+// without reading the slope and the state back and with one launch less.
+template <int RS, int LX, bool FUSE = false>
 __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   extern __shared__ double2 sm[];
   if (a.io.mode == 1 && !a.io.ctl->running) return;
@@ -1368,7 +1421,9 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
     tw = sm;
     lines = sm + M;
   }
-  double* phys = reinterpret_cast<double*>(lines + (a.do_fft ? P * np * M : 0));
+  // (the fused pass transforms the fields' row pairs in the same lines)
+  const int nlines = FUSE ? P / 2 * max(2 * np, n) : P * np;
+  double* phys = reinterpret_cast<double*>(lines + (a.do_fft ? nlines * M : 0));
   const long long r0 = (long long)bx * P;
   // dictionary tables staged in shared memory (read by every point)
   double* spoly = phys + (((long long)P * n * M + 1) & ~1LL);  // 16-byte aligned
@@ -1406,8 +1461,9 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
     }
   }
   if (a.do_fft) {
+    // every spectral value once: it gives the line elements kx and M - kx
     constexpr int kUnroll = 4;
-    const int nel = P * np * M;
+    const int nel = P * np * Mh;
     for (int e0 = tid; e0 < nel; e0 += T * kUnroll) {
       double2 A[kUnroll], B[kUnroll];
 #pragma unroll
@@ -1416,37 +1472,47 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
         A[u] = make_double2(0.0, 0.0);
         B[u] = make_double2(0.0, 0.0);
         if (e >= nel) continue;
-        const int pr = fdiv(e, a.dnpM);
-        const int w = e - pr * np * M;
-        const int cp = fdivc<LX>(w, a.dM);
-        const int kx = w - cp * M;
+        const int q = fdivc<LX ? LX / 2 + 1 : 0>(e, a.dMh);  // row of the tile and channel pair
+        const int kx = e - q * Mh;
+        const int pr = np == 1 ? q : fdiv(q, a.dnp);
         const long long row = r0 + pr;
         if (row >= a.R) continue;
-        const int c0 = 2 * cp, c1 = c0 + 1;
-        const int kk = kx >= Mh ? M - kx : kx;
-        A[u] = a.Sc[((long long)(a.ch_base + c0) * a.R + row) * Mh + kk];
-        if (c1 < a.nch_run) B[u] = a.Sc[((long long)(a.ch_base + c1) * a.R + row) * Mh + kk];
+        const int c0 = 2 * (q - pr * np), c1 = c0 + 1;
+        A[u] = a.Sc[((long long)(a.ch_base + c0) * a.R + row) * Mh + kx];
+        if (c1 < a.nch_run) B[u] = a.Sc[((long long)(a.ch_base + c1) * a.R + row) * Mh + kx];
       }
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         const int e = e0 + u * T;
         if (e >= nel) break;
-        const int pr = fdiv(e, a.dnpM);
-        const int w = e - pr * np * M;
-        const int cp = fdivc<LX>(w, a.dM);
-        const int kx = w - cp * M;
+        const int q = fdivc<LX ? LX / 2 + 1 : 0>(e, a.dMh);
+        const int kx = e - q * Mh;
         double2 Av = A[u], Bv = B[u];
         if (kx == 0 || 2 * kx == M) {
           Av.y = 0.0;
           Bv.y = 0.0;
+        } else {
+          lines[q * M + M - kx] = make_double2(Av.x + Bv.y, Bv.x - Av.y);
         }
-        if (kx >= Mh) {
-          Av.y = -Av.y;
-          Bv.y = -Bv.y;
-        }
-        lines[(pr * np + cp) * M + kx] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
+        lines[q * M + kx] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
       }
     }
+  }
+  double* sy = nullptr;  // FUSE: y and the older slopes' sums of the CTA's points, [field][row][x]
+  double* ss = nullptr;
+  Resolved r2;
+  if constexpr (FUSE) {
+    r2 = resolve(a.io2);
+    sy = reinterpret_cast<double*>(sm) + a.fuse_off;
+    const int PM = P * M;
+    ss = sy + n * PM;
+    const int live = (int)min((long long)PM, (a.R - r0) * M);
+    const long long g0 = r0 * M, RM = (long long)a.R * M;
+    // (the engine's state and slope arrays are 16-byte aligned)
+    if ((M & 1) == 0)
+      stage_older_slopes<2>(r2, n, PM, live, g0, RM, sy, ss);
+    else
+      stage_older_slopes<1>(r2, n, PM, live, g0, RM, sy, ss);
   }
   if (!a.Yout) {
     stage_table(spoly, a.dict.poly, npoly * (int)sizeof(double));  // (npoly is even)
@@ -1484,8 +1550,13 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
 
   const DictTable& D = a.dict;
   // stage-7 epilogue of adaptive steps only (fixed steps pass no partials buffer)
-  const bool err = (a.io.mode == 1 && r.stage == 7 && a.io.err_part != nullptr);
+  const bool err = !FUSE && a.io.mode == 1 && r.stage == 7 && a.io.err_part != nullptr;
   const int npts = P * M;
+  const double cnew = FUSE ? c_a[r2.stage][r2.stage - 2] : 0.0;  // of the new slope in stage s + 1
+  // Two fields in one channel pair: the forward lines of a row pair (one per field) take the
+  // place of its two inverse lines, and a thread reads and writes both at its own x.
+  // Otherwise the new state goes to the staging of the fields and from there to the lines.
+  const bool local = FUSE && n == 2 && np == 1;
   // Each thread evaluates the dictionary at PPT points at once, so that the tables
   // (warp-uniform shared-memory reads, loop control, the power switch) are read once per
   // PPT points.  Points past the tile read a valid address and store nothing.  NF > 0: the
@@ -1493,16 +1564,24 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   // multiply-add per monomial and field); NF = 0: the term list.
   auto points = [&](auto ppt, auto nf) {
     constexpr int PPT = decltype(ppt)::value, NF = decltype(nf)::value;
-    for (int e0 = tid; e0 < npts; e0 += T * PPT) {
-      int phoff[PPT], lnoff[PPT];
+    // (the fused pass: the two rows of a forward line at one x)
+    const int e1 = FUSE ? npts / 2 : npts;
+    for (int e0 = tid; e0 < e1; e0 += FUSE ? T : T * PPT) {
+      int phoff[PPT], lnoff[PPT], psoff[PPT];
+      double yn[FUSE ? PPT : 1][NF > 0 ? NF : 1];
       long long gbase[PPT];
       bool live[PPT];
       double err2[PPT];
 #pragma unroll
       for (int k = 0; k < PPT; ++k) {
-        const int e = e0 + k * T;
-        const int pr = fdivc<LX>(e, a.dM);
-        const int x = e - pr * M;
+        int e = e0 + k * T;
+        int pr = fdivc<LX>(FUSE ? e0 : e, a.dM);
+        const int x = (FUSE ? e0 : e) - pr * M;
+        if (FUSE) {
+          pr = 2 * pr + k;
+          e = pr * M + x;
+        }
+        psoff[k] = e;
         const long long row = r0 + pr;
         live[k] = e < npts && row < a.R;
         phoff[k] = live[k] ? pr * n * M + x : 0;
@@ -1520,7 +1599,8 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
           for (int m = 1; m < MN::count; ++m) mono[k][m] = mono[k][MN::parent(m)] * phys[phoff[k] + MN::var(m) * M];
         }
       }
-      for (int i = 0; i < n; ++i) {
+#pragma unroll(FUSE ? 4 : 1)
+      for (int i = 0; i < (NF > 0 ? NF : n); ++i) {
         double acc[PPT];
         const int fc = sfold[i];
 #pragma unroll
@@ -1566,9 +1646,15 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
         }
 #pragma unroll
         for (int k = 0; k < PPT; ++k) {
+          if (FUSE) yn[FUSE ? k : 0][NF > 0 ? i : 0] = 0.0;
           if (!live[k]) continue;
           const long long gi = (long long)i * a.R * M + gbase[k];
           r.f[gi] = acc[k];
+          if constexpr (FUSE) {
+            const double v = mac(r2.h, mac(cnew, acc[k], ss[i * npts + psoff[k]]), sy[i * npts + psoff[k]]);
+            if (r2.ytemp) r2.ytemp[gi] = v;
+            yn[k][i] = v;
+          }
           if (err) {
             // error kernel of dp45.cu:79-84 (e_2 = 0 drops k2)
             const double ynew = phys[phoff[k] + i * M];
@@ -1578,6 +1664,17 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
             const double ev = r.h * es / (r.atol + r.rtol * fmax(fabs(yold), fabs(ynew)));
             err2[k] += ev * ev;
           }
+        }
+      }
+      if constexpr (FUSE) {
+        const int pl = fdivc<LX>(e0, a.dM), x = e0 - pl * M;
+#pragma unroll
+        for (int i = 0; i < NF; ++i) {
+          if (local)
+            lines[(pl * NF + i) * M + x] = make_double2(yn[0][i], yn[1][i]);
+          else
+#pragma unroll
+            for (int k = 0; k < 2; ++k) phys[((2 * pl + k) * n + i) * M + x] = yn[k][i];
         }
       }
       if (err) {
@@ -1594,8 +1691,29 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   switch (a.dict.poly_nf) {
     case 1: points(I2{}, I1{}); break;
     case 2: points(I2{}, I2{}); break;
-    case 3: points(I1{}, std::integral_constant<int, 3>{}); break;
-    default: points(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{}); break;
+    case 3: points(std::integral_constant<int, FUSE ? 2 : 1>{}, std::integral_constant<int, 3>{}); break;
+    default:
+      if constexpr (!FUSE) points(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{});
+      break;
+  }
+  if constexpr (FUSE) {
+    __syncthreads();
+    // forward lines [row pair][field] (rows past R are zero)
+    const int half = P / 2;
+    if (!local) {
+      const int nel = n * half * M;
+      for (int e = tid; e < nel; e += T) {
+        const int q = fdivc<LX>(e, a.dM);
+        const int x = e - q * M;
+        const int p = q / n, i = q - p * n;
+        lines[e] = make_double2(phys[(2 * p * n + i) * M + x], phys[((2 * p + 1) * n + i) * M + x]);
+      }
+      __syncthreads();
+    }
+    fft_lines_x<RS, LX, false>(lines, M, n * half, a.plan, tw, twz);
+    const int rows = (int)min((long long)P, a.R - r0);
+    for (int i = 0; i < n; ++i)
+      fwd_split<LX>(lines + i * M, n * M, M, Mh, a.dMh, rows, (long long)i * a.R + r0, a.Sf);
   }
   if (err) {
     // one partial sum per grid row, in an order fixed by the row alone (x = lane,
@@ -1615,8 +1733,13 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
 }
 
 template <int RS, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 3 : 1) k_inv_x(InvXArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3)) k_inv_x(InvXArgs a) {
   inv_x_body<RS, LX>(a, blockIdx.x);
+}
+template <int RS, int LX>
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2, 2))
+    k_inv_fwd_x(const __grid_constant__ InvXArgs a) {
+  inv_x_body<RS, LX, true>(a, blockIdx.x);
 }
 
 // ---- x pass of 3D grids with 128- or 256-point rows and a dense-polynomial dictionary
@@ -2353,7 +2476,7 @@ __device__ __forceinline__ void load_args(A* dst, const A* src) {
 // the launch bounds of the single-problem kernels.  The groups of one pass run as
 // concurrent branches (SpectralBatch::launch_stage).
 template <int RS, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 1)
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2))
     k_fwd_x_group(const FwdXArgs* __restrict__ args, const int2* __restrict__ items, int nitems) {
   __shared__ __align__(16) FwdXArgs sa;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -2366,7 +2489,7 @@ __global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 2 : 
 }
 
 template <int RS, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 3 : 1)
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3))
     k_mid_group(const MidArgs* __restrict__ args, const int2* __restrict__ items, int nitems) {
   __shared__ __align__(16) MidArgs sa;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -2379,7 +2502,7 @@ __global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 3 : 
 }
 
 template <int RS, int LX>
-__global__ void __launch_bounds__(LX > 0 ? kSpecBlock : kMaxBlock, LX > 0 ? 3 : 1)
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3))
     k_inv_x_group(const InvXArgs* __restrict__ args, const int2* __restrict__ items, int nitems) {
   __shared__ __align__(16) InvXArgs sa;
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -2416,9 +2539,8 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 // Invariant divisors of each pass's index arithmetic, filled before every launch.
 void prep(FwdXArgs& a) {
-  a.d2M = make_fastdiv(2 * a.M);
   a.dM = make_fastdiv(a.M);
-  a.d2Mh = make_fastdiv(2 * a.Mh);
+  a.dH = make_fastdiv(std::max(1, a.M / 2));
   a.dMh = make_fastdiv(a.Mh);
 }
 void prep(C2CArgs& a) { a.dTW = make_fastdiv(a.TW); }
@@ -2435,7 +2557,8 @@ void prep(MidSolveArgs& a) {
 void prep(InvXArgs& a) {
   const int half = a.M / 2;
   a.dM = make_fastdiv(a.M);
-  a.dnpM = make_fastdiv(std::max(1, a.npairs) * a.M);
+  a.dMh = make_fastdiv(a.Mh);
+  a.dnp = make_fastdiv(std::max(1, a.npairs));
   a.dnhalf = make_fastdiv(std::max(1, a.n * half));
   a.dhalf = make_fastdiv(std::max(1, half));
   a.dnM = make_fastdiv(a.n * a.M);
@@ -2494,6 +2617,15 @@ static bool opt_in_smem(const void* func) {
   return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess;
 }
 
+// Columns per tile of a strided pass over I columns, before the shared-memory limits halve
+// it: a power of two, so that a tile's row is whole 32-byte sectors (3 columns: 48 bytes),
+// that leaves two CTAs per SM.
+static int column_tile(int I) {
+  int TW = 16;
+  while (TW > 1 && TW > I / kTargetCtas) TW /= 2;
+  return TW;
+}
+
 // Geometry of the inverse x pass for nch_run channels (with or without the
 // physical-field staging): rows per CTA, grid, block and dynamic shared memory.
 static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const LinePlan& plan, PassCfg* c,
@@ -2518,14 +2650,32 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
   *tw_smem = tws ? 1 : 0;
 }
 
+// Geometry of the fused inverse/forward x pass: two rows per CTA, 256 threads.  It is taken
+// while its CTAs are at most two per SM, where a pass's time is the latency of one tile and
+// a launch saved is worth more than the fused kernel's serial phases.  Above that the
+// separate passes are faster, with their smaller kernels (3D 100 x 96 x 80: 60 us fused
+// against 42 us; ensemble of 512: 169 against 141 ms).  per_cta 0: not taken.
+static void fuse_geometry(int M, int R, int n, int nch, const LinePlan& plan, size_t dict_bytes, PassCfg* c,
+                          int* fuse_off) {
+  const int lines = std::max(2 * ((nch + 1) / 2), n);  // complex lines of two rows
+  const size_t off = ((size_t)(M + lines * M) * 16 + (size_t)2 * n * M * 8 + dict_bytes + 15) / 16 * 16;
+  const size_t bytes = off + (size_t)4 * n * M * 8;
+  c->per_cta = R / 2 <= kTargetCtas && bytes <= kSmemBudget && lines * M <= kMaxElems ? 2 : 0;
+  c->grid = R / 2;
+  c->block = std::min(kMaxBlock, std::max({128, round_up(stage_threads(plan, lines * M), 32), std::min(256, round_up(M, 32))}));
+  c->smem = bytes;
+  *fuse_off = (int)(off / 8);
+}
+
 // Calls f(radix set, line length) with compile-time values for the plan's lengths:
 // lines of 64..512 points (powers of two, and 96 and 192) get kernels specialised to
 // their length, other power-of-two lines the shift-indexed kernels, every other length
-// the general ones.
+// the general ones (those of radices up to 10 where the block allows).
 template <typename F>
 static void by_length(const LinePlan& p, int block, F&& f) {
   using RP = std::integral_constant<int, kRadixPow2>;
   using RA = std::integral_constant<int, kRadixAll>;
+  using RM = std::integral_constant<int, kRadixMid>;
   switch (block <= kSpecBlock ? p.L : 0) {
     case 64: f(RP{}, std::integral_constant<int, 64>{}); return;
     case 128: f(RP{}, std::integral_constant<int, 128>{}); return;
@@ -2537,6 +2687,8 @@ static void by_length(const LinePlan& p, int block, F&& f) {
   }
   if (plan_is_pow2(p))
     f(RP{}, std::integral_constant<int, 0>{});
+  else if (block <= kSpecBlock && plan_is_mid(p))
+    f(RM{}, std::integral_constant<int, 0>{});
   else
     f(RA{}, std::integral_constant<int, 0>{});
 }
@@ -3013,6 +3165,12 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
     int tws = 0;
     inv_geometry(M, R, n, nch, false, plan_x_, &inv_, &tws, dict_smem_bytes());
   }
+  // the fused inverse/forward x pass: row pairs of a field within one CTA
+  // (RDCU_FUSED_ROWS=0 keeps the passes separate)
+  const char* fz = getenv("RDCU_FUSED_ROWS");
+  fuse_x_ = {};
+  if (nch > 0 && poly_nf_ > 0 && R % 2 == 0 && !explicit_channels_ && !(fz && fz[0] == '0'))
+    fuse_geometry(M, R, n, nch, plan_x_, dict_smem_bytes(), &fuse_x_, &fuse_off_);
   nparts_max = R;  // stage-7 error partials: one per grid row
   // Y-mode channel group
   const int GY = std::min(ych_, 8);
@@ -3023,7 +3181,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
     for (int which = 0; which < 2; ++which) {
       const int G = which == 0 ? nch : GY;
       if (G == 0) continue;
-      int TW = std::max(1, std::min(16, I / kTargetCtas));
+      int TW = column_tile(I);
       int GB = std::min(G, 4);
       while (TW > 1 && std::max(n, GB) * TW * L0 > cta_elems()) TW /= 2;
       while (GB > 1 && std::max(n, GB) * TW * L0 > kMaxElems) --GB;
@@ -3098,6 +3256,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
           optin_ok &= opt_in_smem((const void*)k_fwd_x<RS, LX, 7>);
         }
         optin_ok &= opt_in_smem((const void*)k_inv_x<RS, LX>);
+        optin_ok &= opt_in_smem((const void*)k_inv_fwd_x<RS, LX>);
         optin_ok &= opt_in_smem((const void*)k_mid<RS, LX>);
         optin_ok &= opt_in_smem((const void*)k_c2c<RS, false, LX>);
         optin_ok &= opt_in_smem((const void*)k_c2c<RS, true, LX>);
@@ -3401,6 +3560,37 @@ cudaError_t SpectralPlan::launch_inv_row(const RhsIO& io, cudaStream_t st) {
 bool SpectralPlan::fuse_ok(const RhsIO& io, const RhsIO& next) const {
   return fuse_rows_ && inv_row_ && io.mode == 1 && next.mode == 1 && io.ctl == next.ctl && io.stage >= 2 && io.stage <= 5 &&
          next.stage == io.stage + 1 && !plane_inv_ok(io) && !plane_fwd_ok(next);
+}
+
+bool SpectralPlan::fuse_x_ok(const RhsIO& io, const RhsIO& next) const {
+  return fuse_x_.per_cta > 0 && !inv_row_ && io.mode == 1 && next.mode == 1 && io.ctl == next.ctl && io.stage >= 2 &&
+         io.stage <= 6 && next.stage == io.stage + 1 && !next.err_aux && !plane_inv_ok(io) && !plane_fwd_ok(next);
+}
+
+cudaError_t SpectralPlan::launch_inv_fwd_x(const RhsIO& io, const RhsIO& next, cudaStream_t st) {
+  InvXArgs a{};
+  a.M = M;
+  a.Mh = Mh;
+  a.R = R;
+  a.n = n;
+  a.nch_run = nch;
+  a.npairs = (nch + 1) / 2;
+  a.do_fft = 1;
+  a.tw_smem = 1;
+  a.N = N;
+  a.plan = plan_x_;
+  a.tw = tw_x_;
+  a.Sc = Sc_;
+  a.dict = dict_table();
+  a.io = io;
+  a.io2 = next;
+  a.Sf = Sf_;
+  a.P = fuse_x_.per_cta;
+  a.fuse_off = fuse_off_;
+  prep(a);
+  const PassCfg& g = fuse_x_;
+  by_length(plan_x_, g.block, [&](auto rs, auto lx) { k_inv_fwd_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
+  return cudaGetLastError();
 }
 
 cudaError_t SpectralPlan::launch_inv_fwd_row(const RhsIO& io, const RhsIO& next, cudaStream_t st) {
@@ -3780,6 +3970,10 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
     }
     return launch_inv_row(io, st);
   }
+  if (!Yout && next && fused && fuse_x_ok(io, *next) && ct.ent == ch_ent_ && g_first == 0 && nch_run == nch) {
+    *fused = true;
+    return launch_inv_fwd_x(io, *next, st);
+  }
   for (int c0 = 0; c0 < std::max(1, nch_run); c0 += step) {
     const int cnt = spectral ? std::min(step, nch_run - c0) : 0;
     InvXArgs a{};
@@ -3936,7 +4130,7 @@ bool SpectralPlan::init_precond(int n_, int ndim_, const int* Ns_, const double*
   if (ndim >= 2) {
     const int L0 = Ns[0];
     const int I = (ndim == 3) ? Ns[1] * Mh : Mh;
-    int TW = std::max(1, std::min(16, I / kTargetCtas));
+    int TW = column_tile(I);
     auto smem_of = [&](int tw_) { return (size_t)(L0 + n * tw_ * tile_stride(L0, tw_)) * 16; };
     while (TW > 1 && (smem_of(TW) > kSmemBudget || n * TW * L0 > cta_elems())) TW /= 2;
     if (smem_of(TW) > 227 * 1024 || n * TW * L0 > kMaxElems) {

@@ -147,6 +147,8 @@ class SpectralPlan {
   double* cosv_ = nullptr;
   int sc_off_[3] = {0, 0, 0};
   PassCfg midsolve_{};
+  PassCfg fuse_x_{};  // the general fused inverse/forward x pass (per_cta 0: not taken)
+  int fuse_off_ = 0;
   // spectral buffers
   double2* Sf_ = nullptr;  // field half spectra [n][R][Mh]
   double2* Sc_ = nullptr;  // channel half spectra [max(nch, G)][R][Mh]
@@ -193,6 +195,8 @@ class SpectralPlan {
   // stage io's inverse x pass fused with stage next's forward x pass (k_inv_fwd_row)
   bool fuse_rows_ = false;
   bool fuse_ok(const RhsIO& io, const RhsIO& next) const;
+  bool fuse_x_ok(const RhsIO& io, const RhsIO& next) const;
+  cudaError_t launch_inv_fwd_x(const RhsIO& io, const RhsIO& next, cudaStream_t st);
   cudaError_t launch_inv_fwd_row(const RhsIO& io, const RhsIO& next, cudaStream_t stream);
   // 3D x passes that also transform along axis 1, one thread-block cluster per plane
   // (k_fwd_plane, k_inv_plane): enabled flags and persistent grid sizes

@@ -245,3 +245,43 @@ def test_advance_beyond_the_attempt_log(cuda):
     t, h, _ = s.get_state()
     assert abs(t - 0.5) < 1e-12 and h == 1e-4
     s.close()
+
+
+def _poly_terms(n, ndim):
+    """A dense-polynomial dictionary with one Laplacian per field: u_i' = u_i + lap u_i - u_i^3
+    + 0.3 u_j (j the next field)."""
+    lines = []
+    for i in range(n):
+        lines += ["1.0,%d,%d,1" % (i, i), "-1.0,%d,%d,3" % (i, i), "0.3,%d,%d,1" % (i, (i + 1) % n)]
+        lines += ["%s,%d,%d,1" % (1.0 + 0.2 * i, i, n + ndim * n + (a * ndim + a) * n + i) for a in range(ndim)]
+    return lines
+
+
+@pytest.mark.parametrize("n,Ns", [(2, (2, 16)), (2, (16, 16)), (2, (64, 48)), (2, (20, 15)), (2, (250, 180)),
+                                  (2, (128, 512)), (1, (22, 26)), (3, (10, 21)), (3, (64, 128)), (2, (10, 7, 12)),
+                                  (2, (100, 9, 80)), (2, (6, 4, 1024))])
+@pytest.mark.parametrize("fixed", [False, True])
+def test_fused_x_passes_are_the_separate_ones(cuda, monkeypatch, n, Ns, fixed):
+    """The general fused inverse/forward x pass (an even number of rows per field, any row
+    length) computes what the separate passes compute, bit for bit: row counts that leave
+    the last CTA part of its rows, odd row lengths, one to three fields."""
+    from oracle.problem import parse_term
+
+    prob = Problem(n, Ns, tuple(0.7 * v for v in Ns), [parse_term(s) for s in _poly_terms(n, len(Ns))])
+    y0 = np.random.default_rng(11).uniform(-1, 1, n * prob.N)
+    outs = []
+    for env in (None, "0"):
+        if env is None:
+            monkeypatch.delenv("RDCU_FUSED_ROWS", raising=False)
+        else:
+            monkeypatch.setenv("RDCU_FUSED_ROWS", env)
+        s, yd = _setup(cuda, prob, y0, fixed=fixed)
+        s.set_state(0.0, 1e-3, yd)
+        s.advance(6)
+        out = cuda.empty_like(yd)
+        t, h, _ = s.get_state(out)
+        outs.append((t, h, out.cpu().numpy()))
+        s.close()
+    assert outs[0][:2] == outs[1][:2]
+    np.testing.assert_array_equal(outs[0][2], outs[1][2])
+    assert np.all(np.isfinite(outs[0][2])) and np.any(outs[0][2] != y0)
