@@ -19,6 +19,7 @@
 // Checkpoints: the state every K steps; each segment is recomputed from its
 // checkpoint with the fused forward stages, keeping the stage states Y_1..Y_6.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 
@@ -254,6 +255,148 @@ __global__ void __launch_bounds__(kThreads) k_adj_stage(PointwiseArgs a, Combine
   }
 }
 
+// k_adj_stage for dictionaries whose nonlinear terms are products of at most three of NF <= 3
+// fields (no derivative quantities): the monomials and their derivatives are formed once
+// per point in registers, with the coefficients as a dense table, instead of every term's
+// factor list being read and multiplied out three times from shared memory.  The gradient
+// terms add up in a slot per thread and are summed once at the end (a warp per term) instead of
+// by a shuffle reduction per term and point.  Latency-bound at 256 x 256 (the state is in
+// L2): 16.7 us there with the term lists, 8.4 us so.
+struct PolyArgs {
+  const double* poly;  // [NF][Mono<NF>::count]
+  const int2* terms;   // (field, monomial) of every kept term
+};
+template <int NF>
+constexpr size_t poly_smem(int nkept, int nfold) {
+  return ((size_t)(Mono<NF>::count + NF + nkept + nfold) * kThreads + NF * Mono<NF>::count) * sizeof(double);
+}
+template <int NF>
+__global__ void __launch_bounds__(kThreads) k_adj_poly(const __grid_constant__ PointwiseArgs a,
+                                                       const __grid_constant__ CombineArgs cb,
+                                                       const __grid_constant__ PolyArgs pa, int do_pw, int do_cb) {
+  extern __shared__ double psm[];
+  using MN = Mono<NF>;
+  constexpr int T = kThreads;
+  __shared__ AdjFold sfold[kMaxTerms];
+  __shared__ int2 sterm[kMaxTerms];
+  __shared__ int sorig[kMaxTerms];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* smono = psm;                  // [monomial][thread]
+  double* sw = smono + MN::count * T;   // kbar [field][thread]
+  double* sg = sw + NF * T;             // gradient slots [folded, then kept term][thread]
+  double* spoly = sg + (size_t)(a.nkept + cb.nfold) * T;
+  for (int i = tid; i < NF * MN::count; i += T) spoly[i] = pa.poly[i];
+  for (int i = tid; i < a.nkept; i += T) {
+    sterm[i] = pa.terms[i];
+    sorig[i] = a.terms[i].orig;
+  }
+  for (int i = tid; i < cb.nfold; i += T) sfold[i] = cb.folds[i];
+  for (int i = 0; i < a.nkept + cb.nfold; ++i) sg[i * T + tid] = 0.0;
+  __syncthreads();
+  for (long long base = (long long)blockIdx.x * T; base < a.N; base += (long long)gridDim.x * T) {
+    const long long x = base + tid;
+    if (x >= a.N) break;
+    double lam[NF], ybprev[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) lam[f] = ybprev[f] = 0.0;
+    if (do_pw || cb.final_stage) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) lam[f] = a.lam[f * a.N + x];
+    }
+    if (do_cb) {
+      double v[NF], u[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        v[f] = cb.ubar[f * a.N + x];
+        u[f] = cb.u[f * a.N + x];
+      }
+#pragma unroll 4
+      for (int t = 0; t < cb.nfold; ++t) {
+        const AdjFold fd = sfold[t];
+        const double G = cb.G[(long long)fd.g * a.N + x];
+        double us = 0.0;
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+          if (f == fd.src) {
+            v[f] += fd.C * G;
+            us = u[f];
+          }
+        sg[t * T + tid] += G * us;
+      }
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const long long o = f * a.N + x;
+        if (cb.final_stage) {
+          double l = lam[f] + v[f];
+          for (int i = 2; i <= 6; ++i) l += cb.Yb[(long long)(i - 1) * a.nN + o];
+          cb.lam[o] = l;
+          lam[f] = l;
+        } else {
+          cb.Yb[o] = v[f];
+          ybprev[f] = v[f];  // Ybar of stage a.stage + 1, used below
+        }
+      }
+    }
+    if (!do_pw) continue;
+    double w[NF], u[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const long long o = f * a.N + x;
+      u[f] = a.u[o];
+      double yb[7];
+#pragma unroll
+      for (int l = 2; l <= 6; ++l)
+        yb[l] = l <= a.stage ? 0.0 : l == a.stage + 1 && do_cb ? ybprev[f] : a.Yb[(long long)(l - 1) * a.nN + o];
+      double s = a.hb * lam[f];
+#pragma unroll
+      for (int l = 2; l <= 6; ++l)
+        if (l > a.stage) s += a.ha.c[l] * yb[l];
+      w[f] = s;
+      a.w[o] = s;
+      sw[f * T + tid] = s;
+    }
+    double mono[MN::count], dm[MN::count][NF];
+    mono[0] = 1.0;
+    smono[tid] = 1.0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) dm[0][f] = 0.0;
+#pragma unroll
+    for (int m = 1; m < MN::count; ++m) {
+      const double uv = u[MN::var(m)];
+      mono[m] = mono[MN::parent(m)] * uv;
+      smono[m * T + tid] = mono[m];
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        dm[m][f] = dm[MN::parent(m)][f] * uv + (MN::var(m) == f ? mono[MN::parent(m)] : 0.0);
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      double ub = 0.0;
+#pragma unroll
+      for (int i = 0; i < NF; ++i) {
+        double s = 0.0;
+#pragma unroll
+        for (int m = 1; m < MN::count; ++m) s += spoly[i * MN::count + m] * dm[m][f];
+        ub += w[i] * s;
+      }
+      a.ubar[f * a.N + x] = ub;
+    }
+    for (int t = 0; t < a.nkept; ++t)
+      sg[(cb.nfold + t) * T + tid] += sw[sterm[t].x * T + tid] * smono[sterm[t].y * T + tid];
+  }
+  __syncthreads();
+  for (int t = warp; t < cb.nfold + (do_pw ? a.nkept : 0); t += T / 32) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < T / 32; ++k) s += sg[t * T + k * 32 + lane];
+    s = warp_sum(s);
+    if (lane == 0) {
+      const int orig = t < cb.nfold ? sfold[t].orig : sorig[t - cb.nfold];
+      a.part[(long long)orig * gridDim.x + blockIdx.x] += s;
+    }
+  }
+}
+
 // dL/dC_t = sum over the blocks' accumulated partials (fixed order: deterministic)
 __global__ void k_adj_reduce(const double* part, int nterms, double* gC) {
   const int t = blockIdx.x;
@@ -294,6 +437,17 @@ struct AdjointEngine::Tables {
   int nkept = 0, nfac = 0, nfold = 0, nq = 0;
   std::vector<AdjTerm> h_terms;
   std::vector<AdjFold> h_folds;
+  // dense-polynomial form (k_adj_poly): fields, coefficients and each kept term's monomial
+  int poly_nf = 0;
+  double* poly = nullptr;
+  int2* poly_terms = nullptr;
+  std::vector<int2> h_poly_terms;
+  std::vector<double> poly_table() const {
+    const int count = mono_exponents(poly_nf).size();
+    std::vector<double> P((size_t)poly_nf * count, 0.0);
+    for (size_t t = 0; t < h_terms.size(); ++t) P[(size_t)h_poly_terms[t].x * count + h_poly_terms[t].y] += h_terms[t].C;
+    return P;
+  }
 };
 
 #define RDCU_TRY(x)                   \
@@ -422,8 +576,36 @@ bool AdjointEngine::init(SpectralPlan* fwd, DP45Engine* dp, const std::vector<Ho
   T.nfac = (int)fac.size();
   T.nfold = (int)T.h_folds.size();
   T.nq = nq_;
-  pw_smem_ = pointwise_smem(n, nq_, T.nkept, T.nfac);
-  if (pw_smem_ > 48 * 1024 &&
+  // products of at most three fields: the dense-polynomial kernel
+  if (n <= 3 && nq_ == 0) {
+    const auto ex = mono_exponents(n);
+    bool dense = true;
+    for (const AdjTerm& t : T.h_terms) {
+      std::array<int, 3> e{0, 0, 0};
+      for (int j = 0; j < t.nf; ++j) {
+        dense = dense && fac[t.off + j].eta > 0 && fac[t.off + j].eta <= 3;
+        if (dense) e[fac[t.off + j].q] += fac[t.off + j].eta;
+      }
+      int mono = -1;
+      for (size_t m = 0; m < ex.size(); ++m)
+        if (ex[m] == e) mono = (int)m;
+      dense = dense && mono >= 0;
+      T.h_poly_terms.push_back(make_int2(t.field, mono));
+    }
+    const size_t sm = n == 1   ? poly_smem<1>(T.nkept, T.nfold)
+                      : n == 2 ? poly_smem<2>(T.nkept, T.nfold)
+                               : poly_smem<3>(T.nkept, T.nfold);
+    const void* fn = n == 1 ? (const void*)k_adj_poly<1> : n == 2 ? (const void*)k_adj_poly<2> : (const void*)k_adj_poly<3>;
+    if (dense && sm <= 200 * 1024 &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess) {
+      T.poly_nf = n;
+      pw_smem_ = sm;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  if (!T.poly_nf) pw_smem_ = pointwise_smem(n, nq_, T.nkept, T.nfac);
+  if (!T.poly_nf && pw_smem_ > 48 * 1024 &&
       cudaFuncSetAttribute(k_adj_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pw_smem_) != cudaSuccess) {
     *msg = "adjoint set-up: dictionary too large for the pointwise kernel's shared memory";
     return false;
@@ -435,6 +617,8 @@ bool AdjointEngine::init(SpectralPlan* fwd, DP45Engine* dp, const std::vector<Ho
   };
   if (up(&T.terms, T.h_terms) != cudaSuccess || up(&T.fac, fac) != cudaSuccess ||
       up(&T.folds, T.h_folds) != cudaSuccess || up(&T.qs, qs) != cudaSuccess)
+    return fail("tables");
+  if (T.poly_nf && (up(&T.poly, T.poly_table()) != cudaSuccess || up(&T.poly_terms, T.h_poly_terms) != cudaSuccess))
     return fail("tables");
   if (cudaMalloc((void**)&lam_, sb) != cudaSuccess) return fail("out of device memory");
   if (cudaMalloc((void**)&Yb_, sb * 6) != cudaSuccess) return fail("out of device memory");
@@ -464,7 +648,7 @@ void AdjointEngine::release() {
   store_ = lam_ = Yb_ = tin_ = tout_ = qv_ = ubar_ = part_ = gC_ = nullptr;
   store_steps_ = 0;
   if (tab_) {
-    void* t[] = {tab_->terms, tab_->fac, tab_->folds, tab_->qs};
+    void* t[] = {tab_->terms, tab_->fac, tab_->folds, tab_->qs, tab_->poly, tab_->poly_terms};
     for (void* p : t)
       if (p) cudaFree(p);
     delete tab_;
@@ -480,6 +664,10 @@ cudaError_t AdjointEngine::set_coefficients(const std::vector<double>& C) {
     RDCU_TRY(cudaMemcpy(T.terms, T.h_terms.data(), T.h_terms.size() * sizeof(AdjTerm), cudaMemcpyHostToDevice));
   if (!T.h_folds.empty())
     RDCU_TRY(cudaMemcpy(T.folds, T.h_folds.data(), T.h_folds.size() * sizeof(AdjFold), cudaMemcpyHostToDevice));
+  if (T.poly_nf) {
+    const std::vector<double> P = T.poly_table();
+    RDCU_TRY(cudaMemcpy(T.poly, P.data(), P.size() * sizeof(double), cudaMemcpyHostToDevice));
+  }
   return cudaSuccess;
 }
 
@@ -620,7 +808,13 @@ cudaError_t AdjointEngine::stage_kernels(const double* Y, int stage, double h, c
   ca.Yb = Yb_ + (size_t)(sprev > 0 ? sprev - 1 : 0) * nN_;
   ca.lam = lam_;
   ca.part = part_;
-  k_adj_stage<<<kBlocks, kThreads, pw_smem_, st_>>>(pa, ca, Y ? 1 : 0, Yprev ? 1 : 0);
+  const PolyArgs po{T.poly, T.poly_terms};
+  switch (T.poly_nf) {
+    case 1: k_adj_poly<1><<<kBlocks, kThreads, pw_smem_, st_>>>(pa, ca, po, Y ? 1 : 0, Yprev ? 1 : 0); break;
+    case 2: k_adj_poly<2><<<kBlocks, kThreads, pw_smem_, st_>>>(pa, ca, po, Y ? 1 : 0, Yprev ? 1 : 0); break;
+    case 3: k_adj_poly<3><<<kBlocks, kThreads, pw_smem_, st_>>>(pa, ca, po, Y ? 1 : 0, Yprev ? 1 : 0); break;
+    default: k_adj_stage<<<kBlocks, kThreads, pw_smem_, st_>>>(pa, ca, Y ? 1 : 0, Yprev ? 1 : 0); break;
+  }
   RDCU_TRY(cudaGetLastError());
   if (Y && ng_ > 0) RDCU_TRY(planT_.run_linear(tin_, tout_, st_));
   return cudaSuccess;

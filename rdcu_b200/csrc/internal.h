@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -214,6 +215,23 @@ struct Mono<3> {
     return v[m];
   }
 };
+
+// Exponent vectors (up to 3 variables) of the Mono<nf> monomials.
+inline std::vector<std::array<int, 3>> mono_exponents(int nf) {
+  std::vector<std::array<int, 3>> ex;
+  auto build = [&](auto mn) {
+    using MN = decltype(mn);
+    ex.assign(MN::count, {0, 0, 0});
+    for (int m = 1; m < MN::count; ++m) {
+      ex[m] = ex[MN::parent(m)];
+      ex[m][MN::var(m)] += 1;
+    }
+  };
+  if (nf == 1) build(Mono<1>{});
+  if (nf == 2) build(Mono<2>{});
+  if (nf == 3) build(Mono<3>{});
+  return ex;
+}
 
 // Constant-coefficient linear part of the finite-difference Jacobian, one entry per
 // linear term: row field, source field, FD operator, coefficient.  Its symbol at

@@ -2745,23 +2745,6 @@ std::vector<double> SpectralPlan::poly_table() const {
   return A;
 }
 
-// Exponent vectors (up to 3 variables) of the Mono<nf> monomials.
-static std::vector<std::array<int, 3>> mono_exponents(int nf) {
-  std::vector<std::array<int, 3>> ex;
-  auto build = [&](auto mn) {
-    using MN = decltype(mn);
-    ex.assign(MN::count, {0, 0, 0});
-    for (int m = 1; m < MN::count; ++m) {
-      ex[m] = ex[MN::parent(m)];
-      ex[m][MN::var(m)] += 1;
-    }
-  };
-  if (nf == 1) build(Mono<1>{});
-  if (nf == 2) build(Mono<2>{});
-  if (nf == 3) build(Mono<3>{});
-  return ex;
-}
-
 DictTable SpectralPlan::dict_table() const {
   DictTable d{};
   d.n = n;
@@ -3957,8 +3940,9 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
     RDCU_TRY(cudaGetLastError());
   }
   // inverse x pass: the dictionary needs every channel of a row in one CTA; the Y.dat
-  // output is launched one channel pair at a time
-  const int step = Yout ? 2 : std::max(1, nch_run);
+  // output is launched one channel pair at a time (a linear operator's channels at once
+  // where a row of them fits a CTA's usual size)
+  const int step = Yout && !(yplain && (nch_run + 1) / 2 * M <= cta_elems()) ? 2 : std::max(1, nch_run);
   // stage 7 of an adaptive step: the row kernel's error epilogue reads the terms the
   // forward pass left in err_aux; without them k_inv_x forms the error from y and slopes
   const bool err_epilogue = io.mode == 1 && io.stage == 7 && io.err_part != nullptr;

@@ -247,3 +247,50 @@ def test_long_segments_and_step_sequences(cuda):
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
     s.close()
+
+
+# the dense-polynomial stage kernel (products of at most three of one to three fields) at point
+# counts below, at and above its blocks, against the tangent-linear model
+@pytest.mark.parametrize("n,Ns", [(1, (6, 7)), (2, (16, 16)), (2, (15, 34)), (3, (12, 10)), (3, (5, 9, 8)),
+                                  (2, (300, 256))])
+def test_adjoint_duality_dense_polynomial(cuda, n, Ns):
+    import rdcu_b200 as R
+    from oracle.problem import parse_term
+    from oracle import tangent as otan
+
+    rng = np.random.default_rng(n + sum(Ns))
+    ndim = len(Ns)
+    lines = []
+    for i in range(n):
+        j = (i + 1) % n
+        lines += ["0.7,%d,%d,1" % (i, i), "-1.0,%d,%d,3" % (i, i), "0.4,%d,%d,1,%d,2" % (i, i, j) if j != i else "0.2,0,0,2",
+                  "0.3,%d" % i]
+        lines += ["%s,%d,%d,1" % (1.0 + 0.2 * i, i, n + ndim * n + (a * ndim + a) * n + j) for a in range(ndim)]
+    prob = Problem(n, Ns, tuple(1.0 * v for v in Ns), [parse_term(s) for s in lines])
+    nN = n * prob.N
+    y0, dy, w = rng.uniform(-0.5, 0.5, nN), rng.normal(size=nN), rng.normal(size=nN)
+    C = np.array([t.C for t in prob.terms])
+    dC = rng.normal(size=C.size)
+    hs = [1e-3, 2e-3, 1.5e-3]
+    s = _solver(prob)
+    yd, wd = (cuda.tensor(v, dtype=cuda.float64, device="cuda") for v in (y0, w))
+    gy = cuda.empty_like(yd)
+    cuda.cuda.synchronize()
+    s.adjoint_forward(yd, hs, 2)
+    gC = np.array(s.adjoint_backward(wd, gy))
+    s.close()
+    # central difference of the GPU map along (dy, dC): the map is cubic, error O(eps^2)
+    eps, out = 1e-5, []
+    for sgn in (1, -1):
+        s = _solver(prob)
+        s.set_coefficients(list(C + sgn * eps * dC))
+        z = cuda.tensor(y0 + sgn * eps * dy, dtype=cuda.float64, device="cuda")
+        yT = cuda.empty_like(z)
+        cuda.cuda.synchronize()
+        s.adjoint_forward(z, hs, 2, yT)
+        out.append(yT.cpu().numpy())
+        s.close()
+    lhs = float(w @ (out[0] - out[1])) / (2 * eps)
+    rhs = float(gy.cpu().numpy() @ dy) + float(gC @ dC)
+    # eps^2 for the third derivative, rounding / eps for the difference
+    assert abs(lhs - rhs) <= 1e-6 * (np.linalg.norm(w) * np.linalg.norm(dy))
