@@ -53,6 +53,7 @@ class EnsembleEngine {
   double* state_mem_ = nullptr;  // every member's 3 state + 7 slope buffers and error partials
   DP45Ctl* d_ctl_ = nullptr;
   DP45Ctl* h_ctl_ = nullptr;  // pinned mirror
+  bool ctl_current_ = false;  // h_ctl_ equals d_ctl_
   double** d_parts_ = nullptr;
   double* d_nN_ = nullptr;
   int* d_running_ = nullptr;
@@ -62,6 +63,7 @@ class EnsembleEngine {
   cudaError_t ensure_graph();
   cudaError_t launch_attempt();
   cudaError_t sync_ctl();
+  cudaError_t current_ctl();  // h_ctl_ as the device has it
 };
 
 }  // namespace rdcu

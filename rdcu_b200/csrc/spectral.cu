@@ -3115,8 +3115,13 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
     std::vector<double> A;
     operator_groups(sorted_entries(ch_ent, ch_off, nch), &grp, &A);
     mid_ngrp_ = (int)grp.size();
-    chk(upload_vec(&mid_grp_, grp));
-    chk(upload_vec(&mid_A_, A));
+    // one upload: the groups' entries, then their coefficients
+    std::vector<ChanEntry> blob(grp);
+    static_assert(sizeof(ChanEntry) % sizeof(double) == 0, "coefficients follow the entries");
+    blob.resize(grp.size() + A.size() * sizeof(double) / sizeof(ChanEntry));
+    std::memcpy(static_cast<void*>(blob.data() + grp.size()), A.data(), A.size() * sizeof(double));
+    chk(upload_vec(&mid_grp_, blob));
+    mid_A_ = reinterpret_cast<double*>(mid_grp_ + grp.size());
   }
   chk(upload_vec(&d_terms_, dterms));
   chk(upload_vec(&d_fac_, dfac));
@@ -3829,7 +3834,7 @@ cudaError_t SpectralPlan::ensure_channel_capacity(int rows) {
 void SpectralPlan::release() {
   void* ptrs[] = {tw_x_, tw_ax_[0], tw_ax_[1], tw_ax_[2], kv_, ch_off_, ch_ent_, d_terms_, d_fac_, d_poly_,
                   d_field_begin_, d_fold_, ych_off_, ych_ent_, ych_dst_, Sf_, Sc_, sinv_, cosv_,
-                  mid_grp_, mid_A_, pipe_err_, mid_mz_, mid_mc_, mid_bz_, mid_rz_};
+                  mid_grp_, pipe_err_, mid_mz_, mid_mc_, mid_bz_, mid_rz_};
   if (!arena_)  // arena memory belongs to the caller
     for (void* p : ptrs)
       if (p) cudaFree(p);
