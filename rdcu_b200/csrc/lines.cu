@@ -73,14 +73,25 @@ __device__ __forceinline__ double wrap_pi(double x) {
 
 // Nonzero winding of the plaquette t0 -> t1 -> t2 -> t3 (makelines.py:19-24): the four
 // wrapped differences summed in that order, over 2 pi, rounded half to even.
-// Shortcut with the same answer: when every difference d is below 3 in magnitude, d + pi
-// lies in (0.14, 6.15), no branch of wrap_pi adds or subtracts 2 pi, and each wrapped
-// difference is d to within two roundings of pi-sized values (~1e-15); the exact
-// differences sum to zero, so the rounded ones, and s, stay within ~1e-14 of zero and
-// rint(s / 2 pi) is 0.  A NaN fails the comparisons and takes the full path.
+// The same answer without the divisions and the modulus: with a = d + pi in (-2 pi, 4 pi),
+// wrap_pi subtracts 2 pi when a >= 2 pi, adds it when a < 0 and leaves a alone otherwise, so a
+// wrapped difference is d - 2 pi w, w in {-1, 0, 1}, to within two roundings of pi-sized
+// values (~1e-15).  The exact differences sum to zero, so the sum is within ~1e-14 of
+// -2 pi (w0 + w1 + w2 + w3) and rint(s / 2 pi) is nonzero exactly when that integer is.
+// Differences outside that range, and NaN, take the full path.
 __device__ __forceinline__ bool winds(double t0, double t1, double t2, double t3) {
   const double d0 = t1 - t0, d1 = t2 - t1, d2 = t3 - t2, d3 = t0 - t3;
+  // (below 3 in magnitude: no wrap at all)
   if (fabs(d0) < 3.0 && fabs(d1) < 3.0 && fabs(d2) < 3.0 && fabs(d3) < 3.0) return false;
+  const double a[4] = {d0 + kPi, d1 + kPi, d2 + kPi, d3 + kPi};
+  bool in = true;
+  int w = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    in = in && a[i] > -kTwoPi && a[i] < 2.0 * kTwoPi;
+    w += (a[i] >= kTwoPi ? 1 : 0) - (a[i] < 0.0 ? 1 : 0);
+  }
+  if (in) return w != 0;
   const double s = wrap_pi(d0) + wrap_pi(d1) + wrap_pi(d2) + wrap_pi(d3);
   return rint(s / kTwoPi) != 0.0;
 }
@@ -293,13 +304,8 @@ __global__ void __launch_bounds__(kT) k_roots(const int* __restrict__ label, con
   }
 }
 
-// The components of a frame with few line cubes in one CTA: the forest, its roots and
-// their numbering in shared memory (atomics and root walks at shared-memory latency), the
-// same union-find rules as k_hook / k_flatten / k_roots / k_label, so the labels and the
-// component numbers are identical.  Writes deg, comp, key, order and the component count
-// to *n_comp.
 constexpr int kSmallThreads = 1024;
-constexpr int kSmallNodes = 12288;  // 2 x 4 B per node of shared memory (96 KB)
+constexpr int kSmallNodes = 12288;  // 9 bytes of shared memory per node in k_graph_small (108 KB)
 
 __device__ int uf_find_s(int* parent, int x, int* err) {
   volatile int* P = parent;
@@ -314,32 +320,144 @@ __device__ int uf_find_s(int* parent, int x, int* err) {
   return -1;
 }
 
-__global__ void __launch_bounds__(kSmallThreads) k_components_small(const int* __restrict__ cubes,
-                                                                     const int* __restrict__ node_of,
-                                                                     int* __restrict__ deg, int* __restrict__ comp,
-                                                                     int* __restrict__ key, int* __restrict__ order,
-                                                                     int n, Grid g, int* err, int* n_comp,
-                                                                     int* n_edges) {
+// ---- frames of few line cubes: the cube marks as bits, and the graph in one CTA, with
+// every count on the device, so that the host waits once per frame (for the counts) instead
+// of sizing each step.  flags: 0 error, 1 components, 2 edges, 3 cubes.  A frame with more
+// than kSmallNodes cubes is found again by the general passes.
+constexpr int kBitWords = 1024;  // words of bits per block of k_compact_bits
+
+// Line cube marks (k_mark's rule), a bit per point: a warp's 32 points are one word; and the
+// number of cubes in every kBitWords words (zeroed by the caller).
+__global__ void __launch_bounds__(kT) k_mark_bits(const unsigned char* __restrict__ face, unsigned* __restrict__ bits,
+                                                  int* __restrict__ counts, Grid g) {
+  const int c = blockIdx.x * kT + threadIdx.x;
+  bool m = false;
+  if (c < g.total) {
+    int i, j, k;
+    coords(g, c, i, j, k);
+    const int di = (i + 1 < g.N[0]) ? g.s0 : -(g.N[0] - 1) * g.s0;
+    const int dj = (j + 1 < g.N[1]) ? g.s1 : -(g.N[1] - 1) * g.s1;
+    const int dk = (k + 1 < g.N[2]) ? 1 : -(g.N[2] - 1);
+    m = ((face[c] & 7) | (face[c + dk] & 1) | (face[c + di] & 2) | (face[c + dj] & 4)) != 0;
+  }
+  const unsigned b = __ballot_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && c < g.total) bits[c >> 5] = b;
+  const int cnt = __syncthreads_count(m);
+  if (threadIdx.x == 0 && cnt) atomicAdd(&counts[(c >> 5) / kBitWords], cnt);
+}
+
+// Cubes in ascending order and their nodes, from the bits: a thread per word, after the sum
+// of the counts of the blocks before this one.  node_of is written at the cubes only;
+// readers test the bit first.
+__global__ void __launch_bounds__(kBitWords) k_compact_bits(const unsigned* __restrict__ bits, int nw,
+                                                       const int* __restrict__ counts,
+                                                       int* __restrict__ cubes, int* __restrict__ node_of, int cap,
+                                                       int* __restrict__ flags) {
+  __shared__ int red[32];
+  __shared__ int sbase;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int before = 0;
+  for (int q = threadIdx.x; q < (int)blockIdx.x; q += kBitWords) before += counts[q];
+  const int wi = blockIdx.x * kBitWords + threadIdx.x;
+  const unsigned mine = wi < nw ? bits[wi] : 0u;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 0) red[w] = before;
+  __syncthreads();
+  if (w == 0) {
+    int t = red[lane];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) sbase = t;
+  }
+  __syncthreads();
+  int x = __popc(mine);
+  const int cnt = x;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) red[w] = x;
+  __syncthreads();
+  int off = sbase;
+  for (int q = 0; q < w; ++q) off += red[q];
+  int v = off + x - cnt;
+  for (unsigned m = mine; m; m &= m - 1) {
+    const int c = wi * 32 + __ffs(m) - 1;
+    if (v < cap) {
+      cubes[v] = c;
+      node_of[c] = v;
+    }
+    ++v;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kBitWords - 1) flags[3] = v;
+}
+
+__device__ __forceinline__ int node_at(const unsigned* __restrict__ bits, const int* __restrict__ node_of, int c) {
+  if (bits && !((bits[c >> 5] >> (c & 31)) & 1u)) return -1;
+  return node_of[c];
+}
+
+// The components (numbered by their smallest node, as networkx does) in one CTA: every node first hooks onto
+// its smallest lower neighbour, pointer jumping flattens those trees (lines are long chains,
+// and a chain has almost no other edges), and only the edges to further lower neighbours
+// run the union of k_hook.  Writes comp, deg and the counts.
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    k_graph_small(const unsigned* __restrict__ bits, const int* __restrict__ cubes, const int* __restrict__ node_of,
+                  int* __restrict__ deg, int* __restrict__ comp, Grid g, int* flags) {
   extern __shared__ int sm_int[];
-  int* parent = sm_int;          // [n]
-  int* croot = sm_int + n;       // [n]: label, then component of each root
+  int* parent = sm_int;
+  int* croot = sm_int + kSmallNodes;
+  unsigned char* more = reinterpret_cast<unsigned char*>(croot + kSmallNodes);  // has further lower neighbours
   __shared__ int red[kSmallThreads / 32];
   __shared__ int run;
-  for (int v = threadIdx.x; v < n; v += kSmallThreads) parent[v] = v;
-  __syncthreads();
+  const int n = flags[3];
+  if (n > kSmallNodes) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int dsum = 0;
   for (int v = threadIdx.x; v < n; v += kSmallThreads) {
+    int nb[6], u[6];
+    const int cnt = face_neighbours(g, cubes[v], nb);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) u[q] = q < cnt ? node_at(bits, node_of, nb[q]) : -1;
+    int lo = v, low = 0, d = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      if (u[q] > v) ++d;
+      if (u[q] >= 0 && u[q] < v) {
+        ++low;
+        lo = min(lo, u[q]);
+      }
+    }
+    parent[v] = lo;
+    more[v] = low > 1;
+    deg[v] = d;
+    dsum += d;
+  }
+  for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+  if (lane == 0 && dsum) atomicAdd(&flags[2], dsum);
+  // pointer jumping until nothing moves (at most log2 of the longest chain rounds)
+  for (int it = 0; it < 32; ++it) {
+    __syncthreads();
+    bool moved = false;
+    for (int v = threadIdx.x; v < n; v += kSmallThreads) {
+      const int pa = parent[v], gp = *(volatile int*)&parent[pa];
+      if (gp != pa) {
+        parent[v] = gp;
+        moved = true;
+      }
+    }
+    if (!__syncthreads_or(moved)) break;
+  }
+  for (int v = threadIdx.x; v < n; v += kSmallThreads) {
+    if (!more[v]) continue;
     int nb[6];
     const int cnt = face_neighbours(g, cubes[v], nb);
-    int d = 0;
     for (int q = 0; q < cnt; ++q) {
-      const int u = node_of[nb[q]];
-      if (u <= v) continue;
-      ++d;
+      const int u = node_at(bits, node_of, nb[q]);
+      if (u < 0 || u >= v) continue;
       int a = v, b = u;
       for (int it = 0; it < kUfRetries; ++it) {
-        a = uf_find_s(parent, a, err);
-        b = uf_find_s(parent, b, err);
+        a = uf_find_s(parent, a, flags);
+        b = uf_find_s(parent, b, flags);
         if (a < 0 || b < 0 || a == b) break;
         if (a < b) {
           const int t = a;
@@ -347,17 +465,13 @@ __global__ void __launch_bounds__(kSmallThreads) k_components_small(const int* _
           b = t;
         }
         if (atomicCAS(parent + a, a, b) == a) break;
-        if (it == kUfRetries - 1) atomicExch(err, 1);
+        if (it == kUfRetries - 1) atomicExch(flags, 1);
       }
     }
-    deg[v] = d;
-    dsum += d;
   }
-  for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
-  if ((threadIdx.x & 31) == 0 && dsum) atomicAdd(n_edges, dsum);
   __syncthreads();
   for (int v = threadIdx.x; v < n; v += kSmallThreads) {
-    int r = uf_find_s(parent, v, err);
+    const int r = uf_find_s(parent, v, flags);
     croot[v] = r < 0 ? v : r;
   }
   __syncthreads();
@@ -365,31 +479,148 @@ __global__ void __launch_bounds__(kSmallThreads) k_components_small(const int* _
   if (threadIdx.x == 0) run = 0;
   __syncthreads();
   // roots numbered in node order: ordered block scan over slices of kSmallThreads
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int base = 0; base < n; base += kSmallThreads) {
     const int v = base + threadIdx.x;
     const bool f = v < n && parent[v] == v;
     const unsigned b = __ballot_sync(0xffffffffu, f);
     if (lane == 0) red[w] = __popc(b);
     __syncthreads();
-    int off = 0, tot = 0;
-    for (int q = 0; q < kSmallThreads / 32; ++q) {
-      off += (q < w) ? red[q] : 0;
-      tot += red[q];
+    const int c = red[lane];
+    int off = lane < w ? c : 0, tot = c;
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
     }
     if (f) croot[v] = run + off + __popc(b & ((1u << lane) - 1u));
     __syncthreads();
     if (threadIdx.x == 0) run += tot;
     __syncthreads();
   }
-  for (int v = threadIdx.x; v < n; v += kSmallThreads) {
-    const int c = croot[parent[v]];
-    comp[v] = c;
-    key[v] = c;
-    order[v] = v;
-  }
-  if (threadIdx.x == 0) *n_comp = run;
+  for (int v = threadIdx.x; v < n; v += kSmallThreads) comp[v] = croot[parent[v]];
+  if (threadIdx.x == 0) flags[1] = run;
 }
+
+// Nodes in component order (stable LSD radix sort, 8 bits a pass, as k_rs_hist and
+// k_rs_scatter: slices in order, warps in order, lanes ranked by match_any), their edge
+// offsets and the component offsets, in one CTA.
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    k_order_small(const int* __restrict__ comp, const int* __restrict__ deg, int* __restrict__ order,
+                  int* __restrict__ eoff, long long* __restrict__ comp_noff, long long* __restrict__ comp_eoff,
+                  const int* __restrict__ flags) {
+  extern __shared__ int sm_int[];
+  constexpr int NW = kSmallThreads / 32;
+  int* wc = sm_int;                                    // [warp][digit]
+  unsigned short* key = reinterpret_cast<unsigned short*>(wc + NW * 256);  // component of every node
+  unsigned short* va = key + kSmallNodes;
+  unsigned short* vb = va + kSmallNodes;
+  __shared__ int base[256];
+  __shared__ int red[NW];
+  __shared__ int run;
+  const int n = flags[3], nc = flags[1];
+  if (n > kSmallNodes || n == 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  for (int v = tid; v < n; v += kSmallThreads) {
+    key[v] = (unsigned short)comp[v];
+    va[v] = (unsigned short)v;
+  }
+  for (int t = tid; t < NW * 256; t += kSmallThreads) wc[t] = 0;
+  __syncthreads();
+  for (int shift = 0; ((nc - 1) >> shift) > 0; shift += 8) {
+    if (tid < 256) base[tid] = 0;
+    __syncthreads();
+    for (int v = tid; v < n; v += kSmallThreads) atomicAdd(&base[(key[va[v]] >> shift) & 255], 1);
+    __syncthreads();
+    if (w == 0) {  // exclusive scan of the 256 digit counts, 8 per lane
+      int c[8], s = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        c[q] = base[lane * 8 + q];
+        s += c[q];
+      }
+      int x = s;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      x -= s;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        base[lane * 8 + q] = x;
+        x += c[q];
+      }
+    }
+    __syncthreads();
+    for (int b0 = 0; b0 < n; b0 += kSmallThreads) {
+      const int i = b0 + tid;
+      const bool ok = i < n;
+      const int v = ok ? va[i] : 0;
+      const int d = ok ? (key[v] >> shift) & 255 : 256;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const int rank = __popc(peers & ((1u << lane) - 1u));
+      if (ok && lane == __ffs(peers) - 1) wc[w * 256 + d] = __popc(peers);
+      __syncthreads();
+      if (ok) {
+        int off = base[d] + rank;
+        for (int q = 0; q < w; ++q) off += wc[q * 256 + d];
+        vb[off] = (unsigned short)v;
+      }
+      __syncthreads();
+      if (tid < 256) {
+        int add = 0;
+#pragma unroll 8
+        for (int q = 0; q < NW; ++q) {
+          add += wc[q * 256 + tid];
+          wc[q * 256 + tid] = 0;
+        }
+        base[tid] += add;
+      }
+      __syncthreads();
+    }
+    unsigned short* t = va;
+    va = vb;
+    vb = t;
+  }
+  if (tid == 0) run = 0;
+  __syncthreads();
+  for (int b0 = 0; b0 < n; b0 += kSmallThreads) {
+    const int p = b0 + tid;
+    const bool ok = p < n;
+    const int v = ok ? va[p] : 0;
+    const int d = ok ? deg[v] : 0;
+    int x = d;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) red[w] = x;
+    __syncthreads();
+    const int c = red[lane];
+    int off = lane < w ? c : 0, tot = c;
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    }
+    const int e = run + off + x - d;
+    if (ok) {
+      order[p] = v;
+      eoff[p] = e;
+      const int cv = key[v];
+      if (p == 0 || key[va[p - 1]] != cv) {
+        comp_noff[cv] = p;
+        comp_eoff[cv] = e;
+      }
+      if (p == n - 1) {
+        comp_noff[nc] = n;
+        comp_eoff[nc] = e + d;
+      }
+    }
+    __syncthreads();
+    if (tid == 0) run += tot;
+    __syncthreads();
+  }
+}
+constexpr int kGraphSmem = kSmallNodes * (2 * (int)sizeof(int) + 1);
+constexpr int kOrderSmem = kSmallThreads / 32 * 256 * (int)sizeof(int) + 3 * kSmallNodes * (int)sizeof(unsigned short);
 
 __global__ void __launch_bounds__(kT) k_label(const int* __restrict__ label, const int* __restrict__ comp_of_root,
                                               int* __restrict__ comp, int* __restrict__ key, int* __restrict__ order,
@@ -413,10 +644,11 @@ __device__ __forceinline__ int block_excl_scan(int v, int* red, int* total) {
   }
   if (lane == 31) red[w] = x;
   __syncthreads();
-  int off = 0, tot = 0;
-  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-    off += (q < w) ? red[q] : 0;
-    tot += red[q];
+  const int c = lane < (int)(blockDim.x >> 5) ? red[lane] : 0;
+  int off = lane < w ? c : 0, tot = c;
+  for (int o = 16; o > 0; o >>= 1) {
+    off += __shfl_xor_sync(0xffffffffu, off, o);
+    tot += __shfl_xor_sync(0xffffffffu, tot, o);
   }
   __syncthreads();
   *total = tot;
@@ -531,12 +763,19 @@ __device__ __forceinline__ double scaled(int c, int a, const Grid& g) {
 
 // Node p of the component-sorted order writes its edges to the nodes above it, in
 // ascending order, and the offsets of its component when it is the component's first.
+// bits: set for a small frame, whose cube count is flags[3] and whose component offsets
+// k_order_small has written (comp null).
 __global__ void __launch_bounds__(kT) k_edges(const int* __restrict__ order, const int* __restrict__ eoff,
                                               const int* __restrict__ cubes, const int* __restrict__ node_of,
+                                              const unsigned* __restrict__ bits, const int* __restrict__ flags,
                                               const int* __restrict__ comp, Grid g, double* __restrict__ xyz,
                                               long long* __restrict__ comp_noff, long long* __restrict__ comp_eoff,
                                               int n, int n_comp, int n_edges) {
   const int p = blockIdx.x * kT + threadIdx.x;
+  if (bits) {
+    n = flags[3];
+    if (n > kSmallNodes) return;
+  }
   if (p >= n) return;
   const int v = order[p];
   const int c = cubes[v];
@@ -544,7 +783,7 @@ __global__ void __launch_bounds__(kT) k_edges(const int* __restrict__ order, con
   const int cnt = face_neighbours(g, c, nb);
   int up[6], m = 0;
   for (int q = 0; q < cnt; ++q) {
-    const int u = node_of[nb[q]];
+    const int u = node_at(bits, node_of, nb[q]);
     if (u > v) {
       int s = m++;
       while (s > 0 && up[s - 1] > u) {
@@ -569,6 +808,7 @@ __global__ void __launch_bounds__(kT) k_edges(const int* __restrict__ order, con
     o[4] = scaled(ju, 1, g);
     o[5] = scaled(ku, 2, g);
   }
+  if (!comp) return;
   const int cv = comp[v];
   if (p == 0 || comp[order[p - 1]] != cv) {
     comp_noff[cv] = p;
@@ -766,8 +1006,8 @@ class LinesEngine {
       cudaGetLastError();
       return fail(msg, "cannot create a stream on the device");
     }
-    if (cudaFuncSetAttribute(k_components_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmallNodes * 2 * (int)sizeof(int)) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_graph_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kGraphSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_order_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrderSmem) != cudaSuccess) {
       cudaGetLastError();
       return fail(msg, "cannot configure shared memory");
     }
@@ -777,6 +1017,11 @@ class LinesEngine {
         !node_of_.ensure(N, &device_bytes, st) || !counts_.ensure(nblocks(N, kChunk) + 1, &device_bytes, st) ||
         !flags_.ensure(4, &device_bytes, st) || cudaMallocHost((void**)&h_small_, 4 * sizeof(long long)) != cudaSuccess)
       return fail(msg, "device memory");
+    // a small frame's buffers at their full size: it is found without asking for its counts
+    if (!ensure_nodes(kSmallNodes) || !bits_.ensure((N + 31) / 32, &device_bytes, st) ||
+        !comp_noff_.ensure(kSmallNodes + 1, &device_bytes, st) || !comp_eoff_.ensure(kSmallNodes + 1, &device_bytes, st) ||
+        !xyz_.ensure(3ll * kSmallNodes * 6, &device_bytes, st))
+      return fail(msg, "device memory");
     return true;
   }
 
@@ -784,6 +1029,7 @@ class LinesEngine {
     for (Buf<int>* b : {&node_of_, &counts_, &sums_, &flags_, &cubes_, &parent_, &deg_, &label_, &root_comp_, &comp_,
                         &key_a_, &key_b_, &order_, &val_tmp_, &eoff_, &hist_, &diff32_})
       b->release();
+    bits_.release();
     th_.release();
     src_.release();
     xyz_.release();
@@ -849,6 +1095,29 @@ class LinesEngine {
     }
     const int nb = nblocks(N, kChunk);
     launch(k_faces, nblocks(N, kT), kT, th, face_.p, g);
+    {
+      if (!zero_small_counts(msg)) return RDCU_ERR_CUDA;
+      launch_small_marks();
+      launch_small_compact();
+      launch_small_graph();
+      launch_small_order();
+      launch_small_edges();
+      int* hf = reinterpret_cast<int*>(h_small_);
+      if (!ck(cudaMemcpyAsync(hf, flags_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st), msg) ||
+          !ck(cudaGetLastError(), msg) || !ck(cudaStreamSynchronize(st), msg))
+        return RDCU_ERR_CUDA;
+      if (hf[3] <= kSmallNodes) {
+        if (hf[0] != 0) return fail_code(msg, "union-find iteration bound reached", RDCU_ERR_TIMEOUT);
+        n_cubes = hf[3];
+        n_comp = hf[1];
+        n_edges = hf[2];
+        sorted_ = order_.p;
+        was_small_ = true;
+        have = true;
+        return RDCU_OK;
+      }
+    }
+    was_small_ = false;
     launch(k_mark, nb, kT, face_.p, mark_.p, counts_.p, g);
     int rc = scan(counts_.p, nb, msg);
     if (rc) return rc;
@@ -888,7 +1157,8 @@ class LinesEngine {
       sorted_ = v0;
       launch(k_edge_counts, nblocks(n, kT), kT, sorted_, deg_.p, eoff_.p, nn);
       if ((rc = scan(eoff_.p, nn, msg))) return rc;
-      launch(k_edges, nblocks(n, kT), kT, sorted_, eoff_.p, cubes_.p, node_of_.p, comp_.p, g, xyz_.p, comp_noff_.p,
+      launch(k_edges, nblocks(n, kT), kT, sorted_, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)nullptr,
+             (const int*)nullptr, comp_.p, g, xyz_.p, comp_noff_.p,
              comp_eoff_.p, nn, (int)nc, (int)ne);
     }
     if (!ck(cudaGetLastError(), msg)) return RDCU_ERR_CUDA;
@@ -926,6 +1196,26 @@ class LinesEngine {
       cudaEventRecord(ev[1], st);
       launch(k_faces, nblocks(N, kT), kT, th, face_.p, g);
       cudaEventRecord(ev[2], st);
+      if (was_small_) {
+        if (!zero_small_counts(msg)) return RDCU_ERR_CUDA;
+        launch_small_marks();
+        cudaEventRecord(ev[3], st);
+        launch_small_compact();
+        cudaEventRecord(ev[4], st);
+        launch_small_graph();
+        cudaEventRecord(ev[5], st);
+        launch_small_order();
+        cudaEventRecord(ev[6], st);
+        launch_small_edges();
+        cudaEventRecord(ev[7], st);
+        if (!ck(cudaEventSynchronize(ev[7]), msg)) rc = RDCU_ERR_CUDA;
+        for (int i = 0; i < 7 && rc == RDCU_OK; ++i) {
+          float ms = 0.f;
+          cudaEventElapsedTime(&ms, ev[i], ev[i + 1]);
+          acc[i] += ms;
+        }
+        continue;
+      }
       launch(k_mark, nb, kT, face_.p, mark_.p, counts_.p, g);
       rc = scan(counts_.p, nb, msg);
       cudaEventRecord(ev[3], st);
@@ -948,8 +1238,8 @@ class LinesEngine {
       if (nn > 0 && rc == RDCU_OK) {
         launch(k_edge_counts, nblocks(nn, kT), kT, v0, deg_.p, eoff_.p, nn);
         rc = scan(eoff_.p, nn, msg);
-        launch(k_edges, nblocks(nn, kT), kT, v0, eoff_.p, cubes_.p, node_of_.p, comp_.p, g, xyz_.p, comp_noff_.p,
-               comp_eoff_.p, nn, nc, ne);
+        launch(k_edges, nblocks(nn, kT), kT, v0, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)nullptr,
+               (const int*)nullptr, comp_.p, g, xyz_.p, comp_noff_.p, comp_eoff_.p, nn, nc, ne);
       }
       cudaEventRecord(ev[7], st);
       if (!ck(cudaEventSynchronize(ev[7]), msg)) rc = RDCU_ERR_CUDA;
@@ -1074,6 +1364,8 @@ class LinesEngine {
   Buf<double> th_, src_, xyz_;
   Buf<unsigned char> face_, mark_;
   Buf<int> node_of_, counts_, sums_, flags_;  // flags_[0]: error, flags_[1]: scan total
+  Buf<unsigned> bits_;                        // line cube marks of a small frame
+  bool was_small_ = false;                    // the last frame had at most kSmallNodes cubes
   Buf<int> cubes_, parent_, deg_, label_, root_comp_, comp_, key_a_, key_b_, order_, val_tmp_, eoff_, hist_, diff32_;
   Buf<long long> wide_, comp_noff_, comp_eoff_, diff64_, sets_;
   Buf<int4> packed_, packed_b_;
@@ -1118,16 +1410,31 @@ class LinesEngine {
       if (!b->ensure(n, &device_bytes, st)) return false;
     return hist_.ensure(256ll * (nblocks(n, kChunk) + 1), &device_bytes, st);
   }
+  int bit_words() const { return (g.total + 31) / 32; }
+  bool zero_small_counts(std::string* msg) {
+    return ck(cudaMemsetAsync(flags_.p, 0, 4 * sizeof(int), st), msg) &&
+           ck(cudaMemsetAsync(counts_.p, 0, nblocks(bit_words(), kBitWords) * sizeof(int), st), msg);
+  }
+  void launch_small_marks() { launch(k_mark_bits, nblocks(g.total, kT), kT, face_.p, bits_.p, counts_.p, g); }
+  void launch_small_compact() {
+    launch(k_compact_bits, nblocks(bit_words(), kBitWords), kBitWords, bits_.p, bit_words(), (const int*)counts_.p,
+           cubes_.p, node_of_.p, kSmallNodes, flags_.p);
+  }
+  void launch_small_graph() {
+    launch_smem(k_graph_small, 1, kSmallThreads, kGraphSmem, bits_.p, cubes_.p, node_of_.p, deg_.p, comp_.p, g, flags_.p);
+  }
+  void launch_small_order() {
+    launch_smem(k_order_small, 1, kSmallThreads, kOrderSmem, comp_.p, deg_.p, order_.p, eoff_.p, comp_noff_.p,
+                comp_eoff_.p, flags_.p);
+  }
+  void launch_small_edges() {
+    launch(k_edges, nblocks(kSmallNodes, kT), kT, order_.p, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)bits_.p,
+           (const int*)flags_.p, (const int*)nullptr, g, xyz_.p, comp_noff_.p, comp_eoff_.p, 0, 0, 0);
+  }
   // components of the n >= 1 line cubes (after k_compact): deg, comp, key_a_ and order_,
   // the component count in flags_[1], the edge count added to flags_[2] (zeroed by the
-  // caller).  One CTA in shared memory for small frames.
+  // caller)
   int components(int n, std::string* msg) {
-    if (n <= kSmallNodes) {
-      launch_smem(k_components_small, 1, kSmallThreads, (size_t)n * 2 * sizeof(int), (const int*)cubes_.p,
-                  (const int*)node_of_.p, deg_.p, comp_.p, key_a_.p, order_.p, n, g, flags_.p, flags_.p + 1,
-                  flags_.p + 2);
-      return ck(cudaGetLastError(), msg) ? RDCU_OK : RDCU_ERR_CUDA;
-    }
     const int nbn = nblocks(n, kChunk);
     launch(k_hook, nblocks(n, kT), kT, cubes_.p, node_of_.p, parent_.p, deg_.p, n, g, flags_.p, flags_.p + 2);
     launch(k_flatten, nbn, kT, parent_.p, label_.p, n, counts_.p, flags_.p);
