@@ -15,6 +15,7 @@
 
 #include "dp45.h"
 #include "dp45_ctl.cuh"
+#include "fft_line.cuh"
 
 namespace rdcu {
 
@@ -38,6 +39,7 @@ __global__ void k_dp45_arm(DP45Ctl* c, int check, double t1, double hmin, double
 __global__ void __launch_bounds__(kCtlThreads) k_dp45_ctl(DP45Ctl* c, const double* part, double* log_h,
                                                           double* log_t, int* log_acc, double nN,
                                                           const double* t_eval) {
+  chain_wait();
   dp45_control(c, part, log_h, log_t, log_acc, nN, t_eval);
 }
 
@@ -296,9 +298,8 @@ cudaError_t DP45Engine::launch_attempt_capture(double* const* ytemp_out) {
     RDCU_TRY(sp_->run(io[s], st_, s < 7 ? &io[s + 1] : nullptr, fwd_done, &fused));
     fwd_done = fused;
   }
-  k_dp45_ctl<<<1, kCtlThreads, 0, st_>>>(d_ctl_, err_part_, log_h_, log_t_, log_acc_, (double)nN_,
-                                         d_teval_);
-  return cudaGetLastError();
+  return launch_chain(sp_->chained(io[7]), k_dp45_ctl, 1, kCtlThreads, 0, st_, d_ctl_, (const double*)err_part_, log_h_,
+                      log_t_, log_acc_, (double)nN_, (const double*)d_teval_);
 }
 
 cudaError_t DP45Engine::ensure_graph() {

@@ -299,4 +299,24 @@ struct DP45Bufs {
 // Sets the message rdcu_last_error(NULL) returns on this thread (api.cu).
 void set_thread_error(const std::string& msg);
 
+#ifdef __CUDACC__
+// Launch of a kernel of a chain: with `chain`, its prologue may overlap the kernel before it
+// on the stream (which must be one that calls chain_wait(), or finish first).
+template <typename... KA, typename... A>
+inline cudaError_t launch_chain(bool chain, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chain ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+#endif
+
 }  // namespace rdcu

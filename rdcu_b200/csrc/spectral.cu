@@ -434,9 +434,6 @@ __device__ __forceinline__ void fwd_split(const double2* buf, int LS, int M, int
 template <int RS, int LX, int SF = 0>
 __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
   extern __shared__ double2 sm[];
-  if (a.io.mode == 1 && !a.io.ctl->running) return;
-  Resolved r = resolve(a.io);
-  r.nN = (long long)a.nrows * (LX ? LX : a.M);
   const int M = LX ? LX : a.M;
   const double2* tw = a.tw;
   double2* buf = sm;
@@ -446,6 +443,13 @@ __device__ __forceinline__ void fwd_x_body(const FwdXArgs& a, int bx) {
     tw = sm;
     buf = sm + M;
   }
+  chain_wait();
+  if (a.io.mode == 1 && !a.io.ctl->running) {
+    cp_async_wait_all();
+    return;
+  }
+  Resolved r = resolve(a.io);
+  r.nN = (long long)a.nrows * (LX ? LX : a.M);
   const long long row0 = 2LL * bx * a.P;
   // 16-byte state loads need 16-byte aligned arrays (a caller's y may be offset)
   unsigned long long align = reinterpret_cast<unsigned long long>(r.y) | reinterpret_cast<unsigned long long>(r.ytemp);
@@ -558,6 +562,13 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
   double* sA = reinterpret_cast<double*>(se + nse);
   double* skv = sA + (a.sorted ? a.ngrp * 16 : 0);
   int* soff = reinterpret_cast<int*>(skv + ((a.chan.kv_total + 1) & ~1));
+  const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
+  stage_table(se, a.sorted ? a.grp : a.chan.ent + a.ent0, nse * (int)sizeof(ChanEntry));
+  if (a.sorted) stage_table(sA, a.grpA, a.ngrp * 16 * (int)sizeof(double));
+  stage_table(skv, a.chan.kv, (a.chan.kv_total + 1) / 2 * 16);
+  if (!a.sorted)
+    for (int t = tid; t <= a.G; t += T) soff[t] = a.chan.off[a.ch0 + t] - a.ent0;
+  chain_wait();
   const long long i0 = (long long)bx * TW;
   const int nload = a.nsrc * L0 * TW;
   for (int e = tid; e < nload; e += T) {
@@ -568,12 +579,6 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
     cp_async16(&fb[(f * TW + c) * LS + z], in ? (const void*)&a.Sf[((long long)f * L0 + z) * a.I + ii] : (const void*)a.Sf,
                in);
   }
-  const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
-  stage_table(se, a.sorted ? a.grp : a.chan.ent + a.ent0, nse * (int)sizeof(ChanEntry));
-  if (a.sorted) stage_table(sA, a.grpA, a.ngrp * 16 * (int)sizeof(double));
-  stage_table(skv, a.chan.kv, (a.chan.kv_total + 1) / 2 * 16);
-  if (!a.sorted)
-    for (int t = tid; t <= a.G; t += T) soff[t] = a.chan.off[a.ch0 + t] - a.ent0;
   cp_async_wait_all();
   __syncthreads();
   fft_lines_x<RS, LX, false>(fb, LS, a.nsrc * TW, a.plan, tw, twz);
@@ -717,7 +722,7 @@ __device__ __forceinline__ void mid_body(const MidArgs& a, int bx) {
 }
 
 template <int RS, int LX>
-__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3)) k_mid(MidArgs a) {
+__global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3)) k_mid(const __grid_constant__ MidArgs a) {
   mid_body<RS, LX>(a, blockIdx.x);
 }
 
@@ -1433,6 +1438,16 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   int* sfb = reinterpret_cast<int*>(sfac + a.dict.nfac);
   int* sfold = sfb + n + 1;
   if (!a.Yout) {
+    stage_table(spoly, a.dict.poly, npoly * (int)sizeof(double));  // (npoly is even)
+    if (!a.dict.poly_nf) {
+      for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
+      for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
+      for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
+    }
+    for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
+  }
+  chain_wait();
+  if (!a.Yout) {
     // physical fields of the P rows: asynchronous 16-byte copies where rows and the
     // array's alignment allow (a caller's y may be only 8-byte aligned)
     if ((M & 1) == 0 && (reinterpret_cast<unsigned long long>(r.u) & 15) == 0) {
@@ -1513,15 +1528,6 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
       stage_older_slopes<2>(r2, n, PM, live, g0, RM, sy, ss);
     else
       stage_older_slopes<1>(r2, n, PM, live, g0, RM, sy, ss);
-  }
-  if (!a.Yout) {
-    stage_table(spoly, a.dict.poly, npoly * (int)sizeof(double));  // (npoly is even)
-    if (!a.dict.poly_nf) {
-      for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
-      for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
-      for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
-    }
-    for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
   }
   cp_async_wait_all();
   __syncthreads();
@@ -3550,6 +3556,14 @@ bool SpectralPlan::fuse_ok(const RhsIO& io, const RhsIO& next) const {
          next.stage == io.stage + 1 && !plane_inv_ok(io) && !plane_fwd_ok(next);
 }
 
+// Whether a stage's passes are launched as a chain (a kernel's start and its tables overlap
+// the kernel before it): the latency-bound 2D grids of the fused pass, within a DP45
+// attempt.  128 x 128 run: 2.79 -> 2.53 ms; 256 x 256, where fewer SMs are free for the waiting
+// kernel: 3.13 -> 3.09; adjoint 256 x 256: 39.3 -> 38.2.
+bool SpectralPlan::chained(const RhsIO& io) const {
+  return ndim == 2 && fuse_x_.per_cta > 0 && io.mode == 1 && io.stage >= 2;
+}
+
 bool SpectralPlan::fuse_x_ok(const RhsIO& io, const RhsIO& next) const {
   return fuse_x_.per_cta > 0 && !inv_row_ && io.mode == 1 && next.mode == 1 && io.ctl == next.ctl && io.stage >= 2 &&
          io.stage <= 6 && next.stage == io.stage + 1 && !next.err_aux && !plane_inv_ok(io) && !plane_fwd_ok(next);
@@ -3577,7 +3591,7 @@ cudaError_t SpectralPlan::launch_inv_fwd_x(const RhsIO& io, const RhsIO& next, c
   a.fuse_off = fuse_off_;
   prep(a);
   const PassCfg& g = fuse_x_;
-  by_length(plan_x_, g.block, [&](auto rs, auto lx) { k_inv_fwd_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
+  by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_inv_fwd_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
   return cudaGetLastError();
 }
 
@@ -3908,7 +3922,7 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
       RDCU_TRY(launch_mid_pipe(io, st));
     } else {
       prep(m);
-      by_length(plan_ax_[0], c.block, [&](auto rs, auto lx) { k_mid<decltype(rs)::value, decltype(lx)::value><<<c.grid, c.block, smem, st>>>(m); });
+      by_length(plan_ax_[0], c.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_mid<decltype(rs)::value, decltype(lx)::value>, c.grid, c.block, smem, st, m); });
       RDCU_TRY(cudaGetLastError());
     }
     if (ndim == 3 && !plane_inv) {
@@ -3989,7 +4003,7 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
     a.P = g.per_cta;
     a.tw_smem = tws;
     prep(a);
-    by_length(plan_x_, g.block, [&](auto rs, auto lx) { k_inv_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
+    by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
     RDCU_TRY(cudaGetLastError());
     if (!spectral) break;
   }

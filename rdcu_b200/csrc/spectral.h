@@ -98,6 +98,9 @@ class SpectralPlan {
   // the same with alpha read on the device from alpha_dev (captured solves)
   cudaError_t precond(const double* r, double* z, double alpha, const double* alpha_dev, cudaStream_t stream);
 
+  // the passes of this stage are launched as a chain (launch_chain)
+  bool chained(const RhsIO& io) const;
+
   int n = 0, ndim = 0, Ns[3] = {1, 1, 1};
   double Ls[3] = {1, 1, 1};
   long long N = 0;  // grid points
