@@ -47,7 +47,9 @@ void make_twiddles(int L, std::vector<double2>& tw) {
 
 void set_lin_ops(const std::vector<LinEntry>& lin, LinTable* t) {
   t->nops = 0;
+  t->real = 1;
   for (const LinEntry& e : lin) {
+    if (e.nax == 1) t->real = 0;
     int g = 0;
     while (g < t->nops && !(t->op[g].nax == e.nax && (e.nax < 1 || t->op[g].ax0 == e.ax0) &&
                             (e.nax < 2 || t->op[g].ax1 == e.ax1)))

@@ -248,6 +248,7 @@ constexpr int kMaxPrecFields = 4;  // per-mode dense solve size of the precondit
 constexpr int kMaxLinOps = 13;
 struct LinTable {
   int n, nops, ndim;
+  int real;  // every symbol is real (no first derivative)
   struct {
     int nax, ax0, ax1;
   } op[kMaxLinOps];
@@ -256,7 +257,7 @@ struct LinTable {
   const double* cosv;
   int off[3];
   int Ns[3];
-  double dx[3];
+  double idx[3];       // 1 / dx
   double alpha;        // preconditioner of I + alpha * J_lin
   const double* alpha_dev;  // when set, alpha is read from here (device-resident solves)
 };

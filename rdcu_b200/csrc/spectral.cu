@@ -1275,7 +1275,7 @@ struct MidSolveArgs {
 
 // NF: the largest field count of the mode solves (2, or kMaxPrecFields).  256 x 256, two
 // fields, one column per CTA: 15.6 us with the plan's called stages and 4 x 4 solves,
-// 9.6 us with the length's own stages and 2 x 2 solves.
+// 9.6 us with the length's own stages and 2 x 2 solves, 8.4 us with those by Cramer's rule.
 template <int RS, int LX, int NF>
 __global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2, 2)) k_mid_solve(const __grid_constant__ MidSolveArgs a) {
   extern __shared__ double2 sm[];
@@ -4209,7 +4209,7 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
   for (int a = 0; a < 3; ++a) {
     lt.off[a] = sc_off_[a];
     lt.Ns[a] = Ns[a];
-    lt.dx[a] = Ls[a] / Ns[a];
+    lt.idx[a] = Ns[a] / Ls[a];
   }
   if (ndim >= 2) {
     MidSolveArgs m{};
