@@ -80,14 +80,6 @@ __device__ __forceinline__ double root_sin(int k) {
   return R == 3 ? c_root3[k] : R == 5 ? c_root5[k + 1] : R == 7 ? c_root7[k + 2] : R == 11 ? c_root11[k + 4] : c_root13[k + 5];
 }
 
-// Programmatic dependent launch: waits for the kernels this one depends on (no effect in a
-// launch without the attribute), then lets the next kernel of the chain start its own
-// prologue.  Before the wait a kernel reads only what no kernel of the chain writes.
-__device__ __forceinline__ void chain_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // In-register R-point DFT of v (forward: exp(-2 pi i rk/R); inverse: conjugate).  Odd
 // primes: the sums and differences of the inputs r and R - r take the cosines and sines
 // of the definition, (R-1)^2 real-by-complex products and no table reads (a 5-point DFT

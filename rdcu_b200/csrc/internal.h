@@ -301,6 +301,14 @@ struct DP45Bufs {
 void set_thread_error(const std::string& msg);
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: waits for the kernels this one depends on (no effect in a
+// launch without the attribute), then lets the next kernel of the chain start its own
+// prologue.  Before the wait a kernel reads only what no kernel of the chain writes.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Launch of a kernel of a chain: with `chain`, its prologue may overlap the kernel before it
 // on the stream (which must be one that calls chain_wait(), or finish first).
 template <typename... KA, typename... A>

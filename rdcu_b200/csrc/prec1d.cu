@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(LX > 0 ? 256 : kLineThreads, 1) k_prec_line(co
   double2* X = buf + np * Q;   // its modes: [line][pair][side][b]
   const int nI = Q / 2 + 1, nP = pairs_of(Q, C);
   for (int t = tid; t < Q; t += T) tw[LX > 0 ? swz8(t) : t] = a.tw[t * C];
+  chain_wait();
   for (int p = 0; p < np; ++p) {
     const double* r0 = a.r + (long long)(2 * p) * N + rank;
     const bool two = 2 * p + 1 < n;

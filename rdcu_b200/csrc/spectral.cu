@@ -1283,6 +1283,7 @@ __global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 2, 2)) k_m
   double2* tw = sm;
   double2* fb = sm + L0;
   const bool twz = stage_twiddles<LX>(tw, a.tw, L0);
+  chain_wait();
   const long long i0 = (long long)blockIdx.x * TW;
   const int nload = n * L0 * TW;
   for (int e = tid; e < nload; e += T) {
@@ -4228,9 +4229,9 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
     by_length(plan_ax_[0], midsolve_.block, [&](auto rs, auto lx) {
       constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
       if (n <= 2)
-        k_mid_solve<RS, LX, 2><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
+        launch_chain(ndim == 2, k_mid_solve<RS, LX, 2>, midsolve_.grid, midsolve_.block, midsolve_.smem, st, m);
       else
-        k_mid_solve<RS, LX, kMaxPrecFields><<<midsolve_.grid, midsolve_.block, midsolve_.smem, st>>>(m);
+        launch_chain(ndim == 2, k_mid_solve<RS, LX, kMaxPrecFields>, midsolve_.grid, midsolve_.block, midsolve_.smem, st, m);
     });
     RDCU_TRY(cudaGetLastError());
     if (ndim == 3) {
@@ -4273,7 +4274,7 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
   a.P = g.per_cta;
   a.tw_smem = tws;
   prep(a);
-  by_length(plan_x_, g.block, [&](auto rs, auto lx) { k_inv_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
+  by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(ndim == 2, k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
   return cudaGetLastError();
 }
 
