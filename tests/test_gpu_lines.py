@@ -240,3 +240,35 @@ def test_prefetched_frames(cuda):
     assert same_components(hs[0].lines(), want_lines[2], Ns, Ls)
     for h in hs + [ref]:
         h.close()
+
+
+def test_frames_of_few_and_many_cubes(cuda):
+    """One handle over frames on both sides of the count up to which a frame is found with
+    one wait (12288 cubes), and empty ones, in both orders."""
+    Ns, Ls = (33, 31, 30), (9.0, 8.0, 7.0)
+    few = ol.phase(defect_state(Ns, 31, 0, 2, 0.1), Ns)
+    rng = np.random.default_rng(32)
+    many = rng.uniform(0, 2 * np.pi, Ns)
+    none = np.full(Ns, 1.0)
+    assert 0 < np.count_nonzero(ol.line_cubes(few)) <= 12288 < np.count_nonzero(ol.line_cubes(many))
+    h = _lines(Ns, Ls)
+    for th in (few, many, few, none, many, many, none, few):
+        h.find(np.ascontiguousarray(th).ravel(), 1)
+        if th is none:
+            assert h.lines() == []
+        else:
+            assert same_components(h.lines(), ol.findlines(th, Ns, Ls), Ns, Ls)
+    h.close()
+
+
+@pytest.mark.parametrize("span", [1.0, 3.0, 40.0])
+def test_phases_outside_one_turn(cuda, span):
+    """Phases are taken as they are: differences of many turns wind as numpy's floored modulus
+    says."""
+    Ns, Ls = (12, 11, 10), (3.0, 4.0, 5.0)
+    rng = np.random.default_rng(int(span) + 40)
+    th = rng.uniform(-span * np.pi, span * np.pi, Ns)
+    h = _lines(Ns, Ls)
+    h.find(th.ravel(), 1)
+    assert same_components(h.lines(), ol.findlines(th, Ns, Ls), Ns, Ls)
+    h.close()
