@@ -256,3 +256,20 @@ def test_plane_passes_3d(cuda, monkeypatch, Ns, kind):
         monkeypatch.delenv("RDCU_PLANE_PASSES")
         g, _ = gpu_rhs(cuda, prob, y)
         assert rel_err(f, g) < 1e-13
+
+
+@pytest.mark.parametrize("Ns", [(18, 22), (26, 28), (33, 35), (39, 45), (49, 90), (121, 169), (100, 112), (126, 144),
+                                (150, 180), (240, 250), (9, 15, 14), (10, 12, 96)])
+def test_every_radix_of_the_line_transforms(cuda, Ns):
+    """Lengths that take each odd prime and each composite radix (6, 9, 10, 12, 14, 15, 16)
+    as first, middle or last stage, on both sides of a grid."""
+    for shape in (Ns, Ns[::-1]):
+        rng = np.random.default_rng(sum(shape) * 13 + shape[0])
+        ndim = len(shape)
+        prob = Problem(2, shape, tuple(0.5 * v for v in shape), cgle_terms(ndim))
+        y = rng.uniform(-1, 1, 2 * prob.N)
+        f, Y = gpu_rhs(cuda, prob, y, want_Y=True)
+        fo, Yo = osp.rhs(y, prob, return_Y=True)
+        assert rel_err(f, fo) < TOL
+        for k in range(prob.nY * 2):
+            assert np.max(np.abs(Y[k] - Yo[k])) < TOL * max(np.max(np.abs(Yo[k])), 1e-300), (shape, k)
