@@ -24,6 +24,7 @@ struct FastDiv {
   int s;
 };
 inline FastDiv make_fastdiv(unsigned d) {
+  if (d == 0) d = 1;  // the tile width of a pass that the grid does not have
   int s = 0;
   while ((1ull << s) < d) ++s;
   const unsigned long long num = 1ull << (31 + s);

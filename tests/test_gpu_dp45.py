@@ -285,3 +285,18 @@ def test_fused_x_passes_are_the_separate_ones(cuda, monkeypatch, n, Ns, fixed):
     assert outs[0][:2] == outs[1][:2]
     np.testing.assert_array_equal(outs[0][2], outs[1][2])
     assert np.all(np.isfinite(outs[0][2])) and np.any(outs[0][2] != y0)
+
+
+@pytest.mark.parametrize("Ns", [(128, 128), (24, 18), (15, 9), (48,), (12, 10, 8)])
+@pytest.mark.parametrize("deriv", [True, False])
+def test_profile_passes_of_every_dimension(cuda, Ns, deriv):
+    """The pass times of grids that lack some of the passes (no axis 1, no axis 0, no
+    derivatives), and the state they leave alone."""
+    prob = Problem(2, Ns, tuple(0.8 * v for v in Ns), cgle_terms(len(Ns)) if deriv else
+                   [t for t in cgle_terms(len(Ns)) if all(k < 2 for k in t.ints[1::2])])
+    y0 = np.random.default_rng(3).uniform(-1, 1, 2 * prob.N)
+    s, yd = _setup(cuda, prob, y0)
+    s.set_state(0.0, 1e-3, yd.data_ptr())
+    names = [p[0] for p in s.profile_passes(reps=1)]
+    assert ("mid_axis0" in names) == (deriv and len(Ns) >= 2) and ("c2c_axis1_fwd" in names) == (deriv and len(Ns) == 3)
+    s.close()
