@@ -3135,9 +3135,12 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   if (poly_nf_) chk(upload_vec(&d_poly_, poly_table()));
   chk(upload_vec(&d_field_begin_, field_begin));
   chk(upload_vec(&d_fold_, fold_ch));
-  chk(upload_vec(&ych_off_, y_off));
-  chk(upload_vec(&ych_ent_, y_ent));
-  chk(upload_vec(&ych_dst_, y_dst));
+  if (!arena_) {  // (a plan in an arena writes no Y blocks; without these tables, which are
+                  // larger, the coefficients above take no more of it than the entries alone did)
+    chk(upload_vec(&ych_off_, y_off));
+    chk(upload_vec(&ych_ent_, y_ent));
+    chk(upload_vec(&ych_dst_, y_dst));
+  }
   if (!ok) return false;
 
   // ---- launch configurations
@@ -4191,10 +4194,6 @@ cudaError_t SpectralPlan::launch_forward(const double* y, cudaStream_t st) {
     RDCU_TRY(cudaGetLastError());
   }
   return cudaSuccess;
-}
-
-cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cudaStream_t st) {
-  return precond(r, z, alpha, nullptr, st);
 }
 
 cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, const double* alpha_dev,

@@ -94,8 +94,7 @@ class SpectralPlan {
   // the constant-coefficient linear FD operator of `lin` (solved mode by mode).
   bool init_precond(int n, int ndim, const int* Ns, const double* Ls, const std::vector<LinEntry>& lin,
                     std::string* msg);
-  cudaError_t precond(const double* r, double* z, double alpha, cudaStream_t stream);
-  // the same with alpha read on the device from alpha_dev (captured solves)
+  // alpha is read on the device from alpha_dev if that is set (captured solves)
   cudaError_t precond(const double* r, double* z, double alpha, const double* alpha_dev, cudaStream_t stream);
 
   // the passes of this stage are launched as a chain (launch_chain)
