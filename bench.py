@@ -299,8 +299,9 @@ def run_ours(args, rank, world, local_rank):
                    "window_sim_time": [T_A, T_B], "tau_per_step": TAU,
                    "accepted_steps": acc, "attempts": att, "parallelism": "replicas" if world > 1 else "single",
                    "l2": "inputs > L2 (no flush needed)"},
-        # the passes of six stages and the controller, per attempt
-        "gpu_launches": (sum(weights) + 1) * att * world,
+        # the passes of six stages and the controller, per attempt; in 2D the inverse pass of
+        # stages 2-6 and the next forward pass are one launch
+        "gpu_launches": (sum(weights) + 1 - fused_pairs_2d(Ns)) * att * world,
         "clocks": clk.summary(),
         "e2e": {"value": e2e_value, "unit": "grid-pt·steps/s", "h2d_bytes_per_step": nN * 8 / args.steps,
                 "d2h_bytes_per_step": 2 * nN * 8 / args.steps, "accepted_steps": acc2, "seconds": e2e_s},
@@ -927,6 +928,13 @@ def launches_per_attempt_of(name, names=()):
     if name.startswith("fwd_") or name.startswith("inv_"):
         return 5
     return 6
+
+
+def fused_pairs_2d(Ns):
+    """Pairs of x passes of an attempt that a 2D grid launches as one (see fuse_geometry in
+    spectral.cu: at most 592 rows, an even number of them)."""
+    fused = len(Ns) == 2 and Ns[0] % 2 == 0 and Ns[0] // 2 <= 296
+    return 5 if fused and os.environ.get("RDCU_FUSED_ROWS") != "0" else 0
 
 
 def cpu_baseline(Ns, Ls, y, t, h):
