@@ -269,7 +269,8 @@ constexpr int kMaxBlock = 512;
 __device__ __forceinline__ int swz8(int i) { return i ^ ((i >> 3) & 7); }
 
 // One Stockham stage over nlines lines (stride LS) held in shared memory `buf`.
-// Requires blockDim.x * QMAX >= nlines*L/R; the caller sizes the block for that.
+// Requires blockDim.x * QMAX >= nlines*L/R; the caller sizes the block for that.  QMAX,
+// the butterflies of a thread, fills at most kStageElems values by default.
 // POW2: L and Ns are powers of two (index arithmetic by shifts); otherwise the
 // plan's precomputed invariant divisors are used.
 // SWZ: bit 0 writes the outputs at swz8 positions (a first stage, Ns = 1, R = 8: its
@@ -278,12 +279,11 @@ __device__ __forceinline__ int swz8(int i) { return i ^ ((i >> 3) & 7); }
 // swz8 positions (the span-8 stage reads twiddles r*kk*L/64 for kk = 0..7, which
 // otherwise share a bank group).  Values are unchanged.
 // SWZ < 0: the flags swz instead (lines of a multiple of 8 points only).
-template <int R, bool INV, bool POW2, int SWZ = 0>
+template <int R, bool INV, bool POW2, int SWZ = 0, int QMAX = (R >= kStageElems ? 1 : kStageElems / R)>
 __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines, int L, int Ns, FastDiv dm,
                                                FastDiv dns, const double2* tw, bool twz = false, int swz = 0) {
   const bool swz_in = SWZ < 0 ? (swz & 2) != 0 : (SWZ & 2) != 0;
   const bool swz_out = SWZ < 0 ? (swz & 1) != 0 : (SWZ & 1) != 0;
-  constexpr int QMAX = (R >= kStageElems) ? 1 : (kStageElems / R);
   const int m = L / R;
   const int nb = nlines * m;
   const int T = blockDim.x;
@@ -338,6 +338,12 @@ constexpr int kRadixAll = 1;
 // radices up to 10 only: kernels of this set fit 80 registers where the full set takes 128
 // (and spills), which is half as many warps again for passes bound by latency
 constexpr int kRadixMid = 2;
+// the full set with ceil(8 / R) butterflies per thread, at least kStageElems values whatever
+// the radix: kMaxBlock threads then transform any kMaxBlock * kStageElems values.  For the
+// tiles whose radix-3, -5, -6 or -7 stages have more butterflies than the full set's block
+// (4000 = 16 x 10 x 5 x 5 points: 800 in a stage).  For all lengths it would cost up to 8%
+// (2D attempts, 300 x 330: 194 -> 210 us; 2000 x 1000: 1.34 -> 1.44 ms).
+constexpr int kRadixWide = 3;
 
 inline bool plan_is_pow2(const LinePlan& p) {
   for (int s = 0; s < p.nstages; ++s)
@@ -370,7 +376,9 @@ __device__ __forceinline__ void fft_lines(double2* buf, int LS, int nlines, cons
     const int swz = sw ? (s == 0 ? 1 : s == 1 ? 2 : 0) : 0;
 #define RDCU_STAGE(K, P2)                                                                          \
   case K:                                                                                         \
-    stockham_stage<K, INV, P2, -1>(buf, LS, nlines, L, Ns, dm, dns, tw, false, swz);               \
+    stockham_stage<K, INV, P2, -1, RS == kRadixWide ? (kStageElems + K - 1) / K                    \
+                                   : K >= kStageElems ? 1 : kStageElems / K>(                      \
+        buf, LS, nlines, L, Ns, dm, dns, tw, false, swz);                                          \
     break;
     if (RS == kRadixPow2) {
       switch (R) {

@@ -2537,7 +2537,10 @@ const void* group_kernel_for(int k, int L, int rs) {
     case 512: return group_kernel<kRadixPow2, 512>(k);
     case 96: return group_kernel<kRadixAll, 96>(k);
     case 192: return group_kernel<kRadixAll, 192>(k);
-    default: return rs == kRadixPow2 ? group_kernel<kRadixPow2, 0>(k) : group_kernel<kRadixAll, 0>(k);
+    default:
+      return rs == kRadixPow2 ? group_kernel<kRadixPow2, 0>(k)
+             : rs == kRadixWide ? group_kernel<kRadixWide, 0>(k)
+                                : group_kernel<kRadixAll, 0>(k);
   }
 }
 bool length_specialised(int L) { return L == 64 || L == 96 || L == 128 || L == 192 || L == 256 || L == 512; }
@@ -2589,7 +2592,6 @@ static int cta_elems() {
   return v;
 }
 
-int block_for(const LinePlan& p, int elems);
 int stage_threads(const LinePlan& p, int elems) {
   // each thread stages at most QMAX*R values per stage (see stockham_stage)
   int worst = kStageElems;
@@ -2599,6 +2601,14 @@ int stage_threads(const LinePlan& p, int elems) {
     worst = std::min(worst, per);
   }
   return (elems + worst - 1) / worst;
+}
+
+// The block of a pass whose CTAs transform `elems` (<= kMaxElems) values: as many threads as
+// the plan's stages need, or kMaxBlock of the wide radix set.
+void size_block(const LinePlan& p, int elems, PassCfg* c) {
+  const int t = stage_threads(p, elems);
+  c->wide = t > kMaxBlock;
+  c->block = std::min(kMaxBlock, std::max(128, round_up(t, 32)));
 }
 
 constexpr size_t kSmemBudget = 200 * 1024;
@@ -2643,7 +2653,6 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
   // a single problem spreads its rows over the GPU; a batch member only sizes its tiles
   int P = batch_elems > 0 ? std::max(1, std::min(batch_elems / (M * npm), R))
                           : std::max(1, std::min(std::max(1, cta_elems() / (M * npm)), R / kTargetCtas));
-  auto block_of = [&](int p) { return std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan, p * npm * M), 32))); };
   auto bytes = [&](int p, bool tws) {
     return (size_t)((spectral && tws ? M : 0) + (spectral ? p * np * M : 0)) * 16 +
            (yout ? 0 : ((size_t)p * n * M + 1) / 2 * 16 + extra);
@@ -2652,7 +2661,7 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
   const bool tws = bytes(P, true) <= kSmemBudget;
   c->per_cta = P;
   c->grid = (R + P - 1) / P;
-  c->block = block_of(P);
+  size_block(plan, P * npm * M, c);
   c->smem = bytes(P, tws);
   *tw_smem = tws ? 1 : 0;
 }
@@ -2661,13 +2670,15 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
 // while its CTAs are at most two per SM, where a pass's time is the latency of one tile and
 // a launch saved is worth more than the fused kernel's serial phases.  Above that the
 // separate passes are faster, with their smaller kernels (3D 100 x 96 x 80: 60 us fused
-// against 42 us; ensemble of 512: 169 against 141 ms).  per_cta 0: not taken.
+// against 42 us; ensemble of 512: 169 against 141 ms).  per_cta 0: not taken (nor where
+// its lines, twice a separate pass's, have more butterflies than a block).
 static void fuse_geometry(int M, int R, int n, int nch, const LinePlan& plan, size_t dict_bytes, PassCfg* c,
                           int* fuse_off) {
   const int lines = std::max(2 * ((nch + 1) / 2), n);  // complex lines of two rows
   const size_t off = ((size_t)(M + lines * M) * 16 + (size_t)2 * n * M * 8 + dict_bytes + 15) / 16 * 16;
   const size_t bytes = off + (size_t)4 * n * M * 8;
-  c->per_cta = R / 2 <= kTargetCtas && bytes <= kSmemBudget && lines * M <= kMaxElems ? 2 : 0;
+  const bool fits = bytes <= kSmemBudget && lines * M <= kMaxElems && stage_threads(plan, lines * M) <= kMaxBlock;
+  c->per_cta = R / 2 <= kTargetCtas && fits ? 2 : 0;
   c->grid = R / 2;
   c->block = std::min(kMaxBlock, std::max({128, round_up(stage_threads(plan, lines * M), 32), std::min(256, round_up(M, 32))}));
   c->smem = bytes;
@@ -2677,13 +2688,19 @@ static void fuse_geometry(int M, int R, int n, int nch, const LinePlan& plan, si
 // Calls f(radix set, line length) with compile-time values for the plan's lengths:
 // lines of 64..512 points (powers of two, and 96 and 192) get kernels specialised to
 // their length, other power-of-two lines the shift-indexed kernels, every other length
-// the general ones (those of radices up to 10 where the block allows).
+// the general ones (those of radices up to 10 where the block allows, the wide set where
+// the pass needs it).
 template <typename F>
-static void by_length(const LinePlan& p, int block, F&& f) {
+static void by_length(const LinePlan& p, const PassCfg& c, F&& f) {
   using RP = std::integral_constant<int, kRadixPow2>;
   using RA = std::integral_constant<int, kRadixAll>;
   using RM = std::integral_constant<int, kRadixMid>;
-  switch (block <= kSpecBlock ? p.L : 0) {
+  using RW = std::integral_constant<int, kRadixWide>;
+  if (c.wide) {
+    f(RW{}, std::integral_constant<int, 0>{});
+    return;
+  }
+  switch (c.block <= kSpecBlock ? p.L : 0) {
     case 64: f(RP{}, std::integral_constant<int, 64>{}); return;
     case 128: f(RP{}, std::integral_constant<int, 128>{}); return;
     case 256: f(RP{}, std::integral_constant<int, 256>{}); return;
@@ -2694,7 +2711,7 @@ static void by_length(const LinePlan& p, int block, F&& f) {
   }
   if (plan_is_pow2(p))
     f(RP{}, std::integral_constant<int, 0>{});
-  else if (block <= kSpecBlock && plan_is_mid(p))
+  else if (c.block <= kSpecBlock && plan_is_mid(p))
     f(RM{}, std::integral_constant<int, 0>{});
   else
     f(RA{}, std::integral_constant<int, 0>{});
@@ -2703,10 +2720,10 @@ static void by_length(const LinePlan& p, int block, F&& f) {
 // k_fwd_x on the plan's x lines: a kernel per stage (1..7; the stage of a DP45 launch, 1
 // for a plain evaluation) for 128- and 256-point rows, the runtime-stage kernel
 // otherwise.
-static void launch_fwd_x(const LinePlan& plan, int block, int grid, size_t smem, cudaStream_t st,
-                         const FwdXArgs& a) {
+static void launch_fwd_x(const LinePlan& plan, const PassCfg& c, size_t smem, cudaStream_t st, const FwdXArgs& a) {
   const int stage = a.io.mode == 1 ? std::max(1, a.io.stage) : 1;
-  by_length(plan, block, [&](auto rs, auto lx) {
+  const int grid = c.grid, block = c.block;
+  by_length(plan, c, [&](auto rs, auto lx) {
     constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
     if constexpr (LX == 128 || LX == 256) {
       switch (stage) {
@@ -3151,7 +3168,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
     const bool tws = (size_t)(M + P * M) * 16 <= kSmemBudget;
     fwd_.per_cta = P;
     fwd_.grid = (pairs + P - 1) / P;
-    fwd_.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_x_, P * M), 32)));
+    size_block(plan_x_, P * M, &fwd_);
     fwd_.smem = (size_t)((tws ? M : 0) + P * M) * 16;
   }
   if (((nch + 1) / 2) * M > kMaxElems) {
@@ -3201,7 +3218,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
       }
       PassCfg& c = mid_[which];
       c.grid = (I + TW - 1) / TW;
-      c.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_ax_[0], std::max(n, GB) * TW * L0), 32)));
+      size_block(plan_ax_[0], std::max(n, GB) * TW * L0, &c);
       c.smem = smem_of(TW, GB);
       if (which == 0 && mid_grp_ && nch <= GB && nch <= n)  // in-place channel lines (k_mid)
         c.smem = (size_t)(L0 + n * TW * tile_stride(L0, TW)) * 16 + extra;
@@ -3213,7 +3230,7 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
       while (TW > 1 && ((size_t)(La + TW * tile_stride(La, TW)) * 16 > kSmemBudget || TW * La > cta_elems())) TW /= 2;
       c2c_f_.per_cta = TW;
       c2c_f_.grid = (I1 + TW - 1) / TW;
-      c2c_f_.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_ax_[1], TW * La), 32)));
+      size_block(plan_ax_[1], TW * La, &c2c_f_);
       c2c_f_.smem = (size_t)(La + TW * tile_stride(La, TW)) * 16;
       c2c_i_ = c2c_f_;
     }
@@ -3238,10 +3255,14 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   // opt in to large dynamic shared memory (the limit is per block, static included)
   const int maxsm = 227 * 1024;
   bool optin_ok = true;
-  auto optin_all = [&](const LinePlan& pl) {
+  auto optin_all = [&](const LinePlan& pl, bool wide) {
     // the length-specialised kernels and the general ones larger blocks take
-    for (int blk : {kSpecBlock, kMaxBlock}) {
-      by_length(pl, blk, [&](auto rs, auto lx) {
+    PassCfg cfgs[3];
+    cfgs[0].block = kSpecBlock;
+    cfgs[1].block = kMaxBlock;
+    cfgs[2].wide = true;
+    for (int i = 0; i < (wide ? 3 : 2); ++i) {
+      by_length(pl, cfgs[i], [&](auto rs, auto lx) {
         constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
         optin_ok &= opt_in_smem((const void*)k_fwd_x<RS, LX>);
         if constexpr (LX == 128 || LX == 256) {
@@ -3254,15 +3275,17 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
           optin_ok &= opt_in_smem((const void*)k_fwd_x<RS, LX, 7>);
         }
         optin_ok &= opt_in_smem((const void*)k_inv_x<RS, LX>);
-        optin_ok &= opt_in_smem((const void*)k_inv_fwd_x<RS, LX>);
+        if constexpr (RS != kRadixWide) optin_ok &= opt_in_smem((const void*)k_inv_fwd_x<RS, LX>);
         optin_ok &= opt_in_smem((const void*)k_mid<RS, LX>);
         optin_ok &= opt_in_smem((const void*)k_c2c<RS, false, LX>);
         optin_ok &= opt_in_smem((const void*)k_c2c<RS, true, LX>);
       });
     }
   };
-  optin_all(plan_x_);
-  for (int ax = 0; ax + 1 < ndim; ++ax) optin_all(plan_ax_[ax]);
+  // (the channel pairs of the hot pass, of the Y blocks and of a preconditioner's fields)
+  optin_all(plan_x_, stage_threads(plan_x_, (std::max({nch, n, 1}) + 1) / 2 * M) > kMaxBlock);
+  for (int ax = 0; ax + 1 < ndim; ++ax)
+    optin_all(plan_ax_[ax], ax == 0 ? mid_[0].wide || mid_[1].wide : c2c_f_.wide);
   if (!optin_ok) {
     *msg = "cannot enable large shared memory for the FFT passes";
     return false;
@@ -3595,7 +3618,11 @@ cudaError_t SpectralPlan::launch_inv_fwd_x(const RhsIO& io, const RhsIO& next, c
   a.fuse_off = fuse_off_;
   prep(a);
   const PassCfg& g = fuse_x_;
-  by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_inv_fwd_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
+  by_length(plan_x_, g, [&](auto rs, auto lx) {
+    constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
+    if constexpr (RS != kRadixWide)  // (fuse_geometry: its lines have threads enough)
+      launch_chain(chained(io), k_inv_fwd_x<RS, LX>, g.grid, g.block, g.smem, st, a);
+  });
   return cudaGetLastError();
 }
 
@@ -3926,7 +3953,7 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
       RDCU_TRY(launch_mid_pipe(io, st));
     } else {
       prep(m);
-      by_length(plan_ax_[0], c.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_mid<decltype(rs)::value, decltype(lx)::value>, c.grid, c.block, smem, st, m); });
+      by_length(plan_ax_[0], c, [&](auto rs, auto lx) { launch_chain(chained(io), k_mid<decltype(rs)::value, decltype(lx)::value>, c.grid, c.block, smem, st, m); });
       RDCU_TRY(cudaGetLastError());
     }
     if (ndim == 3 && !plane_inv) {
@@ -3945,7 +3972,7 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
         RDCU_TRY(launch_c2c_pipe(true, nch_run * Ns[0], st, io, to_fused ? 0 : 1));
       } else {
         prep(a);
-        by_length(plan_ax_[1], c2c_i_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<grid, c2c_i_.block, c2c_i_.smem, st>>>(a); });
+        by_length(plan_ax_[1], c2c_i_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<grid, c2c_i_.block, c2c_i_.smem, st>>>(a); });
         RDCU_TRY(cudaGetLastError());
       }
     }
@@ -4007,7 +4034,7 @@ cudaError_t SpectralPlan::launch_passes(const RhsIO& io, const ChanTable& ct, co
     a.P = g.per_cta;
     a.tw_smem = tws;
     prep(a);
-    by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(chained(io), k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
+    by_length(plan_x_, g, [&](auto rs, auto lx) { launch_chain(chained(io), k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
     RDCU_TRY(cudaGetLastError());
     if (!spectral) break;
   }
@@ -4037,7 +4064,7 @@ cudaError_t SpectralPlan::run(const RhsIO& io, cudaStream_t st, const RhsIO* nex
     a.io = io;
     const size_t smem = spectral ? fwd_.smem : 0;
     prep(a);
-    launch_fwd_x(plan_x_, fwd_.block, fwd_.grid, smem, st, a);
+    launch_fwd_x(plan_x_, fwd_, smem, st, a);
     RDCU_TRY(cudaGetLastError());
   }
   if (spectral && ndim == 3) {
@@ -4054,7 +4081,7 @@ cudaError_t SpectralPlan::run(const RhsIO& io, cudaStream_t st, const RhsIO* nex
       RDCU_TRY(launch_c2c_pipe(false, n * Ns[0], st, io));
     } else {
       prep(a);
-      by_length(plan_ax_[1], c2c_f_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(a); });
+      by_length(plan_ax_[1], c2c_f_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(a); });
       RDCU_TRY(cudaGetLastError());
     }
   }
@@ -4079,7 +4106,7 @@ cudaError_t SpectralPlan::run_Y(const double* y, double* Yout, cudaStream_t st) 
   a.S = Sf_;
   a.io = io;
   prep(a);
-  launch_fwd_x(plan_x_, fwd_.block, fwd_.grid, fwd_.smem, st, a);
+  launch_fwd_x(plan_x_, fwd_, fwd_.smem, st, a);
   RDCU_TRY(cudaGetLastError());
   if (ndim == 3) {
     C2CArgs c{};
@@ -4092,7 +4119,7 @@ cudaError_t SpectralPlan::run_Y(const double* y, double* Yout, cudaStream_t st) 
     c.io = io;
     dim3 grid(c2c_f_.grid, n * Ns[0]);
     prep(c);
-    by_length(plan_ax_[1], c2c_f_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(c); });
+    by_length(plan_ax_[1], c2c_f_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(c); });
     RDCU_TRY(cudaGetLastError());
   }
   const ChanTable ct = chan_table(ych_off_, ych_ent_, ych_);
@@ -4146,10 +4173,10 @@ bool SpectralPlan::init_precond(int n_, int ndim_, const int* Ns_, const double*
     }
     midsolve_.per_cta = TW;
     midsolve_.grid = (I + TW - 1) / TW;
-    midsolve_.block = std::min(kMaxBlock, std::max(128, round_up(stage_threads(plan_ax_[0], n * TW * L0), 32)));
+    size_block(plan_ax_[0], n * TW * L0, &midsolve_);
     midsolve_.smem = smem_of(TW);
     bool ok = true;
-    by_length(plan_ax_[0], midsolve_.block, [&](auto rs, auto lx) {
+    by_length(plan_ax_[0], midsolve_, [&](auto rs, auto lx) {
       constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
       ok = opt_in_smem(n <= 2 ? (const void*)k_mid_solve<RS, LX, 2> : (const void*)k_mid_solve<RS, LX, kMaxPrecFields>);
     });
@@ -4177,7 +4204,7 @@ cudaError_t SpectralPlan::launch_forward(const double* y, cudaStream_t st) {
   a.S = Sf_;
   a.io = io;
   prep(a);
-  launch_fwd_x(plan_x_, fwd_.block, fwd_.grid, fwd_.smem, st, a);
+  launch_fwd_x(plan_x_, fwd_, fwd_.smem, st, a);
   RDCU_TRY(cudaGetLastError());
   if (ndim == 3) {
     C2CArgs c{};
@@ -4190,7 +4217,7 @@ cudaError_t SpectralPlan::launch_forward(const double* y, cudaStream_t st) {
     c.io = io;
     dim3 grid(c2c_f_.grid, n * Ns[0]);
     prep(c);
-    by_length(plan_ax_[1], c2c_f_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(c); });
+    by_length(plan_ax_[1], c2c_f_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<grid, c2c_f_.block, c2c_f_.smem, st>>>(c); });
     RDCU_TRY(cudaGetLastError());
   }
   return cudaSuccess;
@@ -4225,7 +4252,7 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
     m.Sc = Sc_;
     m.lin = lt;
     prep(m);
-    by_length(plan_ax_[0], midsolve_.block, [&](auto rs, auto lx) {
+    by_length(plan_ax_[0], midsolve_, [&](auto rs, auto lx) {
       constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
       if (n <= 2)
         launch_chain(ndim == 2, k_mid_solve<RS, LX, 2>, midsolve_.grid, midsolve_.block, midsolve_.smem, st, m);
@@ -4244,7 +4271,7 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
       a.io = RhsIO{};
       dim3 grid(c2c_i_.grid, n * Ns[0]);
       prep(a);
-      by_length(plan_ax_[1], c2c_i_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<grid, c2c_i_.block, c2c_i_.smem, st>>>(a); });
+      by_length(plan_ax_[1], c2c_i_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<grid, c2c_i_.block, c2c_i_.smem, st>>>(a); });
       RDCU_TRY(cudaGetLastError());
     }
   }
@@ -4273,7 +4300,7 @@ cudaError_t SpectralPlan::precond(const double* r, double* z, double alpha, cons
   a.P = g.per_cta;
   a.tw_smem = tws;
   prep(a);
-  by_length(plan_x_, g.block, [&](auto rs, auto lx) { launch_chain(ndim == 2, k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
+  by_length(plan_x_, g, [&](auto rs, auto lx) { launch_chain(ndim == 2, k_inv_x<decltype(rs)::value, decltype(lx)::value>, g.grid, g.block, g.smem, st, a); });
   return cudaGetLastError();
 }
 
@@ -4389,30 +4416,30 @@ cudaError_t SpectralPlan::profile(const RhsIO& io, int reps, cudaStream_t st, st
 
   auto go_fwd = [&]() -> cudaError_t {
     if (plane_fwd) return launch_plane_fwd(io, st);
-    launch_fwd_x(plan_x_, fwd_.block, fwd_.grid, fwd_.smem, st, fa);
+    launch_fwd_x(plan_x_, fwd_, fwd_.smem, st, fa);
     return cudaGetLastError();
   };
   auto go_c2c_f = [&]() -> cudaError_t {
     if (pipe_c2c_) return launch_c2c_pipe(false, n * Ns[0], st, io);
-    by_length(plan_ax_[1], c2c_f_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<gcf, c2c_f_.block, c2c_f_.smem, st>>>(cf); });
+    by_length(plan_ax_[1], c2c_f_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, false, decltype(lx)::value><<<gcf, c2c_f_.block, c2c_f_.smem, st>>>(cf); });
     return cudaGetLastError();
   };
   auto go_mid = [&]() -> cudaError_t {
     if (pipe_mid_) return launch_mid_pipe(io, st);
-    by_length(plan_ax_[0], mc.block, [&](auto rs, auto lx) { k_mid<decltype(rs)::value, decltype(lx)::value><<<mc.grid, mc.block, mc.smem, st>>>(m); });
+    by_length(plan_ax_[0], mc, [&](auto rs, auto lx) { k_mid<decltype(rs)::value, decltype(lx)::value><<<mc.grid, mc.block, mc.smem, st>>>(m); });
     return cudaGetLastError();
   };
   // rev: the axis-1 inverse pass's tile order (in order before the fused row pass)
   auto go_c2c_i = [&](int rev) -> cudaError_t {
     if (pipe_c2c_) return launch_c2c_pipe(true, nch * Ns[0], st, io, rev);
-    by_length(plan_ax_[1], c2c_i_.block, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<gci, c2c_i_.block, c2c_i_.smem, st>>>(ci); });
+    by_length(plan_ax_[1], c2c_i_, [&](auto rs, auto lx) { k_c2c<decltype(rs)::value, true, decltype(lx)::value><<<gci, c2c_i_.block, c2c_i_.smem, st>>>(ci); });
     return cudaGetLastError();
   };
   auto go_inv = [&]() -> cudaError_t {
     if (plane_inv) return launch_plane_inv(io, st);
     if (inv_row_ && !(io.mode == 1 && io.stage == 7 && io.err_part != nullptr && !io.err_aux))
       return launch_inv_row(io, st);
-    by_length(plan_x_, g.block, [&](auto rs, auto lx) { k_inv_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
+    by_length(plan_x_, g, [&](auto rs, auto lx) { k_inv_x<decltype(rs)::value, decltype(lx)::value><<<g.grid, g.block, g.smem, st>>>(a); });
     return cudaGetLastError();
   };
 
@@ -4576,10 +4603,10 @@ bool SpectralBatch::init(const std::vector<BatchMember>& members, int elems_, st
     size_t smem = 0;
   };
   std::map<std::pair<int, int>, Acc> acc[3];
-  auto add = [&](int k, int L, const LinePlan& plan, int block, size_t smem, int m, int ntiles) {
-    Acc& g = acc[k][{L, plan_is_pow2(plan) ? kRadixPow2 : kRadixAll}];
-    g.block = std::max(g.block, block);
-    g.smem = std::max(g.smem, smem);
+  auto add = [&](int k, int L, const LinePlan& plan, const PassCfg& c, int m, int ntiles) {
+    Acc& g = acc[k][{L, plan_is_pow2(plan) ? kRadixPow2 : c.wide ? kRadixWide : kRadixAll}];
+    g.block = std::max(g.block, c.block);
+    g.smem = std::max(g.smem, c.smem);
     for (int j = 0; j < ntiles; ++j) g.items.push_back(make_int2(m, j));
   };
   // a specialised length keeps its blocks within the specialised kernels' 256 threads
@@ -4597,8 +4624,10 @@ bool SpectralBatch::init(const std::vector<BatchMember>& members, int elems_, st
     const int Pf = std::max(1, std::min(elems_for(M) / M, pairs));
     const bool ftws = (size_t)(M + Pf * M) * 16 <= kSmemBudget;
     const int gf = (pairs + Pf - 1) / Pf;
-    add(0, M, p.plan_x_, std::min(kMaxBlock, std::max(128, round_up(stage_threads(p.plan_x_, Pf * M), 32))),
-        spectral ? (size_t)((ftws ? M : 0) + Pf * M) * 16 : 0, m, gf);
+    PassCfg gfw;
+    size_block(p.plan_x_, Pf * M, &gfw);
+    gfw.smem = spectral ? (size_t)((ftws ? M : 0) + Pf * M) * 16 : 0;
+    add(0, M, p.plan_x_, gfw, m, gf);
     // mid tiles: TW columns per item, every channel at once when the plan does so
     const int L0 = p.Ns[0], I = Mh;
     const int GBp = p.mid_[0].per_cta >> 16;
@@ -4615,15 +4644,17 @@ bool SpectralBatch::init(const std::vector<BatchMember>& members, int elems_, st
       return false;
     }
     const int gm = (I + TW - 1) / TW;
-    if (spectral)
-      add(1, L0, p.plan_ax_[0],
-          std::min(kMaxBlock, std::max(128, round_up(stage_threads(p.plan_ax_[0], std::max(n, GB) * TW * L0), 32))),
-          sorted && nch <= n ? (size_t)(L0 + n * TW * tile_stride(L0, TW)) * 16 + extra : smem_of(TW, GB), m, gm);
+    if (spectral) {
+      PassCfg gmd;
+      size_block(p.plan_ax_[0], std::max(n, GB) * TW * L0, &gmd);
+      gmd.smem = sorted && nch <= n ? (size_t)(L0 + n * TW * tile_stride(L0, TW)) * 16 + extra : smem_of(TW, GB);
+      add(1, L0, p.plan_ax_[0], gmd, m, gm);
+    }
     // inv_x tiles
     PassCfg gi;
     int itws = 0;
     inv_geometry(M, R, n, nch, false, p.plan_x_, &gi, &itws, p.dict_smem_bytes(), elems_for(M));
-    add(2, M, p.plan_x_, gi.block, gi.smem, m, gi.grid);
+    add(2, M, p.plan_x_, gi, m, gi.grid);
     for (int st = 1; st <= 7; ++st) {
       RhsIO io{};
       io.mode = 1;

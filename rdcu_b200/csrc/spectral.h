@@ -39,6 +39,7 @@ struct PassCfg {
   int grid = 0, block = 0;
   size_t smem = 0;
   int per_cta = 0;  // pairs / rows / columns per CTA
+  bool wide = false;  // the tile's stages need more threads than a block has (kRadixWide)
 };
 
 // Caller-provided device memory for a plan (bump allocation, never freed by the plan).

@@ -287,6 +287,31 @@ def test_fused_x_passes_are_the_separate_ones(cuda, monkeypatch, n, Ns, fixed):
     assert np.all(np.isfinite(outs[0][2])) and np.any(outs[0][2] != y0)
 
 
+# Lines whose radix-5, -6 or -7 stages have more than 512 butterflies in a CTA: the four
+# lines that the fused x passes hold for three fields or for three channels, the two of one
+# field (or of two fields in one channel pair).  3 steps of h = 1e-3 leave rounding
+# differences only: the file's bound for fixed steps, 1e-10.
+@pytest.mark.parametrize("n,Ns", [(3, (64, 650)), (3, (64, 750)), (3, (64, 875)), (3, (32, 910)), (1, (24, 1375)),
+                                  (1, (24, 2000)), (2, (24, 1375)), (2, (10, 1925))])
+def test_fixed_steps_of_many_butterflies(cuda, n, Ns):
+    from oracle.problem import parse_term
+
+    prob = Problem(n, Ns, tuple(0.7 * v for v in Ns), [parse_term(s) for s in _poly_terms(n, len(Ns))])
+    y0 = np.random.default_rng(sum(Ns)).uniform(-1, 1, n * prob.N)
+    s, yd = _setup(cuda, prob, y0, fixed=True)
+    s.set_state(0.0, 1e-3, yd)
+    s.advance(3)
+    out = cuda.empty_like(yd)
+    s.get_state(out)
+    s.close()
+    o = _oracle(prob, y0, True)
+    t = 0.0
+    for _ in range(3):
+        _, t, _ = o.step(t, 1e-3, 0.0, np.inf)
+        o.k[0] = o.k[6]
+    assert rel_err(out.cpu().numpy(), o.y) < 1e-10
+
+
 @pytest.mark.parametrize("Ns", [(128, 128), (24, 18), (15, 9), (48,), (12, 10, 8)])
 @pytest.mark.parametrize("deriv", [True, False])
 def test_profile_passes_of_every_dimension(cuda, Ns, deriv):

@@ -122,6 +122,21 @@ def test_finished_members_are_not_stepped(cuda):
     ens.close()
 
 
+@pytest.mark.parametrize("Ns", [(1375, 8), (8, 1750)])
+def test_members_of_many_butterflies(cuda, Ns):
+    """Lines with more radix-5 butterflies in a tile than a CTA has threads."""
+    import rdcu_b200 as R
+
+    members = [dict(n=2, Ns=Ns, Ls=(0.78 * Ns[0], 0.78 * Ns[1]), terms=_cgle(1.0, -0.5), rtol=1e-8, atol=1e-8)] * 2
+    ys = _ics(members, 9)
+    ens = R.Ensemble(members)
+    res = _run_ensemble(cuda, ens, members, ys, [0.0, 0.0], 1e-3, 0.05)
+    for m, y0, r in zip(members, ys, res):
+        ref = _single(cuda, m, y0, 0.0, 1e-3, 0.05)
+        assert r[3:] == ref[3:] and np.array_equal(r[0], ref[0])
+    ens.close()
+
+
 def test_error_paths(cuda):
     import rdcu_b200 as R
 

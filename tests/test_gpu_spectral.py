@@ -273,3 +273,23 @@ def test_every_radix_of_the_line_transforms(cuda, Ns):
         assert rel_err(f, fo) < TOL
         for k in range(prob.nY * 2):
             assert np.max(np.abs(Y[k] - Yo[k])) < TOL * max(np.max(np.abs(Yo[k])), 1e-300), (shape, k)
+
+
+# Radix-5, -6 or -7 stages of more than 512 butterflies: one line along the last axis (1D and
+# rows), two lines (fields) along axis 0, one line along axis 1, four channel lines
+@pytest.mark.parametrize("n,Ns", [(1, (2625,)), (2, (3750,)), (2, (4000,)), (2, (3969,)), (2, (1375, 8)), (2, (1750, 9)),
+                                  (2, (2000, 4)), (3, (875, 6)), (1, (4000, 3)), (2, (3, 2800)), (2, (2, 3125, 4))])
+def test_stages_of_many_butterflies(cuda, n, Ns):
+    rng = np.random.default_rng(sum(Ns) + n)
+    ndim = len(Ns)
+    lines = []
+    for i in range(n):
+        lines += ["1.0,%d,%d,1" % (i, i), "-1.0,%d,%d,3" % (i, i)]
+        lines += ["%s,%d,%d,1" % (1.0 + 0.2 * i, i, n + ndim * n + (a * ndim + a) * n + (i + 1) % n) for a in range(ndim)]
+    prob = Problem(n, Ns, tuple(0.5 * v for v in Ns), [parse_term(s) for s in lines])
+    y = rng.uniform(-1, 1, n * prob.N)
+    f, Y = gpu_rhs(cuda, prob, y, want_Y=True)
+    fo, Yo = osp.rhs(y, prob, return_Y=True)
+    assert rel_err(f, fo) < TOL
+    for k in range(prob.nY * n):
+        assert np.max(np.abs(Y[k] - Yo[k])) < TOL * max(np.max(np.abs(Yo[k])), 1e-300), k
