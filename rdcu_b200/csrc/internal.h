@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <array>
 #include <cstdint>
 #include <string>
@@ -300,6 +301,21 @@ struct DP45Bufs {
 
 // Sets the message rdcu_last_error(NULL) returns on this thread (api.cu).
 void set_thread_error(const std::string& msg);
+
+// Allows a kernel the largest dynamic shared memory the device grants next to its static
+// shared memory (*limit, in bytes).  The limit belongs to the function, whatever handle
+// launches it: set to one handle's size, it would fail the launches of another that needs
+// more.
+inline bool opt_in_smem(const void* func, size_t* limit = nullptr) {
+  cudaFuncAttributes fa;
+  if (cudaFuncGetAttributes(&fa, func) != cudaSuccess) return false;
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
+  const int dyn = optin - (int)fa.sharedSizeBytes;
+  if (limit) *limit = (size_t)std::max(0, dyn);
+  return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess;
+}
 
 #ifdef __CUDACC__
 // Programmatic dependent launch: waits for the kernels this one depends on (no effect in a

@@ -247,8 +247,8 @@ bool LinePrecond::init(int n, int N, double L, const std::vector<LinEntry>& lin)
   set_lin_ops(lin, &lin_);
   bool ok = put(&tw_, tw, &device_bytes) && put(&sinv_, sv, &device_bytes) &&
             put(&cosv_, cv, &device_bytes);
-  ok = ok && cudaFuncSetAttribute((const void*)kernel_of(C_, N_ / C_, n_), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)line_smem(Q, C_, np)) == cudaSuccess;
+  size_t limit = 0;
+  ok = ok && opt_in_smem((const void*)kernel_of(C_, Q, n_), &limit) && line_smem(Q, C_, np) <= limit;
   if (!ok) {
     cudaGetLastError();
     release();

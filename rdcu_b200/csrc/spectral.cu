@@ -2622,18 +2622,6 @@ constexpr int kTargetCtas = 2 * 148;
     if (_e != cudaSuccess) return _e;      \
   } while (0)
 
-// Allows a kernel the largest dynamic shared memory the device grants next to its
-// static shared memory.
-static bool opt_in_smem(const void* func) {
-  cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, func) != cudaSuccess) return false;
-  int dev = 0, optin = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
-  const int dyn = optin - (int)fa.sharedSizeBytes;
-  return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess;
-}
-
 // Columns per tile of a strided pass over I columns, before the shared-memory limits halve
 // it: a power of two, so that a tile's row is whole 32-byte sectors (3 columns: 48 bytes),
 // that leaves two CTAs per SM.

@@ -218,3 +218,33 @@ def test_line_preconditioner_matches_direct_solves(cuda, n, N):
     assert np.max(np.abs(np.array(h) - oh) / np.abs(oh)) < 1e-8  # the tolerance of the oracle comparison above
     for a, b in zip(states, ost):
         assert rel_err(a, b) < 1e-8
+
+
+def test_a_shorter_line_leaves_a_longer_one_alone(cuda):
+    """Two live handles whose line preconditioners are the same kernel (clusters of eight) with
+    different shared memory: the longer line solves as it does alone."""
+    import rdcu_b200 as R
+
+    def handle(N):
+        prob = Problem(2, (N,), (0.05 * N,), cgle_terms(1))
+        x = np.arange(N) / N
+        return _solver(prob, rtol=1e-6, atol=1e-6), np.concatenate([np.cos(2 * np.pi * x), 0.5 * np.sin(4 * np.pi * x)])
+
+    def run(s, y0):
+        s.set_state(0.0, 1e-4, np.array(y0))
+        s.solve(0.01, [])
+        out = np.empty_like(y0)
+        s.get_state(out)
+        iters, solves, _ = s.linear_stats()
+        assert 0 < iters <= 20 * solves  # preconditioned
+        return out
+
+    a, ya = handle(16384)
+    alone = run(a, ya)
+    a.close()
+    a, ya = handle(16384)
+    b, yb = handle(12000)
+    np.testing.assert_array_equal(run(a, ya), alone)
+    run(b, yb)
+    a.close()
+    b.close()
