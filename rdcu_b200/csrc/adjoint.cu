@@ -596,19 +596,21 @@ bool AdjointEngine::init(SpectralPlan* fwd, DP45Engine* dp, const std::vector<Ho
                       : n == 2 ? poly_smem<2>(T.nkept, T.nfold)
                                : poly_smem<3>(T.nkept, T.nfold);
     const void* fn = n == 1 ? (const void*)k_adj_poly<1> : n == 2 ? (const void*)k_adj_poly<2> : (const void*)k_adj_poly<3>;
-    if (dense && sm <= 200 * 1024 &&
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess) {
+    size_t limit = 0;
+    if (dense && sm <= 200 * 1024 && opt_in_smem(fn, &limit) && sm <= limit) {
       T.poly_nf = n;
       pw_smem_ = sm;
     } else {
       cudaGetLastError();
     }
   }
-  if (!T.poly_nf) pw_smem_ = pointwise_smem(n, nq_, T.nkept, T.nfac);
-  if (!T.poly_nf && pw_smem_ > 48 * 1024 &&
-      cudaFuncSetAttribute(k_adj_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pw_smem_) != cudaSuccess) {
-    *msg = "adjoint set-up: dictionary too large for the pointwise kernel's shared memory";
-    return false;
+  if (!T.poly_nf) {
+    pw_smem_ = pointwise_smem(n, nq_, T.nkept, T.nfac);
+    size_t limit = 0;
+    if (!opt_in_smem((const void*)k_adj_stage, &limit) || pw_smem_ > limit) {
+      *msg = "adjoint set-up: dictionary too large for the pointwise kernel's shared memory";
+      return false;
+    }
   }
   const size_t sb = (size_t)nN_ * sizeof(double);
   auto fail = [&](const char* w) {

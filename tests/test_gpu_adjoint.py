@@ -292,3 +292,37 @@ def test_adjoint_duality_dense_polynomial(cuda, n, Ns):
     rhs = float(gy.cpu().numpy() @ dy) + float(gC @ dC)
     # eps^2 for the third derivative, rounding / eps for the difference
     assert abs(lhs - rhs) <= 1e-6 * (np.linalg.norm(w) * np.linalg.norm(dy))
+
+
+def _derivative_products(nq):
+    """n = 2 in 2D: products of the first nq derivative quantities (Y index 2..13) with a field, and
+    cubic terms: the term-list stage kernel (k_adj_stage)."""
+    lines = ["1.0,0,0,1", "-1.0,0,0,3", "1.0,1,1,1", "-1.0,1,1,3"]
+    lines += ["0.01,%d,%d,1,%d,1" % (q % 2, 2 + q, (q + 1) % 2) for q in range(nq)]
+    return lines
+
+
+# The larger handle's kernel needs more shared memory than the smaller one's, which is
+# created (and run) between the two runs of the larger.
+@pytest.mark.parametrize("kind", ["dense", "terms"])
+def test_a_smaller_handle_leaves_a_larger_one_alone(cuda, kind):
+    from oracle.problem import parse_term
+
+    rng = np.random.default_rng(23)
+    if kind == "dense":
+        big = Problem(2, (16, 12), (12.0, 9.0), cgle_terms(2))
+        small = Problem(2, (24,), (18.0,), cgle_terms(1)[:6])
+    else:
+        big = Problem(2, (16, 12), (12.0, 9.0), [parse_term(s) for s in _derivative_products(12)])
+        small = Problem(2, (16, 12), (12.0, 9.0), [parse_term(s) for s in _derivative_products(9)])
+    hs = [1e-3, 2e-3]
+    data = [(smooth_field(rng, p, amp=0.5), rng.normal(size=p.n * p.N)) for p in (big, small)]
+    a = _solver(big)
+    first = _grads(cuda, a, data[0][0], hs, 1, data[0][1])
+    b = _solver(small)
+    _grads(cuda, b, data[1][0], hs, 1, data[1][1])
+    again = _grads(cuda, a, data[0][0], hs, 1, data[0][1])
+    for x, y in zip(first, again):
+        np.testing.assert_array_equal(x, y)
+    a.close()
+    b.close()
