@@ -326,3 +326,41 @@ def test_a_smaller_handle_leaves_a_larger_one_alone(cuda, kind):
         np.testing.assert_array_equal(x, y)
     a.close()
     b.close()
+
+
+# k_adj_poly (a dense polynomial) against k_adj_stage, which the same dictionary takes with a
+# term of degree 4 and coefficient 0: the same sums in another order.  Point counts below a
+# block, with part of a block at the end, and beyond the grid's 296 blocks of 256 threads.  Bounds:
+# 1e-12 of the largest value of dL/dy0, and 1e-12 of the sum of magnitudes h sum |w| m that makes
+# up a coefficient's gradient (|m| <= 1 for the monomials of |u| < 1, a few for the Laplacians).
+@pytest.mark.parametrize("n,Ns", [(1, (6, 7)), (1, (200, 400)), (2, (15, 33)), (2, (300, 256)), (3, (5, 9, 8)),
+                                  (3, (280, 275))])
+def test_dense_polynomial_stage_is_the_term_list_one(cuda, n, Ns):
+    from oracle.problem import parse_term
+
+    rng = np.random.default_rng(n + sum(Ns))
+    ndim = len(Ns)
+    lines = []
+    for i in range(n):
+        j = (i + 1) % n
+        lines += ["0.7,%d,%d,1" % (i, i), "-1.0,%d,%d,3" % (i, i), "0.4,%d,%d,1,%d,2" % (i, i, j) if j != i else "0.2,0,0,2",
+                  "0.3,%d" % i, "-0.6,%d,%d,2" % (i, j)]
+        if n == 3:
+            lines.append("0.5,%d,0,1,1,1,2,1" % i)
+        lines += ["%s,%d,%d,1" % (1.0 + 0.2 * i, i, n + ndim * n + (a * ndim + a) * n + j) for a in range(ndim)]
+    hs = [1e-2, 2e-2, 1.5e-2]
+    y0 = 0.9 * smooth_field(rng, Problem(n, Ns, tuple(1.0 * v for v in Ns), []), amp=0.2, modes=2)
+    y0 = np.clip(y0, -0.9, 0.9)
+    w = rng.normal(size=y0.size)
+    res = []
+    for extra in ([], ["0.0,0,0,4"]):
+        prob = Problem(n, Ns, tuple(1.0 * v for v in Ns), [parse_term(s) for s in lines + extra])
+        s = _solver(prob)
+        res.append(_grads(cuda, s, y0, hs, 2, w))
+        s.close()
+    (yTa, ga, Ca), (yTb, gb, Cb) = res
+    assert rel_err(yTa, yTb) < 1e-12
+    assert rel_err(ga, gb) < 1e-12
+    assert np.max(np.abs(ga - w)) > 1e-3 * np.max(np.abs(w))  # the steps' own part is well above the bound
+    assert np.max(np.abs(Ca - Cb[:-1])) < 1e-12 * sum(hs) * np.sum(np.abs(w))
+    assert np.min(np.abs(Ca)) > 1e-9 * sum(hs) * np.sum(np.abs(w))
