@@ -3387,7 +3387,8 @@ void SpectralPlan::setup_pipes() {
   if (!encode_rows(&tm_sf_, Sf_, 2 * I, (long long)n * Ns[0], Ns[0]) || !encode_sc_map()) return;
   const void* fn = Ns[0] == 128 ? (mid_tab_ ? (const void*)k_mid_pipe<128, true> : (const void*)k_mid_pipe<128, false>)
                                 : (mid_tab_ ? (const void*)k_mid_pipe<256, true> : (const void*)k_mid_pipe<256, false>);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  size_t limit = 0;
+  if (!opt_in_smem(fn, &limit) || smem > limit) {  // (the tables, hence smem, differ from plan to plan)
     cudaGetLastError();
     return;
   }

@@ -293,3 +293,24 @@ def test_stages_of_many_butterflies(cuda, n, Ns):
     assert rel_err(f, fo) < TOL
     for k in range(prob.nY * n):
         assert np.max(np.abs(Y[k] - Yo[k])) < TOL * max(np.max(np.abs(Yo[k])), 1e-300), k
+
+
+def test_a_smaller_grid_leaves_a_larger_one_alone(cuda):
+    """Two live handles of the tiled axis-0 pass whose tables differ in size (a mixed
+    derivative: k_mid_pipe), the smaller created between two runs of the larger."""
+    terms = [parse_term(s) for s in ["1.0,0,0,1", "0.7,0,5,1", "0.5,0,4,1", "0.3,0,12,1", "-1.0,0,0,3"]]
+    big = Problem(1, (256, 60, 64), (50.0, 20.0, 20.0), terms)
+    small = Problem(1, (256, 4, 6), (50.0, 4.0, 6.0), terms)
+    y = np.random.default_rng(2).uniform(-1, 1, big.N)
+    a = _solver(big)
+    yd = cuda.tensor(y, device="cuda")
+    f = [cuda.empty_like(yd) for _ in range(2)]
+    cuda.cuda.synchronize()
+    a.rhs(yd, f[0])
+    b = _solver(small)
+    a.rhs(yd, f[1])
+    cuda.cuda.synchronize()
+    assert rel_err(f[0].cpu().numpy(), osp.rhs(y, big)) < TOL
+    assert cuda.equal(f[0], f[1])
+    a.close()
+    b.close()
