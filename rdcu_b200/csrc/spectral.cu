@@ -2613,6 +2613,8 @@ void size_block(const LinePlan& p, int elems, PassCfg* c) {
 
 constexpr size_t kSmemBudget = 200 * 1024;
 constexpr int kTargetCtas = 2 * 148;
+// Largest number of lines (in all CTAs) of a fused x pass that is chained: 128 CTAs of two
+constexpr int kChainLines = 2 * 128;
 
 }  // namespace
 
@@ -2654,23 +2656,35 @@ static void inv_geometry(int M, int R, int n, int nch_run, bool yout, const Line
   *tw_smem = tws ? 1 : 0;
 }
 
-// Geometry of the fused inverse/forward x pass: two rows per CTA, 256 threads.  It is taken
-// while its CTAs are at most two per SM, where a pass's time is the latency of one tile and
-// a launch saved is worth more than the fused kernel's serial phases.  Above that the
-// separate passes are faster, with their smaller kernels (3D 100 x 96 x 80: 60 us fused
-// against 42 us; ensemble of 512: 169 against 141 ms).  per_cta 0: not taken (nor where
-// its lines, twice a separate pass's, have more butterflies than a block).
+// Geometry of the fused inverse/forward x pass: two rows per CTA in 128 to 512 threads.  It
+// is taken while its CTAs run at once, at most two per SM (init looks whether two fit where
+// they have to): a pass's time is then the latency of one tile, and a launch saved is worth
+// more than the fused kernel's serial phases.  Otherwise the separate passes are faster,
+// with their smaller kernels (3D 100 x 96 x 80: 60 us fused against 42 us; ensemble of 512:
+// 169 against 141 ms).  2D attempts of two fields, us, fused and separate: 64 x 250 100 and
+// 121, 256 x 512 127 and 143, 512 x 250 152 and 165, 588 x 512 201 and 218, 128 x 1000 158
+// and 176, 256 x 1400 253 and 260.  Where a CTA has an SM to itself (shared memory, or more than
+// 256 threads) and the CTAs are more than the SMs: 300 x 1000 300 and 247, 384 x 1200 382 and
+// 306, 512 x 900 329 and 277; but 512 x 1200 406 and 446, 588 x 1280 671 and 733, where the
+// ten state and slope arrays take more than two thirds of L2 and the separate passes wait for
+// memory: the fused pass stays there.  Three fields (or channels: four lines in
+// a CTA), 256 threads and less: 128 x 256 109 and 113, 384 x 512 212 and 213; more:
+// 64 x 640 184 and 166, 256 x 640 217 and 209, hence at most 2048 values then.
+// per_cta 0: not taken (nor where its lines, twice a separate pass's, have more butterflies
+// than a block).  *chain: the attempt's kernels are launched as a chain (SpectralPlan::chained).
 static void fuse_geometry(int M, int R, int n, int nch, const LinePlan& plan, size_t dict_bytes, PassCfg* c,
-                          int* fuse_off) {
+                          int* fuse_off, bool* chain) {
   const int lines = std::max(2 * ((nch + 1) / 2), n);  // complex lines of two rows
   const size_t off = ((size_t)(M + lines * M) * 16 + (size_t)2 * n * M * 8 + dict_bytes + 15) / 16 * 16;
   const size_t bytes = off + (size_t)4 * n * M * 8;
-  const bool fits = bytes <= kSmemBudget && lines * M <= kMaxElems && stage_threads(plan, lines * M) <= kMaxBlock;
+  const bool fits = bytes <= kSmemBudget && lines * M <= (lines > 2 ? kMaxElems / 2 : kMaxElems) &&
+                    stage_threads(plan, lines * M) <= kMaxBlock;
   c->per_cta = R / 2 <= kTargetCtas && fits ? 2 : 0;
   c->grid = R / 2;
   c->block = std::min(kMaxBlock, std::max({128, round_up(stage_threads(plan, lines * M), 32), std::min(256, round_up(M, 32))}));
   c->smem = bytes;
   *fuse_off = (int)(off / 8);
+  *chain = c->per_cta > 0 && c->grid * lines <= kChainLines;
 }
 
 // Calls f(radix set, line length) with compile-time values for the plan's lengths:
@@ -3172,8 +3186,9 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   // (RDCU_FUSED_ROWS=0 keeps the passes separate)
   const char* fz = getenv("RDCU_FUSED_ROWS");
   fuse_x_ = {};
+  chain_x_ = false;
   if (nch > 0 && poly_nf_ > 0 && R % 2 == 0 && !explicit_channels_ && !(fz && fz[0] == '0'))
-    fuse_geometry(M, R, n, nch, plan_x_, dict_smem_bytes(), &fuse_x_, &fuse_off_);
+    fuse_geometry(M, R, n, nch, plan_x_, dict_smem_bytes(), &fuse_x_, &fuse_off_, &chain_x_);
   nparts_max = R;  // stage-7 error partials: one per grid row
   // Y-mode channel group
   const int GY = std::min(ych_, 8);
@@ -3277,6 +3292,30 @@ bool SpectralPlan::init(int n_, int ndim_, const int* Ns_, const double* Ls_,
   if (!optin_ok) {
     *msg = "cannot enable large shared memory for the FFT passes";
     return false;
+  }
+  // the fused pass's CTAs at once, or data beyond L2 (see fuse_geometry; a CTA per SM always fits)
+  int dev = 0, nsm = 0, l2 = 0;
+  if (fuse_x_.per_cta > 0 && cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess && fuse_x_.grid > nsm) {
+    int per_sm = 0;
+    by_length(plan_x_, fuse_x_, [&](auto rs, auto lx) {
+      constexpr int RS = decltype(rs)::value, LX = decltype(lx)::value;
+      if constexpr (RS != kRadixWide)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inv_fwd_x<RS, LX>, fuse_x_.block, fuse_x_.smem) !=
+            cudaSuccess) {
+          cudaGetLastError();
+          per_sm = 0;
+        }
+    });
+    if (fuse_x_.grid > per_sm * nsm) {
+      if (10LL * 8 * n * N <= l2 / 3 * 2LL) {
+        fuse_x_ = {};
+        chain_x_ = false;
+      } else {
+        chain_x_ = true;  // (512 x 1200: 406 us, 418 not chained; 588 x 1400: 663 and 686)
+      }
+    }
   }
   if (fwd_.smem > (size_t)maxsm || inv_.smem > (size_t)maxsm) {
     *msg = "grid too large for the shared-memory x pass";
@@ -3574,10 +3613,14 @@ bool SpectralPlan::fuse_ok(const RhsIO& io, const RhsIO& next) const {
 
 // Whether a stage's passes are launched as a chain (a kernel's start and its tables overlap
 // the kernel before it): the latency-bound 2D grids of the fused pass, within a DP45
-// attempt.  128 x 128 run: 2.79 -> 2.53 ms; 256 x 256, where fewer SMs are free for the waiting
-// kernel: 3.13 -> 3.09; adjoint 256 x 256: 39.3 -> 38.2.
+// attempt, that leave SMs free for the waiting kernel's CTAs.  Those that start early are
+// spread over what room there is, and a pass of several of them on one SM takes as much longer:
+// 2D attempts of two fields, us, chained and not: 64 x 250 100 and 110, 256 x 128 100 and 101,
+// 256 x 256 103 and 107, but 280 x 512 164 and 156, 384 x 128 164 and 131, 512 x 250 199 and
+// 152, 576 x 256 193 and 158 (at the worst lengths; 300 x 128 137 and 139); three fields,
+// 128 x 128 97 and 107, 256 x 256 154 and 127.  Adjoint 256 x 256: 39.3 -> 38.2 ms.
 bool SpectralPlan::chained(const RhsIO& io) const {
-  return ndim == 2 && fuse_x_.per_cta > 0 && io.mode == 1 && io.stage >= 2;
+  return ndim == 2 && chain_x_ && io.mode == 1 && io.stage >= 2;
 }
 
 bool SpectralPlan::fuse_x_ok(const RhsIO& io, const RhsIO& next) const {

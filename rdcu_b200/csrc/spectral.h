@@ -152,6 +152,7 @@ class SpectralPlan {
   PassCfg midsolve_{};
   PassCfg fuse_x_{};  // the general fused inverse/forward x pass (per_cta 0: not taken)
   int fuse_off_ = 0;
+  bool chain_x_ = false;  // an attempt's kernels are launched as a chain
   // spectral buffers
   double2* Sf_ = nullptr;  // field half spectra [n][R][Mh]
   double2* Sc_ = nullptr;  // channel half spectra [max(nch, G)][R][Mh]
