@@ -5,12 +5,16 @@
 // Passes of one frame (grid of N points, n line cubes):
 //   k_phase     th = atan2(v, u) + pi                              16 B read, 8 B written /pt
 //   k_faces     winding of the three plaquettes at every point     8 B read, 1 B written /pt
-//   k_mark      line cubes (either side of a winding plaquette)    1 B read, 1 B written /pt
-//   k_compact   ascending cube list and the grid -> node map       1 B read, 4 B written /pt
-//   k_hook      union-find over face neighbours (lock-free CAS)    per node
-//   k_flatten, k_roots, k_label  component of every node, numbered by smallest cube
-//   radix passes: nodes stably sorted by component
+//   k_mark_bits line cubes (either side of a winding plaquette)    1 B read, 1 bit written /pt
+//   k_compact_bits  ascending cube list and the cubes' nodes       1 bit read /pt, 8 B written /cube
+//   k_neighbours, k_graph_small  component of every node, numbered by smallest cube
+//   k_order_small  nodes stably sorted by component
 //   k_edges     each component's edges (u < v ascending) as scaled coordinates
+// and, for frames of more than kSmallNodes cubes, instead of the three before k_edges:
+//   k_compact_all  the list again, whole
+//   k_hook      union-find over face neighbours (lock-free CAS)    per node
+//   k_flatten, k_roots, k_label  component of every node
+//   radix passes: nodes stably sorted by component
 // The grid passes are HBM-bound streaming passes (one thread per point, coalesced along
 // the last axis; neighbour reads hit L2).  The graph passes touch only the n line cubes.
 #include <cuda_runtime.h>
@@ -131,31 +135,6 @@ __device__ __forceinline__ int block_sum(int v, int* red) {
   return s;
 }
 
-// Line cube c: a winding plaquette on one of its six faces.  A (0,1) plaquette at p
-// borders cubes p and p - e2, a (1,2) one p and p - e0, a (2,0) one p and p - e1
-// (makelines.py:28-36), so cube c looks at its own three faces and at the (0,1) face of
-// c + e2, the (1,2) face of c + e0 and the (2,0) face of c + e1.
-__global__ void __launch_bounds__(kT) k_mark(const unsigned char* __restrict__ face, unsigned char* __restrict__ mark,
-                                             int* __restrict__ counts, Grid g) {
-  __shared__ int red[kT / 32];
-  int cnt = 0;
-  for (int r = 0; r < kSlices; ++r) {
-    const int c = blockIdx.x * kChunk + r * kT + threadIdx.x;
-    if (c < g.total) {
-      int i, j, k;
-      coords(g, c, i, j, k);
-      const int di = (i + 1 < g.N[0]) ? g.s0 : -(g.N[0] - 1) * g.s0;
-      const int dj = (j + 1 < g.N[1]) ? g.s1 : -(g.N[1] - 1) * g.s1;
-      const int dk = (k + 1 < g.N[2]) ? 1 : -(g.N[2] - 1);
-      const int m = ((face[c] & 7) | (face[c + dk] & 1) | (face[c + di] & 2) | (face[c + dj] & 4)) != 0;
-      mark[c] = (unsigned char)m;
-      cnt += m;
-    }
-  }
-  const int s = block_sum(cnt, red);
-  if (threadIdx.x == 0) counts[blockIdx.x] = s;
-}
-
 // Exclusive prefix of one slice's flags over the block, in index order; returns the
 // block's total for the slice.
 __device__ __forceinline__ int block_rank(bool f, int* wcnt, int* pre) {
@@ -171,32 +150,6 @@ __device__ __forceinline__ int block_rank(bool f, int* wcnt, int* pre) {
   *pre = off + __popc(b & ((1u << lane) - 1u));
   __syncthreads();
   return tot;
-}
-
-// Cubes in ascending index order (np.unique order of makelines.py:38-39), the grid ->
-// node map (-1 off the lines) and the union-find forest's initial singletons.
-__global__ void __launch_bounds__(kT) k_compact(const unsigned char* __restrict__ mark, const int* __restrict__ offs,
-                                                int* __restrict__ cubes, int* __restrict__ node_of,
-                                                int* __restrict__ parent, int total) {
-  __shared__ int wcnt[kT / 32];
-  int run = offs[blockIdx.x];
-  for (int r = 0; r < kSlices; ++r) {
-    const int c = blockIdx.x * kChunk + r * kT + threadIdx.x;
-    const bool m = c < total && mark[c];
-    int pre;
-    const int tot = block_rank(m, wcnt, &pre);
-    if (c < total) {
-      if (m) {
-        const int v = run + pre;
-        cubes[v] = c;
-        node_of[c] = v;
-        parent[v] = v;
-      } else {
-        node_of[c] = -1;
-      }
-    }
-    run += tot;
-  }
 }
 
 // Face neighbours of cube c (periodic): up to two per axis of length >= 3, one per axis of
@@ -251,8 +204,13 @@ __device__ void uf_union(int* parent, int a, int b, int* err) {
   atomicExch(err, 1);
 }
 
+// Node of point c, -1 off the lines (node_of is written at the cubes only).
+__device__ __forceinline__ int node_at(const unsigned* __restrict__ bits, const int* __restrict__ node_of, int c) {
+  return ((bits[c >> 5] >> (c & 31)) & 1u) ? node_of[c] : -1;
+}
+
 __global__ void __launch_bounds__(kT) k_hook(const int* __restrict__ cubes, const int* __restrict__ node_of,
-                                             int* parent, int* __restrict__ deg, int n, Grid g, int* err,
+                                             const unsigned* __restrict__ bits, int* parent, int* __restrict__ deg, int n, Grid g, int* err,
                                              int* n_edges) {
   const int v = blockIdx.x * kT + threadIdx.x;
   int d = 0;
@@ -260,7 +218,7 @@ __global__ void __launch_bounds__(kT) k_hook(const int* __restrict__ cubes, cons
     int nb[6];
     const int cnt = face_neighbours(g, cubes[v], nb);
     for (int q = 0; q < cnt; ++q) {
-      const int u = node_of[nb[q]];
+      const int u = node_at(bits, node_of, nb[q]);
       if (u > v) {
         ++d;
         uf_union(parent, v, u, err);
@@ -320,15 +278,19 @@ __device__ int uf_find_s(int* parent, int x, int* err) {
   return -1;
 }
 
-// ---- frames of few line cubes: the cube marks as bits, and the graph in one CTA, with
-// every count on the device, so that the host waits once per frame (for the counts) instead
-// of sizing each step.  flags: 0 error, 1 components, 2 edges, 3 cubes,
-// 4 further edges.  A frame with more
-// than kSmallNodes cubes is found again by the general passes.
+// ---- the cube marks as bits; and frames of few line cubes: the graph in one CTA, with every
+// count on the device, so that the host waits once per frame (for the counts) instead of
+// sizing each step.  flags: 0 error, 1 components, 2 edges, 3 cubes, 4 further edges.  A
+// frame of more than kSmallNodes cubes (the kernels after the compaction return at once) goes
+// on from the same marks and counts with the general passes.
 constexpr int kBitWords = 1024;  // words of bits per block of k_compact_bits
 
-// Line cube marks (k_mark's rule), a bit per point: a warp's 32 points are one word; and the
-// number of cubes in every kBitWords words (zeroed by the caller).
+// Line cube c: a winding plaquette on one of its six faces.  A (0,1) plaquette at p
+// borders cubes p and p - e2, a (1,2) one p and p - e0, a (2,0) one p and p - e1
+// (makelines.py:28-36), so cube c looks at its own three faces and at the (0,1) face of
+// c + e2, the (1,2) face of c + e0 and the (2,0) face of c + e1.  A bit per point: a warp's
+// 32 points are one word; and the number of cubes in every kBitWords words (zeroed by the
+// caller).
 __global__ void __launch_bounds__(kT) k_mark_bits(const unsigned char* __restrict__ face, unsigned* __restrict__ bits,
                                                   int* __restrict__ counts, Grid g) {
   const int c = blockIdx.x * kT + threadIdx.x;
@@ -347,25 +309,26 @@ __global__ void __launch_bounds__(kT) k_mark_bits(const unsigned char* __restric
   if (threadIdx.x == 0 && cnt) atomicAdd(&counts[(c >> 5) / kBitWords], cnt);
 }
 
-// Cubes in ascending order and their nodes, from the bits: a thread per word, after the sum
-// of the counts of the blocks before this one.  node_of is written at the cubes only;
-// readers test the bit first.
-__global__ void __launch_bounds__(kBitWords) k_compact_bits(const unsigned* __restrict__ bits, int nw,
-                                                       const int* __restrict__ counts,
-                                                       int* __restrict__ cubes, int* __restrict__ node_of, int cap,
-                                                       int* __restrict__ flags) {
+// The thread's word of bits (a thread per word, T threads per block), and the number of cubes
+// before it: those of the groups of kBitWords words before the block's, from their counts,
+// and those of the words before it in its group.
+template <int T>
+__device__ __forceinline__ unsigned word_and_offset(const unsigned* __restrict__ bits, int nw,
+                                                    const int* __restrict__ counts, int* off) {
+  static_assert(kBitWords % T == 0, "blocks within a group");
   __shared__ int red[32];
   __shared__ int sbase;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int w0 = blockIdx.x * T, g0 = w0 / kBitWords;
   int before = 0;
-  for (int q = threadIdx.x; q < (int)blockIdx.x; q += kBitWords) before += counts[q];
-  const int wi = blockIdx.x * kBitWords + threadIdx.x;
-  const unsigned mine = wi < nw ? bits[wi] : 0u;
+  for (int q = threadIdx.x; q < g0; q += T) before += counts[q];
+  for (int q = g0 * kBitWords + threadIdx.x; q < w0; q += T) before += __popc(bits[q]);
+  const unsigned mine = w0 + (int)threadIdx.x < nw ? bits[w0 + threadIdx.x] : 0u;
   for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
   if (lane == 0) red[w] = before;
   __syncthreads();
   if (w == 0) {
-    int t = red[lane];
+    int t = lane < T / 32 ? red[lane] : 0;
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) sbase = t;
   }
@@ -378,23 +341,50 @@ __global__ void __launch_bounds__(kBitWords) k_compact_bits(const unsigned* __re
   }
   if (lane == 31) red[w] = x;
   __syncthreads();
-  int off = sbase;
-  for (int q = 0; q < w; ++q) off += red[q];
-  int v = off + x - cnt;
-  for (unsigned m = mine; m; m &= m - 1) {
-    const int c = wi * 32 + __ffs(m) - 1;
-    if (v < cap) {
-      cubes[v] = c;
-      node_of[c] = v;
-    }
-    ++v;
-  }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kBitWords - 1) flags[3] = v;
+  int base = sbase;
+  for (int q = 0; q < w; ++q) base += red[q];
+  *off = base + x - cnt;
+  return mine;
 }
 
-__device__ __forceinline__ int node_at(const unsigned* __restrict__ bits, const int* __restrict__ node_of, int c) {
-  if (bits && !((bits[c >> 5] >> (c & 31)) & 1u)) return -1;
-  return node_of[c];
+// Cubes in ascending order (np.unique order of makelines.py:38-39) and their nodes, the
+// first `cap` of them, and their number.
+__global__ void __launch_bounds__(kBitWords) k_compact_bits(const unsigned* __restrict__ bits, int nw,
+                                                       const int* __restrict__ counts,
+                                                       int* __restrict__ cubes, int* __restrict__ node_of, int cap,
+                                                       int* __restrict__ flags) {
+  int v;
+  const unsigned mine = word_and_offset<kBitWords>(bits, nw, counts, &v);
+  const int wi = blockIdx.x * kBitWords + threadIdx.x;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kBitWords - 1) flags[3] = v + __popc(mine);
+  for (unsigned m = mine; m && v < cap; m &= m - 1) {
+    const int c = wi * 32 + __ffs(m) - 1;
+    cubes[v] = c;
+    node_of[c] = v;
+    ++v;
+  }
+}
+
+// The same for every cube, and the union-find forest's initial singletons: a lane per point
+// of a word, since the words of such frames may be full (a warp's stores are then one line).
+__global__ void __launch_bounds__(kT) k_compact_all(const unsigned* __restrict__ bits, int nw,
+                                                    const int* __restrict__ counts, int* __restrict__ cubes,
+                                                    int* __restrict__ node_of, int* __restrict__ parent) {
+  int off;
+  const unsigned mine = word_and_offset<kT>(bits, nw, counts, &off);
+  const int lane = threadIdx.x & 31;
+  const int w0 = blockIdx.x * kT + (threadIdx.x & ~31);
+  for (unsigned words = __ballot_sync(0xffffffffu, mine != 0); words; words &= words - 1) {
+    const int q = __ffs(words) - 1;
+    const unsigned m = __shfl_sync(0xffffffffu, mine, q);
+    const int o = __shfl_sync(0xffffffffu, off, q);
+    if ((m >> lane) & 1u) {
+      const int v = o + __popc(m & ((1u << lane) - 1u)), c = (w0 + q) * 32 + lane;
+      cubes[v] = c;
+      node_of[c] = v;
+      parent[v] = v;
+    }
+  }
 }
 
 // Every node's smallest lower neighbour (itself if it has none), its number of larger
@@ -767,7 +757,7 @@ __device__ __forceinline__ double scaled(int c, int a, const Grid& g) {
 
 // Node p of the component-sorted order writes its edges to the nodes above it, in
 // ascending order, and the offsets of its component when it is the component's first.
-// bits: set for a small frame, whose cube count is flags[3] and whose component offsets
+// flags: set for a small frame, whose cube count is flags[3] and whose component offsets
 // k_order_small has written (comp null).
 __global__ void __launch_bounds__(kT) k_edges(const int* __restrict__ order, const int* __restrict__ eoff,
                                               const int* __restrict__ cubes, const int* __restrict__ node_of,
@@ -776,7 +766,7 @@ __global__ void __launch_bounds__(kT) k_edges(const int* __restrict__ order, con
                                               long long* __restrict__ comp_noff, long long* __restrict__ comp_eoff,
                                               int n, int n_comp, int n_edges) {
   const int p = blockIdx.x * kT + threadIdx.x;
-  if (bits) {
+  if (flags) {
     n = flags[3];
     if (n > kSmallNodes) return;
   }
@@ -1017,7 +1007,7 @@ class LinesEngine {
     }
     const long long N = g.total;
     if (!th_.ensure(N, &device_bytes, st) || !src_.ensure(2 * N, &device_bytes, st) ||
-        !face_.ensure(N, &device_bytes, st) || !mark_.ensure(N, &device_bytes, st) ||
+        !face_.ensure(N, &device_bytes, st) ||
         !node_of_.ensure(N, &device_bytes, st) || !counts_.ensure(nblocks(N, kChunk) + 1, &device_bytes, st) ||
         !flags_.ensure(5, &device_bytes, st) || cudaMallocHost((void**)&h_small_, 4 * sizeof(long long)) != cudaSuccess)
       return fail(msg, "device memory");
@@ -1039,7 +1029,6 @@ class LinesEngine {
     src_.release();
     xyz_.release();
     face_.release();
-    mark_.release();
     wide_.release();
     comp_noff_.release();
     comp_eoff_.release();
@@ -1098,74 +1087,73 @@ class LinesEngine {
       launch(k_phase, nblocks(N, kT), kT, d, th_.p, N);
       th = th_.p;
     }
-    const int nb = nblocks(N, kChunk);
     launch(k_faces, nblocks(N, kT), kT, th, face_.p, g);
-    {
-      if (!zero_small_counts(msg)) return RDCU_ERR_CUDA;
-      launch_small_marks();
-      launch_small_compact();
-      launch_small_graph();
-      launch_small_order();
-      launch_small_edges();
-      int* hf = reinterpret_cast<int*>(h_small_);
+    if (!zero_small_counts(msg)) return RDCU_ERR_CUDA;
+    launch_small_marks();
+    launch_small_compact();
+    // A frame found after a large one is expected to be large too: the wait for its counts comes
+    // before the small frame's kernels (which large ones would launch to no end).
+    int* hf = reinterpret_cast<int*>(h_small_);
+    for (bool graph = was_small_;; graph = true) {
+      if (graph) {
+        launch_small_graph();
+        launch_small_order();
+        launch_small_edges();
+      }
       if (!ck(cudaMemcpyAsync(hf, flags_.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st), msg) ||
           !ck(cudaGetLastError(), msg) || !ck(cudaStreamSynchronize(st), msg))
         return RDCU_ERR_CUDA;
-      if (hf[3] <= kSmallNodes) {
-        if (hf[0] != 0) return fail_code(msg, "union-find iteration bound reached", RDCU_ERR_TIMEOUT);
-        n_cubes = hf[3];
-        n_comp = hf[1];
-        n_edges = hf[2];
-        sorted_ = order_.p;
-        was_small_ = true;
-        have = true;
-        return RDCU_OK;
-      }
+      was_small_ = hf[3] <= kSmallNodes;
+      if (graph || !was_small_) break;
     }
-    was_small_ = false;
-    launch(k_mark, nb, kT, face_.p, mark_.p, counts_.p, g);
-    int rc = scan(counts_.p, nb, msg);
-    if (rc) return rc;
-    const long long n = read_total(msg);
-    if (n < 0) return RDCU_ERR_CUDA;
+    if (was_small_) {
+      if (hf[0] != 0) return fail_code(msg, "union-find iteration bound reached", RDCU_ERR_TIMEOUT);
+      n_cubes = hf[3];
+      n_comp = hf[1];
+      n_edges = hf[2];
+      sorted_ = order_.p;
+      have = true;
+      return RDCU_OK;
+    }
+    // the marks and counts stand (128^3, 22469 cubes: 268 us a frame with byte marks and their
+    // count made again here and the small frame's kernels first, 239 so)
+    const long long n = hf[3];
     n_cubes = n;
     n_edges = n_comp = 0;
     if (!ensure_nodes(n)) return fail_code(msg, "device memory", RDCU_ERR_NOMEM);
     if (!ck(cudaMemsetAsync(flags_.p, 0, 3 * sizeof(int), st), msg)) return RDCU_ERR_CUDA;
-    launch(k_compact, nb, kT, mark_.p, counts_.p, cubes_.p, node_of_.p, parent_.p, N);
-    if (n > 0) {
-      const int nn = (int)n;
-      const int nbn = nblocks(n, kChunk);
-      if ((rc = components(nn, msg))) return rc;
-      // one read: union-find error flag, component count, edge count
-      int* hf = reinterpret_cast<int*>(h_small_);
-      if (!ck(cudaMemcpyAsync(hf, flags_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st), msg) ||
-          !ck(cudaStreamSynchronize(st), msg))
-        return RDCU_ERR_CUDA;
-      if (hf[0] != 0) return fail_code(msg, "union-find iteration bound reached", RDCU_ERR_TIMEOUT);
-      const long long nc = hf[1], ne = hf[2];
-      n_comp = nc;
-      n_edges = ne;
-      if (!comp_noff_.ensure(nc + 1, &device_bytes, st) || !comp_eoff_.ensure(nc + 1, &device_bytes, st) ||
-          !xyz_.ensure(ne * 6, &device_bytes, st))
-        return fail_code(msg, "device memory", RDCU_ERR_NOMEM);
-      // nodes stably sorted by component, 8 bits a pass; then the edges (no further host
-      // reads: edges(), cubes() and correlate() synchronise before using the results)
-      int *k0 = key_a_.p, *v0 = order_.p, *k1 = key_b_.p, *v1 = val_tmp_.p;
-      for (int shift = 0; ((nc - 1) >> shift) > 0; shift += 8) {
-        launch(k_rs_hist, nbn, kT, k0, nn, shift, hist_.p, nbn);
-        if ((rc = scan(hist_.p, 256 * nbn, msg))) return rc;
-        launch(k_rs_scatter, nbn, kT, k0, v0, k1, v1, nn, shift, hist_.p, nbn);
-        std::swap(k0, k1);
-        std::swap(v0, v1);
-      }
-      sorted_ = v0;
-      launch(k_edge_counts, nblocks(n, kT), kT, sorted_, deg_.p, eoff_.p, nn);
-      if ((rc = scan(eoff_.p, nn, msg))) return rc;
-      launch(k_edges, nblocks(n, kT), kT, sorted_, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)nullptr,
-             (const int*)nullptr, comp_.p, g, xyz_.p, comp_noff_.p,
-             comp_eoff_.p, nn, (int)nc, (int)ne);
+    launch_compact_all();
+    const int nn = (int)n;
+    const int nbn = nblocks(n, kChunk);
+    int rc = components(nn, msg);
+    if (rc) return rc;
+    // one read: union-find error flag, component count, edge count
+    if (!ck(cudaMemcpyAsync(hf, flags_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st), msg) ||
+        !ck(cudaStreamSynchronize(st), msg))
+      return RDCU_ERR_CUDA;
+    if (hf[0] != 0) return fail_code(msg, "union-find iteration bound reached", RDCU_ERR_TIMEOUT);
+    const long long nc = hf[1], ne = hf[2];
+    n_comp = nc;
+    n_edges = ne;
+    if (!comp_noff_.ensure(nc + 1, &device_bytes, st) || !comp_eoff_.ensure(nc + 1, &device_bytes, st) ||
+        !xyz_.ensure(ne * 6, &device_bytes, st))
+      return fail_code(msg, "device memory", RDCU_ERR_NOMEM);
+    // nodes stably sorted by component, 8 bits a pass; then the edges (no further host
+    // reads: edges(), cubes() and correlate() synchronise before using the results)
+    int *k0 = key_a_.p, *v0 = order_.p, *k1 = key_b_.p, *v1 = val_tmp_.p;
+    for (int shift = 0; ((nc - 1) >> shift) > 0; shift += 8) {
+      launch(k_rs_hist, nbn, kT, k0, nn, shift, hist_.p, nbn);
+      if ((rc = scan(hist_.p, 256 * nbn, msg))) return rc;
+      launch(k_rs_scatter, nbn, kT, k0, v0, k1, v1, nn, shift, hist_.p, nbn);
+      std::swap(k0, k1);
+      std::swap(v0, v1);
     }
+    sorted_ = v0;
+    launch(k_edge_counts, nblocks(n, kT), kT, sorted_, deg_.p, eoff_.p, nn);
+    if ((rc = scan(eoff_.p, nn, msg))) return rc;
+    launch(k_edges, nblocks(n, kT), kT, sorted_, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)bits_.p,
+           (const int*)nullptr, comp_.p, g, xyz_.p, comp_noff_.p,
+           comp_eoff_.p, nn, (int)nc, (int)ne);
     if (!ck(cudaGetLastError(), msg)) return RDCU_ERR_CUDA;
     have = true;
     return RDCU_OK;
@@ -1182,15 +1170,15 @@ class LinesEngine {
   int profile(const double* src, int kind, bool on_device, int reps, std::vector<PassTime>* out, std::string* msg) {
     int rc = find(src, kind, on_device, msg);
     if (rc) return rc;
-    const int N = g.total, nb = nblocks(N, kChunk);
+    const int N = g.total;
     const int nn = (int)n_cubes, nbn = nblocks(n_cubes, kChunk), nc = (int)n_comp, ne = (int)n_edges;
     const double* d = on_device ? src : src_.p;
     const double* th = kind == RDCU_LINES_STATE ? th_.p : d;
     const char* names[7] = {"phase", "faces", "mark", "compact", "components", "sort", "edges"};
     int passes = 0;
     for (int shift = 0; nc > 1 && ((nc - 1) >> shift) > 0; shift += 8) ++passes;
-    const double bytes[7] = {kind == RDCU_LINES_STATE ? 24.0 * N : 0.0, 9.0 * N, 2.0 * N,
-                             5.0 * N + 12.0 * nn, 48.0 * nn, 16.0 * passes * nn, 28.0 * nn + 48.0 * ne};
+    const double bytes[7] = {kind == RDCU_LINES_STATE ? 24.0 * N : 0.0, 9.0 * N, 1.125 * N,
+                             0.125 * N + 8.0 * nn, 48.0 * nn, 16.0 * passes * nn, 28.0 * nn + 48.0 * ne};
     cudaEvent_t ev[8];
     for (auto& e : ev)
       if (!ck(cudaEventCreate(&e), msg)) return RDCU_ERR_CUDA;
@@ -1201,10 +1189,10 @@ class LinesEngine {
       cudaEventRecord(ev[1], st);
       launch(k_faces, nblocks(N, kT), kT, th, face_.p, g);
       cudaEventRecord(ev[2], st);
+      if (!zero_small_counts(msg)) rc = RDCU_ERR_CUDA;
+      launch_small_marks();
+      cudaEventRecord(ev[3], st);
       if (was_small_) {
-        if (!zero_small_counts(msg)) return RDCU_ERR_CUDA;
-        launch_small_marks();
-        cudaEventRecord(ev[3], st);
         launch_small_compact();
         cudaEventRecord(ev[4], st);
         launch_small_graph();
@@ -1212,38 +1200,23 @@ class LinesEngine {
         launch_small_order();
         cudaEventRecord(ev[6], st);
         launch_small_edges();
-        cudaEventRecord(ev[7], st);
-        if (!ck(cudaEventSynchronize(ev[7]), msg)) rc = RDCU_ERR_CUDA;
-        for (int i = 0; i < 7 && rc == RDCU_OK; ++i) {
-          float ms = 0.f;
-          cudaEventElapsedTime(&ms, ev[i], ev[i + 1]);
-          acc[i] += ms;
+      } else {
+        launch_compact_all();
+        cudaEventRecord(ev[4], st);
+        if (rc == RDCU_OK) rc = components(nn, msg);
+        cudaEventRecord(ev[5], st);
+        int *k0 = key_a_.p, *v0 = order_.p, *k1 = key_b_.p, *v1 = val_tmp_.p;
+        for (int shift = 0; rc == RDCU_OK && ((nc - 1) >> shift) > 0; shift += 8) {
+          launch(k_rs_hist, nbn, kT, k0, nn, shift, hist_.p, nbn);
+          rc = scan(hist_.p, 256 * nbn, msg);
+          launch(k_rs_scatter, nbn, kT, k0, v0, k1, v1, nn, shift, hist_.p, nbn);
+          std::swap(k0, k1);
+          std::swap(v0, v1);
         }
-        continue;
-      }
-      launch(k_mark, nb, kT, face_.p, mark_.p, counts_.p, g);
-      rc = scan(counts_.p, nb, msg);
-      cudaEventRecord(ev[3], st);
-      launch(k_compact, nb, kT, mark_.p, counts_.p, cubes_.p, node_of_.p, parent_.p, N);
-      cudaEventRecord(ev[4], st);
-      if (nn > 0 && rc == RDCU_OK) {
-        cudaMemsetAsync(flags_.p, 0, 3 * sizeof(int), st);
-        rc = components(nn, msg);
-      }
-      cudaEventRecord(ev[5], st);
-      int *k0 = key_a_.p, *v0 = order_.p, *k1 = key_b_.p, *v1 = val_tmp_.p;
-      for (int shift = 0; nn > 0 && rc == RDCU_OK && ((nc - 1) >> shift) > 0; shift += 8) {
-        launch(k_rs_hist, nbn, kT, k0, nn, shift, hist_.p, nbn);
-        rc = scan(hist_.p, 256 * nbn, msg);
-        launch(k_rs_scatter, nbn, kT, k0, v0, k1, v1, nn, shift, hist_.p, nbn);
-        std::swap(k0, k1);
-        std::swap(v0, v1);
-      }
-      cudaEventRecord(ev[6], st);
-      if (nn > 0 && rc == RDCU_OK) {
+        cudaEventRecord(ev[6], st);
         launch(k_edge_counts, nblocks(nn, kT), kT, v0, deg_.p, eoff_.p, nn);
-        rc = scan(eoff_.p, nn, msg);
-        launch(k_edges, nblocks(nn, kT), kT, v0, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)nullptr,
+        if (rc == RDCU_OK) rc = scan(eoff_.p, nn, msg);
+        launch(k_edges, nblocks(nn, kT), kT, v0, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)bits_.p,
                (const int*)nullptr, comp_.p, g, xyz_.p, comp_noff_.p, comp_eoff_.p, nn, nc, ne);
       }
       cudaEventRecord(ev[7], st);
@@ -1367,11 +1340,11 @@ class LinesEngine {
 
  private:
   Buf<double> th_, src_, xyz_;
-  Buf<unsigned char> face_, mark_;
+  Buf<unsigned char> face_;
   Buf<int> node_of_, counts_, sums_, flags_;  // flags_[0]: error, flags_[1]: scan total
-  Buf<unsigned> bits_;                        // line cube marks of a small frame
+  Buf<unsigned> bits_;                        // line cube marks
   Buf<int2> extra_;                           // its edges beyond each node's lowest
-  bool was_small_ = false;                    // the last frame had at most kSmallNodes cubes
+  bool was_small_ = true;                     // the last frame had at most kSmallNodes cubes
   Buf<int> cubes_, parent_, deg_, label_, root_comp_, comp_, key_a_, key_b_, order_, val_tmp_, eoff_, hist_, diff32_;
   Buf<long long> wide_, comp_noff_, comp_eoff_, diff64_, sets_;
   Buf<int4> packed_, packed_b_;
@@ -1426,6 +1399,10 @@ class LinesEngine {
     launch(k_compact_bits, nblocks(bit_words(), kBitWords), kBitWords, bits_.p, bit_words(), (const int*)counts_.p,
            cubes_.p, node_of_.p, kSmallNodes, flags_.p);
   }
+  void launch_compact_all() {
+    launch(k_compact_all, nblocks(bit_words(), kT), kT, (const unsigned*)bits_.p, bit_words(),
+           (const int*)counts_.p, cubes_.p, node_of_.p, parent_.p);
+  }
   void launch_small_graph() {
     launch(k_neighbours, nblocks(kSmallNodes, kT), kT, (const unsigned*)bits_.p, (const int*)cubes_.p,
            (const int*)node_of_.p, parent_.p, deg_.p, extra_.p, g, flags_.p);
@@ -1440,12 +1417,12 @@ class LinesEngine {
     launch(k_edges, nblocks(kSmallNodes, kT), kT, order_.p, eoff_.p, cubes_.p, node_of_.p, (const unsigned*)bits_.p,
            (const int*)flags_.p, (const int*)nullptr, g, xyz_.p, comp_noff_.p, comp_eoff_.p, 0, 0, 0);
   }
-  // components of the n >= 1 line cubes (after k_compact): deg, comp, key_a_ and order_,
+  // components of the n >= 1 line cubes (after k_compact_all): deg, comp, key_a_ and order_,
   // the component count in flags_[1], the edge count added to flags_[2] (zeroed by the
   // caller)
   int components(int n, std::string* msg) {
     const int nbn = nblocks(n, kChunk);
-    launch(k_hook, nblocks(n, kT), kT, cubes_.p, node_of_.p, parent_.p, deg_.p, n, g, flags_.p, flags_.p + 2);
+    launch(k_hook, nblocks(n, kT), kT, cubes_.p, node_of_.p, (const unsigned*)bits_.p, parent_.p, deg_.p, n, g, flags_.p, flags_.p + 2);
     launch(k_flatten, nbn, kT, parent_.p, label_.p, n, counts_.p, flags_.p);
     if (int rc = scan(counts_.p, nbn, msg)) return rc;
     launch(k_roots, nbn, kT, label_.p, counts_.p, root_comp_.p, n);
@@ -1464,12 +1441,6 @@ class LinesEngine {
       launch(k_chunk_scan, nb, kT, a, n, (const int*)sums_.p);
     }
     return ck(cudaGetLastError(), msg) ? RDCU_OK : RDCU_ERR_CUDA;
-  }
-  long long read_total(std::string* msg) {
-    if (!ck(cudaMemcpyAsync(h_small_, flags_.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st), msg) ||
-        !ck(cudaStreamSynchronize(st), msg))
-      return -1;
-    return *(int*)h_small_;
   }
 };
 

@@ -272,3 +272,21 @@ def test_phases_outside_one_turn(cuda, span):
     h.find(th.ravel(), 1)
     assert same_components(h.lines(), ol.findlines(th, Ns, Ls), Ns, Ls)
     h.close()
+
+
+@pytest.mark.parametrize("Ns,amp", [((40, 41, 43), 3.0), ((40, 41, 43), 1.1), ((64, 32, 49), 1.1)])
+def test_large_frames_over_several_groups_of_marks(cuda, Ns, amp):
+    """More than 12288 cubes on grids of several 32768-point groups of marks with a partial
+    last word, full words and sparse ones, alternating with a frame of few cubes."""
+    Ls = (9.0, 8.0, 7.0)
+    rng = np.random.default_rng(5)
+    many = np.pi + amp * rng.normal(size=Ns)
+    few = ol.phase(defect_state(Ns, 33, 0, 2, 0.1), Ns)
+    assert np.count_nonzero(ol.line_cubes(few)) <= 12288 < np.count_nonzero(ol.line_cubes(many))
+    h = _lines(Ns, Ls)
+    for th in (many, few, many, many, few, few):
+        h.find(np.ascontiguousarray(th).ravel(), 1)
+        assert same_components(h.lines(), ol.findlines(th, Ns, Ls), Ns, Ls)
+        idx, off = h.cubes()
+        assert np.array_equal(np.sort(idx), np.flatnonzero(ol.line_cubes(th)))
+    h.close()
