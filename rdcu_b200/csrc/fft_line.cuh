@@ -40,6 +40,16 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pr
   const int n = pred ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
 }
+// W = 4, 8 or 16 bytes, both addresses W-byte aligned
+template <int W>
+__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
+  if constexpr (W == 16) {
+    cp_async16(smem, gmem, true);
+  } else {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gmem), "n"(W) : "memory");
+  }
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 // commit the copies issued so far as a group; wait until at most one group is pending
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }

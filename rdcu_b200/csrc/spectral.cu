@@ -260,10 +260,11 @@ __device__ __forceinline__ bool stage_twiddles(double2* dst, const double2* src,
   return swz;
 }
 
-// Starts the copy of `bytes` (a multiple of 16, both addresses 16-byte aligned).
+// Starts the copy of `bytes` (a multiple of W, both addresses W-byte aligned).
+template <int W = 16>
 __device__ __forceinline__ void stage_table(void* dst, const void* src, int bytes) {
-  for (int t = threadIdx.x * 16; t < bytes; t += blockDim.x * 16)
-    cp_async16(static_cast<char*>(dst) + t, static_cast<const char*>(src) + t, true);
+  for (int t = threadIdx.x * W; t < bytes; t += blockDim.x * W)
+    cp_async<W>(static_cast<char*>(dst) + t, static_cast<const char*>(src) + t);
 }
 
 // acc + c k rounded once: the stage sums are formed by several kernels, which must agree
@@ -1412,7 +1413,10 @@ __device__ __forceinline__ void stage_older_slopes(const Resolved& r, int n, int
 // completes stage s + 1's state (stage_value_t's terms in its order), which is written,
 // transformed and split into half spectra: the separate passes' arithmetic, bit for bit,
 // without reading the slope and the state back and with one launch less.
-template <int RS, int LX, bool FUSE = false>
+// GROUP: in a batched kernel, whose tiles are large and whose code stays cached: plain copies of the
+// term tables and four points per thread throughout (the asynchronous ones spill there:
+// ensemble of 128 x 128 members 17.5 -> 18.6 ms).
+template <int RS, int LX, bool FUSE = false, bool GROUP = false>
 __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   extern __shared__ double2 sm[];
   if (a.io.mode == 1 && !a.io.ctl->running) return;
@@ -1440,12 +1444,21 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
   int* sfold = sfb + n + 1;
   if (!a.Yout) {
     stage_table(spoly, a.dict.poly, npoly * (int)sizeof(double));  // (npoly is even)
-    if (!a.dict.poly_nf) {
-      for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
-      for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
-      for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
+    if constexpr (GROUP) {
+      if (!a.dict.poly_nf) {
+        for (int t = tid; t < a.dict.nterms; t += T) sterm[t] = a.dict.terms[t];
+        for (int t = tid; t < a.dict.nfac; t += T) sfac[t] = a.dict.fac[t];
+        for (int t = tid; t <= n; t += T) sfb[t] = a.dict.field_begin[t];
+      }
+      for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
+    } else {
+      if (!a.dict.poly_nf) {
+        stage_table<8>(sterm, a.dict.terms, a.dict.nterms * (int)sizeof(DictTerm));
+        stage_table<8>(sfac, a.dict.fac, a.dict.nfac * (int)sizeof(DictFactor));
+        stage_table<4>(sfb, a.dict.field_begin, (n + 1) * (int)sizeof(int));
+      }
+      stage_table<4>(sfold, a.dict.fold, n * (int)sizeof(int));
     }
-    for (int t = tid; t < n; t += T) sfold[t] = a.dict.fold[t];
   }
   chain_wait();
   if (!a.Yout) {
@@ -1700,7 +1713,13 @@ __device__ __forceinline__ void inv_x_body(const InvXArgs& a, int bx) {
     case 2: points(I2{}, I2{}); break;
     case 3: points(std::integral_constant<int, FUSE ? 2 : 1>{}, std::integral_constant<int, 3>{}); break;
     default:
-      if constexpr (!FUSE) points(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{});
+      if constexpr (!FUSE) {
+        // (a tile of few points runs through its code once or twice, from a cold instruction cache)
+        if (!GROUP && npts <= 2 * T)
+          points(I1{}, std::integral_constant<int, 0>{});
+        else
+          points(std::integral_constant<int, 4>{}, std::integral_constant<int, 0>{});
+      }
       break;
   }
   if constexpr (FUSE) {
@@ -2516,7 +2535,7 @@ __global__ void __launch_bounds__(lb_threads(RS, LX), lb_ctas(RS, LX, 3))
     const int2 w = items[it];
     load_args(&sa, args + w.x);
     __syncthreads();
-    inv_x_body<RS, LX>(sa, w.y);
+    inv_x_body<RS, LX, false, true>(sa, w.y);
     __syncthreads();
   }
 }
