@@ -248,3 +248,10 @@ def test_a_shorter_line_leaves_a_longer_one_alone(cuda):
     run(b, yb)
     a.close()
     b.close()
+
+
+# a cluster of every size (1 to 8 CTAs), and lines above 8192 points
+@pytest.mark.parametrize("n,N", [(2, 1024), (2, 2000), (2, 2187), (2, 2560), (2, 3125), (2, 4374), (2, 4802), (2, 12000),
+                                 (4, 9216), (1, 16384)])
+def test_line_preconditioner_of_every_cluster(cuda, n, N):
+    test_line_preconditioner_matches_direct_solves(cuda, n, N)

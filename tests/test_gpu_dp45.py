@@ -312,6 +312,33 @@ def test_fixed_steps_of_many_butterflies(cuda, n, Ns):
     assert rel_err(out.cpu().numpy(), o.y) < 1e-10
 
 
+@pytest.mark.parametrize("Ns", [(60,), (256,), (260,), (20, 24)])
+def test_adaptive_sequence_of_a_term_list(cuda, Ns):
+    """The error epilogue after a term list, in tiles of few points and of more."""
+    from oracle.problem import parse_term
+
+    nd = len(Ns)
+    lines = ["-0.1,0,0,4", "0.2,0,%d,1,1,1" % 2, "-1.0,1,1,3", "0.5,1,0,1"]
+    lines += ["%s,%d,%d,1" % (0.7 + 0.2 * i, i, 2 + 2 * nd + (a * nd + a) * 2 + i) for i in range(2) for a in range(nd)]
+    prob = Problem(2, Ns, tuple(0.8 * v for v in Ns), [parse_term(s) for s in lines])
+    y0 = np.random.default_rng(4).uniform(-1, 1, 2 * prob.N)
+    s, yd = _setup(cuda, prob, y0)
+    s.set_state(0.0, 1e-2, yd.data_ptr())
+    o = _oracle(prob, y0, False)
+    t = to = 0.0
+    hg = ho = 1e-2
+    for _ in range(12):
+        acc, t, hg = s.step(t, hg)
+        ok, to, ho = o.step(to, ho, 0.0, np.inf)
+        if ok:
+            o.k[0] = o.k[6]
+        assert acc == ok and abs(hg - ho) <= 1e-9 * abs(ho)
+    out = cuda.empty_like(yd)
+    s.get_state(out.data_ptr())
+    s.close()
+    assert rel_err(out.cpu().numpy(), o.y) < 1e-9
+
+
 @pytest.mark.parametrize("Ns", [(128, 128), (24, 18), (15, 9), (48,), (12, 10, 8)])
 @pytest.mark.parametrize("deriv", [True, False])
 def test_profile_passes_of_every_dimension(cuda, Ns, deriv):

@@ -314,3 +314,17 @@ def test_a_smaller_grid_leaves_a_larger_one_alone(cuda):
     assert cuda.equal(f[0], f[1])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("Ns", [(5,), (128,), (250,), (256,), (260,), (288,), (2048,), (6, 40), (16, 22), (600, 12)])
+def test_term_lists_on_both_sides_of_a_small_tile(cuda, Ns):
+    """A dictionary that is no dense polynomial (degree 4, a derivative in a product) on tiles of up
+    to and above two points per thread (256 points of 128 threads), and of several rows."""
+    ndim, n = len(Ns), 2
+    d0, d00 = n, n + ndim * n
+    lines = ["0.3,0,0,4", "-1.0,0,0,3", "0.2,0,%d,1,1,1" % d0, "0.7,0,%d,1" % d00, "0.9,1,%d,1" % (d00 + 1), "-1.0,1,1,3",
+             "0.4,1", "-0.5,1,0,2,1,2"]
+    prob = Problem(n, Ns, tuple(0.6 * v for v in Ns), [parse_term(s) for s in lines])
+    y = np.random.default_rng(Ns[0]).uniform(-1, 1, n * prob.N)
+    f, _ = gpu_rhs(cuda, prob, y)
+    assert rel_err(f, osp.rhs(y, prob)) < TOL
