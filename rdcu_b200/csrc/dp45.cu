@@ -15,7 +15,6 @@
 
 #include "dp45.h"
 #include "dp45_ctl.cuh"
-#include "fft_line.cuh"
 
 namespace rdcu {
 

@@ -223,7 +223,6 @@ bool FDProblem::init(int n_, int ndim_, const int* Ns_, const double* Ls_, const
   for (int a = 0; a < ndim; ++a) {
     const double scale = Ls[a] / Ns[a];  // rdcu.cu:442
     T.s1[a] = 0.5 / scale;
-    T.inv_dx[a] = 1.0 / scale;
     for (int b = 0; b < ndim; ++b) {
       const double sc = (Ls[a] / Ns[a]) * (Ls[b] / Ns[b]);  // rdcu.cu:496
       T.r1[a][b] = 1.0 / sc;

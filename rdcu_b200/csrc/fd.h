@@ -32,7 +32,6 @@ struct FDTables {
   int n, ndim, nY, nterms, ncontrib;
   int Ns[3];
   unsigned stride[3];    // of the axes, in points
-  double inv_dx[3];      // 1/dx per axis (first derivative scale uses 0.5/dx exactly as below)
   double s1[3];          // 0.5/dx_a  (rdcu.cu:442-446)
   // 1, 2 and 1/2 over dx_a dx_b (rdcu.cu:496,502-504,561-564): the stencil values, divided
   // once on the host (the same IEEE quotients; a division per stencil was most of k_fd_rhs)

@@ -97,7 +97,7 @@ __device__ __forceinline__ double root_sin(int k) {
 template <int R, bool INV>
 struct Dft {
   static_assert(R == 3 || R == 5 || R == 7 || R == 11 || R == 13, "odd primes");
-  __device__ __forceinline__ static void run(double2 (&v)[R], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[R]) {
     constexpr int H = (R - 1) / 2;
     double2 a[H], b[H];  // per output pair (k, R - k): cosine and sine sums
     const double2 v0 = v[0];
@@ -134,7 +134,7 @@ struct Dft {
 
 template <bool INV>
 struct Dft<2, INV> {
-  __device__ __forceinline__ static void run(double2 (&v)[2], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[2]) {
     double2 a = v[0], b = v[1];
     v[0] = c_add(a, b);
     v[1] = c_sub(a, b);
@@ -143,7 +143,7 @@ struct Dft<2, INV> {
 
 template <bool INV>
 struct Dft<4, INV> {
-  __device__ __forceinline__ static void run(double2 (&v)[4], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[4]) {
     double2 t0 = c_add(v[0], v[2]), t1 = c_sub(v[0], v[2]);
     double2 t2 = c_add(v[1], v[3]), t3 = c_rot<INV>(c_sub(v[1], v[3]));
     v[0] = c_add(t0, t2);
@@ -155,13 +155,13 @@ struct Dft<4, INV> {
 
 template <bool INV>
 struct Dft<8, INV> {
-  __device__ __forceinline__ static void run(double2 (&v)[8], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[8]) {
     // X[k] = E[k] + W^k O[k], X[k+4] = E[k] - W^k O[k]; E, O = 4-point DFTs of the
     // even and odd inputs; W = exp(-+ 2 pi i / 8).
     double2 e[4] = {v[0], v[2], v[4], v[6]};
     double2 o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4, INV>::run(e, nullptr, 0);
-    Dft<4, INV>::run(o, nullptr, 0);
+    Dft<4, INV>::run(e);
+    Dft<4, INV>::run(o);
     const double s = 0.70710678118654752440;  // sqrt(1/2)
     // W^1 = s(1 -+ i), W^2 = -+ i, W^3 = s(-1 -+ i)
     double2 w1o = INV ? make_double2(s * (o[1].x - o[1].y), s * (o[1].x + o[1].y))
@@ -192,14 +192,14 @@ struct DftCoprime {
     for (int n2 = 0; n2 < N2; ++n2) {
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) t[n2][n1] = v[(N2 * n1 + N1 * n2) % N];
-      Dft<N1, INV>::run(t[n2], nullptr, 0);
+      Dft<N1, INV>::run(t[n2]);
     }
     double2 u[N1][N2];
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) {
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) u[k1][n2] = t[n2][k1];
-      Dft<N2, INV>::run(u[k1], nullptr, 0);
+      Dft<N2, INV>::run(u[k1]);
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) v[k] = u[k % N1][k % N2];
@@ -208,7 +208,7 @@ struct DftCoprime {
 #define RDCU_DFT_COPRIME(R, N1, N2)                                                        \
   template <bool INV>                                                                      \
   struct Dft<R, INV> {                                                                     \
-    __device__ __forceinline__ static void run(double2 (&v)[R], const double2*, int) {     \
+    __device__ __forceinline__ static void run(double2 (&v)[R]) {     \
       DftCoprime<N1, N2, INV>::run(v);                                                     \
     }                                                                                      \
   }
@@ -222,13 +222,13 @@ RDCU_DFT_COPRIME(15, 3, 5);
 // R x R points in two steps: X[k1 + R k2] = sum_n2 W^(n2 k1) W_R^(n2 k2) sum_n1 x[R n1 + n2] W_R^(n1 k1)
 template <bool INV>
 struct Dft<9, INV> {
-  __device__ __forceinline__ static void run(double2 (&v)[9], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[9]) {
     double2 t[3][3];
 #pragma unroll
     for (int n2 = 0; n2 < 3; ++n2) {
 #pragma unroll
       for (int n1 = 0; n1 < 3; ++n1) t[n2][n1] = v[3 * n1 + n2];
-      Dft<3, INV>::run(t[n2], nullptr, 0);
+      Dft<3, INV>::run(t[n2]);
 #pragma unroll
       for (int k1 = 1; k1 < 3; ++k1)
         if (n2 > 0) t[n2][k1] = c_mul(t[n2][k1], make_double2(c_w9[2 * n2 * k1], INV ? c_w9[2 * n2 * k1 + 1] : -c_w9[2 * n2 * k1 + 1]));
@@ -236,7 +236,7 @@ struct Dft<9, INV> {
 #pragma unroll
     for (int k1 = 0; k1 < 3; ++k1) {
       double2 u[3] = {t[0][k1], t[1][k1], t[2][k1]};
-      Dft<3, INV>::run(u, nullptr, 0);
+      Dft<3, INV>::run(u);
 #pragma unroll
       for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = u[k2];
     }
@@ -244,13 +244,13 @@ struct Dft<9, INV> {
 };
 template <bool INV>
 struct Dft<16, INV> {
-  __device__ __forceinline__ static void run(double2 (&v)[16], const double2*, int) {
+  __device__ __forceinline__ static void run(double2 (&v)[16]) {
     double2 t[4][4];
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
 #pragma unroll
       for (int n1 = 0; n1 < 4; ++n1) t[n2][n1] = v[4 * n1 + n2];
-      Dft<4, INV>::run(t[n2], nullptr, 0);
+      Dft<4, INV>::run(t[n2]);
 #pragma unroll
       for (int k1 = 1; k1 < 4; ++k1) {
         if (n2 == 0) continue;
@@ -261,7 +261,7 @@ struct Dft<16, INV> {
 #pragma unroll
     for (int k1 = 0; k1 < 4; ++k1) {
       double2 u[4] = {t[0][k1], t[1][k1], t[2][k1], t[3][k1]};
-      Dft<4, INV>::run(u, nullptr, 0);
+      Dft<4, INV>::run(u);
 #pragma unroll
       for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = u[k2];
     }
@@ -320,7 +320,7 @@ __device__ __forceinline__ void stockham_stage(double2* buf, int LS, int nlines,
         if (r > 0 && tstep != 0) x = c_mul(x, tw_get<INV>(tw, twz ? swz8(r * tstep) : r * tstep));
         v[q][r] = x;
       }
-      Dft<R, INV>::run(v[q], tw, L);
+      Dft<R, INV>::run(v[q]);
       dbase[q] = line * LS;
       dst[q] = jd * Ns * R + kk;
     } else {

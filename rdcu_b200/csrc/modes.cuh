@@ -22,10 +22,12 @@ __device__ __forceinline__ double2 lin_symbol(const LinTable& t, int g, const in
   return make_double2(-2.0 * sa * sb * t.idx[a] * t.idx[b], 0.0);
 }
 
-// The operators and their coefficients are kernel parameters (constant memory): reading
-// the entry list from global memory, entry by entry, was a third of k_mid_solve's time.
-// x = (I + alpha L(k))^-1 r at one mode, n <= NF <= kMaxPrecFields, Gaussian elimination
-// with partial pivoting; a (numerically) singular mode is passed through unchanged.
+// x = (I + alpha L(k))^-1 r at one mode, n <= NF <= kMaxPrecFields, by Gaussian elimination
+// with partial pivoting, or Cramer's rule where it does; a (numerically) singular mode is
+// passed through unchanged.
+// The operators and their coefficients come with the kernel's parameters (constant memory):
+// reading the entry list from global memory, entry by entry, was a third of k_mid_solve's
+// time.
 template <int NF>
 __device__ __forceinline__ void mode_solve(const LinTable& t, const int* nidx, double2* v, int n) {
   static_assert(NF <= kMaxPrecFields, "mode solves of at most kMaxPrecFields fields");
@@ -120,7 +122,6 @@ __device__ __forceinline__ void mode_solve(const LinTable& t, const int* nidx, d
     const double inv = 1.0 / (piv.x * piv.x + piv.y * piv.y);
     b[k] = c_mul(acc, make_double2(piv.x * inv, -piv.y * inv));
   }
-  
 #pragma unroll
   for (int i = 0; i < NF; ++i)
     if (i < n) v[i] = b[i];

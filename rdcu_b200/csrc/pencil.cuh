@@ -161,7 +161,7 @@ struct WarpLine {
   template <bool INV, typename At>
   __device__ __forceinline__ void transform(double2 (&v)[8], At at) const {
     // stage 1: radix 8, span 1: inputs v[r] = x[ml + LPL r]; outputs 8 ml + r, swizzled
-    Dft<8, INV>::run(v, nullptr, 0);
+    Dft<8, INV>::run(v);
 #pragma unroll
     for (int r = 0; r < 8; ++r) *at(swz8(8 * ml + r)) = v[r];
     __syncwarp();
@@ -174,7 +174,7 @@ struct WarpLine {
         if (r > 0 && tw_on) x = twid<INV>(x, w2[r - 1]);
         v[r] = x;
       }
-      Dft<8, INV>::run(v, nullptr, 0);
+      Dft<8, INV>::run(v);
       __syncwarp();
       const int d0 = (ml >> 3) * 64 + (ml & 7);
 #pragma unroll
@@ -192,7 +192,7 @@ struct WarpLine {
         if (r > 0 && j != 0) x = twid<INV>(x, w3[q][r - 1]);
         t[q][r] = x;
       }
-      Dft<R3, INV>::run(t[q], nullptr, 0);
+      Dft<R3, INV>::run(t[q]);
     }
     // output j + 64 r = ml + LPL (q + QB3 r)
 #pragma unroll

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(LX > 0 ? 256 : kLineThreads, 1) k_prec_line(co
       v[r] = src[p * Q + av];
       if (r > 0) v[r] = c_mul(v[r], __ldg(&a.tw[r * av]));
     }
-    if constexpr (C > 1) Dft<C, false>::run(v, a.tw, N);
+    if constexpr (C > 1) Dft<C, false>::run(v);
 #pragma unroll
     for (int b = 0; b < C; ++b) X[e * C + b] = v[b];
   }
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(LX > 0 ? 256 : kLineThreads, 1) k_prec_line(co
     double2 v[C];
 #pragma unroll
     for (int b = 0; b < C; ++b) v[b] = X[e * C + b];
-    if constexpr (C > 1) Dft<C, true>::run(v, a.tw, N);
+    if constexpr (C > 1) Dft<C, true>::run(v);
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       if (r > 0) v[r] = c_mul(v[r], tw_get<true>(a.tw, r * av));

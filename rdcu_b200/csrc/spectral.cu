@@ -2302,7 +2302,7 @@ __global__ void __launch_bounds__(kPlaneFwdThreads, 1) k_fwd_plane(PlaneArgs a) 
       double2 v[8];
 #pragma unroll
       for (int q2 = 0; q2 < 8; ++q2) v[q2] = rows[(q1 + 4 * q2) * Mh + kx];
-      Dft<8, false>::run(v, nullptr, 0);
+      Dft<8, false>::run(v);
       if (q1 > 0) {
 #pragma unroll
         for (int k2 = 1; k2 < 8; ++k2) v[k2] = c_mul(v[k2], a.twy[C * q1 * k2]);
@@ -2317,7 +2317,7 @@ __global__ void __launch_bounds__(kPlaneFwdThreads, 1) k_fwd_plane(PlaneArgs a) 
       double2 w[4];
 #pragma unroll
       for (int q1 = 0; q1 < 4; ++q1) w[q1] = rows[(q1 + 4 * k2) * Mh + kx];
-      Dft<4, false>::run(w, nullptr, 0);
+      Dft<4, false>::run(w);
 #pragma unroll
       for (int k1 = 0; k1 < 4; ++k1) {
         const int t = (int)rank * (k2 + 8 * k1);
@@ -2333,7 +2333,7 @@ __global__ void __launch_bounds__(kPlaneFwdThreads, 1) k_fwd_plane(PlaneArgs a) 
       double2 v[C];
 #pragma unroll
       for (int rr = 0; rr < C; ++rr) v[rr] = cl_load(cl_map(src, rr));
-      Dft<C, false>::run(v, nullptr, 0);
+      Dft<C, false>::run(v);
       double2* dst = a.S + (((long long)f * a.N0 + z) * N1 + aa) * Mh + kx;
 #pragma unroll
       for (int b = 0; b < C; ++b) dst[(long long)32 * b * Mh] = v[b];
@@ -2375,7 +2375,7 @@ __global__ void __launch_bounds__(kPlaneInvThreads, 1) k_inv_plane(PlaneArgs a) 
         double2 v[C];
 #pragma unroll
         for (int b = 0; b < C; ++b) v[b] = src[(long long)32 * b * Mh];
-        Dft<C, true>::run(v, nullptr, 0);
+        Dft<C, true>::run(v);
 #pragma unroll
         for (int rr = 0; rr < C; ++rr) {
           const int t = rr * aa;
@@ -2394,7 +2394,7 @@ __global__ void __launch_bounds__(kPlaneInvThreads, 1) k_inv_plane(PlaneArgs a) 
           const int aa = k2 + 8 * k1;
           w[k1] = cl_load(cl_map(zo + ((int)rank * AC + aa % AC) * Mh + kx, aa / AC));
         }
-        Dft<4, true>::run(w, nullptr, 0);
+        Dft<4, true>::run(w);
 #pragma unroll
         for (int q1 = 0; q1 < 4; ++q1) {
           const int t = C * k2 * q1;
@@ -2408,7 +2408,7 @@ __global__ void __launch_bounds__(kPlaneInvThreads, 1) k_inv_plane(PlaneArgs a) 
         double2 v[8];
 #pragma unroll
         for (int k2 = 0; k2 < 8; ++k2) v[k2] = rc[(q1 + 4 * k2) * Mh + kx];
-        Dft<8, true>::run(v, nullptr, 0);
+        Dft<8, true>::run(v);
 #pragma unroll
         for (int q2 = 0; q2 < 8; ++q2) rc[(q1 + 4 * q2) * Mh + kx] = v[q2];
       }
