@@ -932,7 +932,8 @@ def launches_per_attempt_of(name, names=()):
 
 def fused_pairs_2d(Ns):
     """Pairs of x passes of an attempt that a 2D grid launches as one (see fuse_geometry in
-    spectral.cu: at most 592 rows, an even number of them)."""
+    spectral.cu: at most 592 rows, an even number of them; rows of up to 800 points, which
+    two fields' CTAs share an SM with)."""
     fused = len(Ns) == 2 and Ns[0] % 2 == 0 and Ns[0] // 2 <= 296
     return 5 if fused and os.environ.get("RDCU_FUSED_ROWS") != "0" else 0
 
