@@ -352,3 +352,11 @@ def test_profile_passes_of_every_dimension(cuda, Ns, deriv):
     names = [p[0] for p in s.profile_passes(reps=1)]
     assert ("mid_axis0" in names) == (deriv and len(Ns) >= 2) and ("c2c_axis1_fwd" in names) == (deriv and len(Ns) == 3)
     s.close()
+
+
+@pytest.mark.parametrize("n,Ns", [(2, (256, 40)), (2, (260, 40)), (2, (512, 64)), (1, (588, 50)), (3, (128, 36)),
+                                  (3, (130, 36)), (3, (40, 512)), (3, (40, 520)), (2, (300, 900)), (2, (512, 1100))])
+def test_fused_x_passes_across_their_rules(cuda, monkeypatch, n, Ns):
+    """Chained and not (256 lines in all CTAs), fused and not (CTAs that share an SM or have it to
+    themselves, four lines of up to 512 points, a state beyond L2)."""
+    test_fused_x_passes_are_the_separate_ones(cuda, monkeypatch, n, Ns, False)
